@@ -31,35 +31,42 @@ __device__ __forceinline__ int3 stencil_centre(float4 q, const DevConsts& c) {
     return stencil_centre(make_float3(q.x, q.y, q.z), c);
 }
 
+// Row o (0..8, in the reference's order) of the stencil around `ctr`: [x, y),
+// empty as (0, 0).
+__device__ __forceinline__ int2 run_of_row(int o, int3 ctr, const DevConsts& c,
+                                           const int32_t* __restrict__ cstart,
+                                           const int32_t* __restrict__ cend) {
+    const uint32_t Gx = c.Gi[0], Gy = c.Gi[1], Gz = c.Gi[2];
+    const int xlo = ctr.x > 0 ? ctr.x - 1 : 0;
+    const int xhi = ctr.x + 1 < (int)Gx ? ctr.x + 1 : (int)Gx - 1;
+    const int ny = ctr.y + (o / 3) - 1, nz = ctr.z + (o % 3) - 1;
+    int32_t first = -1, last = -1;
+    if (ny >= 0 && ny < (int)Gy && nz >= 0 && nz < (int)Gz) {
+        const uint32_t base = c.cell_base + (uint32_t)ny * c.GxGz + (uint32_t)nz * Gx;
+        for (int xx = xlo; xx <= xhi; ++xx) {
+            const int32_t s = __ldg(cstart + base + (uint32_t)xx);
+            if (s != -1) {
+                if (first == -1) first = s;
+                last = __ldg(cend + base + (uint32_t)xx);
+            }
+        }
+    }
+    if (!check_ok(c, first == -1 ||
+                         (first >= 0 && first <= last && (uint32_t)last <= c.n_total)))
+        first = -1;
+    return first == -1 ? make_int2(0, 0) : make_int2(first, last);
+}
+
 __device__ __forceinline__ void runs_of(int3 ctr, const DevConsts& c,
                                         const int32_t* __restrict__ cstart,
                                         const int32_t* __restrict__ cend, Runs& r) {
-    const uint32_t Gx = c.Gi[0], Gy = c.Gi[1], Gz = c.Gi[2];
-    const int cx = ctr.x, cy = ctr.y, cz = ctr.z;
-    const int xlo = cx > 0 ? cx - 1 : 0;
-    const int xhi = cx + 1 < (int)Gx ? cx + 1 : (int)Gx - 1;
 #pragma unroll
     for (int o = 0; o < 9; ++o) {
-        const int ny = cy + (o / 3) - 1, nz = cz + (o % 3) - 1;
-        int32_t first = -1, last = -1;
-        if (ny >= 0 && ny < (int)Gy && nz >= 0 && nz < (int)Gz) {
-            const uint32_t base = c.cell_base + (uint32_t)ny * c.GxGz + (uint32_t)nz * Gx;
-            for (int xx = xlo; xx <= xhi; ++xx) {
-                const int32_t s = __ldg(cstart + base + (uint32_t)xx);
-                if (s != -1) {
-                    if (first == -1) first = s;
-                    last = __ldg(cend + base + (uint32_t)xx);
-                }
-            }
-        }
-        if (!check_ok(c, first == -1 || (first >= 0 && first <= last &&
-                                          (uint32_t)last <= c.n_total)))
-            first = -1;
-        r.b[o] = first == -1 ? 0 : first;
-        r.e[o] = first == -1 ? 0 : last;
+        const int2 be = run_of_row(o, ctr, c, cstart, cend);
+        r.b[o] = be.x;
+        r.e[o] = be.y;
     }
 }
-
 
 // `ctr` returns the stencil centre (stencil_centre of the sweep's predicted
 // position): the visits call it where they build the runs, so no centre stays

@@ -623,52 +623,281 @@ k_delta_p(const float4* __restrict__ L, const float4* __restrict__ XP,
 //
 // One warp per sorted particle i, for scenes too small to fill the GPU with a
 // thread per particle (and for clumped states, where each particle has
-// thousands of neighbours): the lanes test 32 consecutive candidates of a run
-// at once (coalesced loads), each in-range lane computes its pair term, and
-// every lane then folds the terms into the particle's sums in ascending
-// candidate order, reading them from the owning lanes by shuffles.  The terms
-// are the same functions and the folding order the same visit order as the
-// one-thread sweeps, so the bits are the same.
+// thousands of neighbours).  The warp's 32 lanes walk the 9 stencil rows as
+// one flattened candidate sequence (visit order), 32 candidates per step:
+//  1. every lane tests its candidate; the in-range ones are appended, in
+//     order, to a queue in shared memory (offset d and one payload word);
+//  2. when 32 are queued, every lane evaluates one pair and stores its terms
+//     in shared memory, one row per term component;
+//  3. lane c folds component c of the 32 terms into the particle's sum, in
+//     order, four terms per shared-memory load.
+// The terms are the same functions and the folding order the same visit order
+// as the one-thread sweeps, so the bits are the same.
+//
+// What bounds it: instruction issue.  Evaluating a pair on the lane that found
+// it and folding it on all lanes from shuffles spends ~14 instructions per
+// term for the fold and an evaluation per 32-candidate step whatever the number
+// in range (5 of 32 in a lattice at rest); queued, a full batch costs ~80
+// instructions of evaluation and ~45 of folding for 32 terms.  The stencil
+// rows are found by 9 lanes at once instead of by every lane in turn.
+// Measured per launch against the shuffled fold.  16,384 particles at rest:
+// lambda 30.6 -> 17.9 us, delta-p 30.2 -> 18.2, vorticity 36.7 -> 22.2 and
+// 28.0 -> 19.4; ncu: 900 warp instructions per particle, issue slots 65% busy
+// (the grid is 2.7 waves).  The same scene collapsed (substep 96): lambda
+// 2,043 -> 221 us, the first vorticity pass 2,368 -> 386.  The heavy particles
+// of 2,097,152 (20 substeps): lambda 287 -> 81 us, delta-p 114 -> 60.  Blocks
+// of 2 warps instead of 8 measured the same.
+//
+// Piles of coincident particles: a step whose 32 candidates all carry the same
+// offset and payload is not queued but counted, and a counted stretch is added
+// with repeat_step (repeat_add.h: the bits of the sequential sum).
 constexpr int kCoop = 3;
 constexpr uint32_t kFull = 0xFFFFFFFFu;
+// A step looks for equal candidates from this many stencil candidates up: below,
+// piles are too short to pay for the test (an interior particle of the lattice
+// at rest has 216 candidates).
+constexpr uint32_t kCoopRunsFrom = 256;
 
 __device__ __forceinline__ float shf(float v, int src) { return __shfl_sync(kFull, v, src); }
 __device__ __forceinline__ float3 shf3(float3 v, int src) {
     return make_float3(shf(v.x, src), shf(v.y, src), shf(v.z, src));
 }
+__device__ __forceinline__ bool same_bits(float a, float b) {
+    return __float_as_uint(a) == __float_as_uint(b);
+}
+__device__ __forceinline__ bool same_bits3(float3 a, float3 b) {
+    return same_bits(a.x, b.x) && same_bits(a.y, b.y) && same_bits(a.z, b.z);
+}
 
-// Calls term(j, d, r2) on every in-range candidate's own lane (returning
-// whether the candidate has a term), then fold(src_lane) on all lanes for
-// each in-range candidate with a term, in visit order.
-template <class Ctr, class T, class Fo>
-__device__ __forceinline__ void coop_visit(uint32_t i, Ctr&& ctr, const DevConsts& c,
-                                           const int32_t* __restrict__ cstart,
-                                           const int32_t* __restrict__ cend,
-                                           const float4* __restrict__ X, float3 pi, T&& term,
-                                           Fo&& fold) {
-    const uint32_t lane = threadIdx.x & 31u;
-    Runs r;
-    runs_of(ctr(), c, cstart, cend, r);
-#pragma unroll 1
-    for (int o = 0; o < 9; ++o) {
-        const int32_t e = r.e[o];
-#pragma unroll 1
-        for (int32_t base = r.b[o]; base < e; base += 32) {
-            const uint32_t j = (uint32_t)base + lane;
-            bool has = false;
-            if ((int32_t)j < e && j != i) {
-                const float3 d = sub3(pi, xyz(__ldg(X + j)));
-                const float r2 = dot3(d, d);
-                if (!(r2 > c.r2cut)) has = term(j, d, r2);
-            }
-            uint32_t m = __ballot_sync(kFull, has);
-            while (m) {
-                const int src = __ffs(m) - 1;
-                m &= m - 1;
-                fold(src);
+// A warp's share of shared memory.  Term rows are 36 floats apart, so that the
+// 16-byte loads of up to 8 rows at one column fall in different banks.
+constexpr int kCoopRows = 8;
+struct CoopShared {
+    float4 queue[64];
+    float t[kCoopRows][36];
+    int2 run[10];
+};
+
+// The pair terms of each sweep.  kRows term rows; lane c < kSums keeps sum c,
+// acc <- fma(row s_row(c), row a_row(c), acc), or acc + row a_row(c) where
+// kAdd.  kSkipCoincident: a candidate at distance 0 has no term.  payload() is
+// the word queued with a candidate, same() whether two payloads give the same
+// term.
+struct CoopLambda {
+    static constexpr int kRows = 5, kSums = 5;
+    static constexpr bool kAdd = true, kSkipCoincident = false;
+    static __device__ __forceinline__ int s_row(int) { return 0; }
+    static __device__ __forceinline__ int a_row(int c) { return c; }
+    __device__ __forceinline__ float payload(uint32_t, float4) const { return 0.0f; }
+    __device__ __forceinline__ bool same(float, float) const { return true; }
+    __device__ __forceinline__ void terms(const DevConsts& c, float3 d, float r2, float,
+                                          float* t) const {
+        const float len = fsqrt(r2);
+        t[0] = w_poly6(c, len);  // calclambda.glsl:80-82
+        // a coincident candidate adds no gradient (:60); +0 leaves the other
+        // four sums as they are (they start at +0, so none is ever -0)
+        float3 g = make_float3(0.0f, 0.0f, 0.0f);
+        if (len != 0.0f) g = scale3(d, grad_scale(c.kg_lambda, c.h, len));  // :86-87
+        t[1] = dot3(g, g);                                                   // :89
+        t[2] = g.x;                                                          // :93
+        t[3] = g.y;
+        t[4] = g.z;
+    }
+};
+struct CoopDeltaP {
+    static constexpr int kRows = 4, kSums = 3;
+    static constexpr bool kAdd = false, kSkipCoincident = true;
+    float li;
+    static __device__ __forceinline__ int s_row(int) { return 0; }
+    static __device__ __forceinline__ int a_row(int c) { return 1 + c; }
+    __device__ __forceinline__ float payload(uint32_t, float4 Lj) const { return Lj.w; }
+    __device__ __forceinline__ bool same(float a, float b) const { return same_bits(a, b); }
+    __device__ __forceinline__ void terms(const DevConsts& c, float3 d, float r2, float lj,
+                                          float* t) const {
+        const float len = fsqrt(r2);
+        float sc = fmul(c.scale, w_poly6(c, len));  // updatepos.glsl:57
+        sc = fmul(sc, sc);                           // :58
+        sc = fmul(sc, sc);                           // :59
+        sc = fmul(c.negk, sc);                       // :60
+        t[0] = fadd(fadd(li, lj), sc);               // :65
+        const float3 g = scale3(d, grad_scale(c.kg, c.h, len));
+        t[1] = g.x;
+        t[2] = g.y;
+        t[3] = g.z;
+    }
+};
+struct CoopVortA {
+    static constexpr int kRows = 8, kSums = 6;
+    static constexpr bool kAdd = false, kSkipCoincident = false;
+    const float4* __restrict__ VS;
+    float3 vi;
+    // sums 0-2 (XSPH) scale by row 0, sums 3-5 (vorticity) by row 1 (ones:
+    // fma(1, a, acc) is the rounded acc + a)
+    static __device__ __forceinline__ int s_row(int c) { return c < 3 ? 0 : 1; }
+    static __device__ __forceinline__ int a_row(int c) { return 2 + c; }
+    __device__ __forceinline__ float payload(uint32_t j, float4) const {
+        return __uint_as_float(j);
+    }
+    __device__ __forceinline__ bool same(float a, float b) const {
+        return same_bits3(xyz(__ldg(VS + __float_as_uint(a))), xyz(__ldg(VS + __float_as_uint(b))));
+    }
+    __device__ __forceinline__ void terms(const DevConsts& c, float3 d, float r2, float j,
+                                          float* t) const {
+        const float len = fsqrt(r2);
+        const float3 v = sub3(xyz(__ldg(VS + __float_as_uint(j))), vi);  // vorticity.glsl:50
+        t[0] = w_poly6(c, len);                                           // :52-54
+        t[1] = 1.0f;
+        t[2] = v.x;
+        t[3] = v.y;
+        t[4] = v.z;
+        // (a coincident candidate adds no curl; +0 keeps a sum that starts at +0)
+        float3 w = make_float3(0.0f, 0.0f, 0.0f);
+        if (len != 0.0f) w = cross3(v, scale3(d, grad_scale(c.kg, c.h, len)));  // :55
+        t[5] = w.x;
+        t[6] = w.y;
+        t[7] = w.z;
+    }
+};
+struct CoopVortB {
+    static constexpr int kRows = 4, kSums = 3;
+    static constexpr bool kAdd = false, kSkipCoincident = true;
+    static __device__ __forceinline__ int s_row(int) { return 0; }
+    static __device__ __forceinline__ int a_row(int c) { return 1 + c; }
+    __device__ __forceinline__ float payload(uint32_t, float4 Qj) const { return Qj.w; }
+    __device__ __forceinline__ bool same(float a, float b) const { return same_bits(a, b); }
+    __device__ __forceinline__ void terms(const DevConsts& c, float3 d, float r2, float qj,
+                                          float* t) const {
+        t[0] = qj;  // vorticity.glsl:72
+        const float3 g = scale3(d, grad_scale(c.kg, c.h, fsqrt(r2)));
+        t[1] = g.x;
+        t[2] = g.y;
+        t[3] = g.z;
+    }
+};
+
+// Sweeps particle i's stencil around `ctr` with one warp (every lane calls);
+// lane c < Op::kSums returns sum c, the other lanes sum 0.
+template <class Op>
+__device__ __forceinline__ float coop_visit(uint32_t i, int3 ctr, const DevConsts& c,
+                                            const int32_t* __restrict__ cstart,
+                                            const int32_t* __restrict__ cend,
+                                            const float4* __restrict__ X, float3 pi,
+                                            CoopShared& sm, const Op& op) {
+    const int lane = (int)(threadIdx.x & 31u);
+    const uint32_t before = (1u << lane) - 1u;
+    int2 mine = make_int2(0, lane == 9 ? 0x7FFFFFFF : 0);  // row 9 ends the sequence
+    if (lane < 9) mine = run_of_row(lane, ctr, c, cstart, cend);
+    if (lane < 10) sm.run[lane] = mine;
+    const bool look = __reduce_add_sync(kFull, lane < 9 ? (uint32_t)(mine.y - mine.x) : 0u) >=
+                      kCoopRunsFrom;
+    const int sum = lane < Op::kSums ? lane : 0;
+    const float* const arow = sm.t[Op::a_row(sum)];
+    const float* const srow = sm.t[Op::s_row(sum)];
+    float acc = 0.0f;
+    uint32_t qn = 0, qh = 0;  // queued candidates; the queue's head (0 or 32)
+    // a stretch of `pm` equal candidates waiting to be added (the queue is then empty)
+    uint32_t pm = 0;
+    float3 pd = make_float3(0.0f, 0.0f, 0.0f);
+    float pp = 0.0f;
+    __syncwarp();
+
+    auto batch = [&](uint32_t cnt) {  // evaluate and fold the queue's first cnt (<= 32)
+        if ((uint32_t)lane < cnt) {
+            const float4 e = sm.queue[qh + lane];
+            const float3 d = xyz(e);
+            float t[Op::kRows];
+            op.terms(c, d, dot3(d, d), e.w, t);
+#pragma unroll
+            for (int k = 0; k < Op::kRows; ++k) sm.t[k][lane] = t[k];
+        }
+        __syncwarp();
+        uint32_t k = 0;
+#pragma unroll 2
+        for (; k + 4 <= cnt; k += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(arow + k);
+            if constexpr (Op::kAdd) {
+                acc = fadd(fadd(fadd(fadd(acc, a.x), a.y), a.z), a.w);
+            } else {
+                const float4 s = *reinterpret_cast<const float4*>(srow + k);
+                acc = ffma(s.w, a.w, ffma(s.z, a.z, ffma(s.y, a.y, ffma(s.x, a.x, acc))));
             }
         }
+        for (; k < cnt; ++k) acc = Op::kAdd ? fadd(acc, arow[k]) : ffma(srow[k], arow[k], acc);
+        __syncwarp();
+    };
+    auto add_stretch = [&] {  // pm equal candidates in a row
+        float t[Op::kRows];
+        op.terms(c, pd, dot3(pd, pd), pp, t);
+        if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < Op::kRows; ++k) sm.t[k][0] = t[k];
+        }
+        __syncwarp();
+        const float a = arow[0], s = srow[0];
+        if constexpr (Op::kAdd)
+            acc = repeat_add(acc, a, pm);
+        else
+            acc = repeat_step(acc, pm, [s, a](float x) { return ffma(s, a, x); });
+        pm = 0;
+        __syncwarp();
+    };
+
+    int row = 0;
+    int2 be = sm.run[0];
+    int j = be.x + lane;
+    for (;; j += 32) {
+        while (j >= be.y && row < 9) {  // past its row: the lane goes on in the next one
+            const int over = j - be.y;
+            be = sm.run[++row];
+            j = be.x + over;
+        }
+        const bool valid = row < 9;
+        if (!__any_sync(kFull, valid)) break;
+        float3 d = make_float3(0.0f, 0.0f, 0.0f);
+        float r2 = 0.0f, pay = 0.0f;
+        bool in = false;
+        if (valid) {
+            const float4 xj = __ldg(X + j);
+            d = sub3(pi, xyz(xj));
+            r2 = dot3(d, d);
+            pay = op.payload((uint32_t)j, xj);
+            in = !(r2 > c.r2cut) && (uint32_t)j != i && !(Op::kSkipCoincident && r2 == 0.0f);
+        }
+        const uint32_t m = __ballot_sync(kFull, in);
+        if (m == 0u) continue;
+        // all 32 candidates equal (the particle itself may be one of them)?
+        if (look) {
+            const float r20 = shf(r2, 0);
+            if (__all_sync(kFull, valid && r2 == r20)) {
+                const float3 d0 = shf3(d, 0);
+                const float p0 = shf(pay, 0);
+                if (__all_sync(kFull, same_bits3(d, d0) && op.same(pay, p0))) {
+                    if (pm == 0u || !(same_bits3(pd, d0) && op.same(pp, p0))) {
+                        if (pm) add_stretch();
+                        if (qn) batch(qn);
+                        qn = 0;
+                        pd = d0;
+                        pp = p0;
+                    }
+                    pm += (uint32_t)__popc(m);
+                    continue;
+                }
+            }
+        }
+        if (pm) add_stretch();
+        if (in) sm.queue[(qh + qn + (uint32_t)__popc(m & before)) & 63u] =
+            make_float4(d.x, d.y, d.z, pay);
+        qn += (uint32_t)__popc(m);
+        __syncwarp();
+        if (qn >= 32u) {
+            batch(32u);
+            qh ^= 32u;
+            qn -= 32u;
+        }
     }
+    if (pm) add_stretch();
+    if (qn) batch(qn);
+    return acc;
 }
 
 // Particles a cooperative kernel processes: all n (list == nullptr, one warp
@@ -680,6 +909,8 @@ struct CoopWork {
 };
 
 #define PBF_COOP_FOR_EACH(i)                                                                  \
+    __shared__ CoopShared shared_[kBlock / 32];                                               \
+    CoopShared& sm = shared_[threadIdx.x >> 5];                                               \
     const uint32_t warp0_ = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;                     \
     const uint32_t nwarps_ = (gridDim.x * blockDim.x) >> 5;                                    \
     const uint32_t total_ = wk.list ? *wk.count : n;                                           \
@@ -694,32 +925,9 @@ k_lambda_coop(const float4* __restrict__ P, const float4* __restrict__ XP,
     PBF_COOP_FOR_EACH(i) {
         const auto& c = cp.at(i);
         const float3 pi = xyz(P[i]);
-        auto ctr = [&] { return stencil_centre(XP[i], c); };  // neighbourcells.glsl:57
-        LambdaAcc a{0.0f, 0.0f, make_float3(0.0f, 0.0f, 0.0f)};
-        float tw = 0.0f, tgg = 0.0f;
-        float3 tg = make_float3(0.0f, 0.0f, 0.0f);
-        bool tgrad = false;
-        coop_visit(i, ctr, c, cstart, cend, P, pi,
-                   [&](uint32_t, float3 d, float r2) {
-                       const float len = fsqrt(r2);
-                       tw = w_poly6(c, len);
-                       tgrad = len != 0.0f;
-                       if (tgrad) {
-                           tg = scale3(d, grad_scale(c.kg_lambda, c.h, len));
-                           tgg = dot3(tg, tg);
-                       }
-                       return true;
-                   },
-                   [&](int src) {
-                       a.rho = fadd(a.rho, shf(tw, src));  // calclambda.glsl:80-82
-                       const bool g = __shfl_sync(kFull, tgrad, src);
-                       const float gg = shf(tgg, src);
-                       const float3 gv = shf3(tg, src);
-                       if (g) {
-                           a.sumk = fadd(a.sumk, gg);  // :89
-                           a.gi = add3(a.gi, gv);       // :93
-                       }
-                   });
+        const float s = coop_visit(i, stencil_centre(XP[i], c), c, cstart, cend, P, pi, sm,
+                                   CoopLambda{});  // neighbourcells.glsl:57
+        const LambdaAcc a{shf(s, 0), shf(s, 1), make_float3(shf(s, 2), shf(s, 3), shf(s, 4))};
         if ((threadIdx.x & 31u) == 0u) {
             L[i] = make_float4(pi.x, pi.y, pi.z, lambda_finish(c, a));
             if (aux) aux[i] = lambda_aux(a);
@@ -737,24 +945,9 @@ k_delta_p_coop(const float4* __restrict__ L, const float4* __restrict__ XP,
         const auto& c = cp.at(i);
         const float4 Li = L[i];
         const float3 pi = xyz(Li);
-        const float li = Li.w;
-        auto ctr = [&] { return stencil_centre(XP[i], c); };  // neighbourcells.glsl:57
-        float3 dp = make_float3(0.0f, 0.0f, 0.0f);
-        float tcoef = 0.0f;
-        float3 tg = make_float3(0.0f, 0.0f, 0.0f);
-        coop_visit(i, ctr, c, cstart, cend, L, pi,
-                   [&](uint32_t j, float3 d, float r2) {
-                       const float len = fsqrt(r2);
-                       if (len == 0.0f) return false;
-                       float sc = fmul(c.scale, w_poly6(c, len));  // updatepos.glsl:57
-                       sc = fmul(sc, sc);                           // :58
-                       sc = fmul(sc, sc);                           // :59
-                       sc = fmul(c.negk, sc);                       // :60
-                       tcoef = fadd(fadd(li, __ldg(L + j).w), sc);  // :65
-                       tg = scale3(d, grad_scale(c.kg, c.h, len));
-                       return true;
-                   },
-                   [&](int src) { dp = fma3(shf(tcoef, src), shf3(tg, src), dp); });  // :65
+        const float s = coop_visit(i, stencil_centre(XP[i], c), c, cstart, cend, L, pi, sm,
+                                   CoopDeltaP{Li.w});  // neighbourcells.glsl:57
+        const float3 dp = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
         if ((threadIdx.x & 31u) == 0u) {
             float3 q = fma3(c.oorho, dp, pi);  // :85
             q.x = (q.x < c.lo[0]) ? c.lo[0] : q.x;
@@ -781,26 +974,10 @@ k_vorticity_a_coop(const float4* __restrict__ P, const float4* __restrict__ VS,
         const auto& c = cp.at(i);
         const float3 pi = xyz(P[i]);
         const float3 vi = xyz(VS[i]);
-        auto ctr = [&] { return stencil_centre(XP[i], c); };  // neighbourcells.glsl:57
-        float3 acc = make_float3(0.0f, 0.0f, 0.0f), w = make_float3(0.0f, 0.0f, 0.0f);
-        float tw = 0.0f;
-        float3 tv = make_float3(0.0f, 0.0f, 0.0f), tc = make_float3(0.0f, 0.0f, 0.0f);
-        bool tgrad = false;
-        coop_visit(i, ctr, c, cstart, cend, P, pi,
-                   [&](uint32_t j, float3 d, float r2) {
-                       const float len = fsqrt(r2);
-                       tv = sub3(xyz(__ldg(VS + j)), vi);  // vorticity.glsl:50
-                       tw = w_poly6(c, len);
-                       tgrad = len != 0.0f;
-                       if (tgrad) tc = cross3(tv, scale3(d, grad_scale(c.kg, c.h, len)));  // :55
-                       return true;
-                   },
-                   [&](int src) {
-                       acc = fma3(shf(tw, src), shf3(tv, src), acc);  // :52-54
-                       const bool g = __shfl_sync(kFull, tgrad, src);
-                       const float3 cv = shf3(tc, src);
-                       if (g) w = add3(w, cv);  // :55
-                   });
+        const float s = coop_visit(i, stencil_centre(XP[i], c), c, cstart, cend, P, pi, sm,
+                                   CoopVortA{VS, vi});  // neighbourcells.glsl:57
+        const float3 acc = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
+        const float3 w = make_float3(shf(s, 3), shf(s, 4), shf(s, 5));
         if ((threadIdx.x & 31u) == 0u) {
             const float3 vx = fma3(c.cx, acc, vi);  // :58
             VX[i] = make_float4(vx.x, vx.y, vx.z, 0.0f);
@@ -820,19 +997,9 @@ k_vorticity_b_coop(const float4* __restrict__ Q, const float4* __restrict__ VX,
     PBF_COOP_FOR_EACH(i) {
         const auto& c = cp.at(i);
         const float3 pi = xyz(Q[i]);
-        auto ctr = [&] { return stencil_centre(XP[i], c); };  // neighbourcells.glsl:57
-        float3 eta = make_float3(0.0f, 0.0f, 0.0f);
-        float tq = 0.0f;
-        float3 tg = make_float3(0.0f, 0.0f, 0.0f);
-        coop_visit(i, ctr, c, cstart, cend, Q, pi,
-                   [&](uint32_t j, float3 d, float r2) {
-                       const float len = fsqrt(r2);
-                       if (len == 0.0f) return false;
-                       tq = __ldg(Q + j).w;
-                       tg = scale3(d, grad_scale(c.kg, c.h, len));
-                       return true;
-                   },
-                   [&](int src) { eta = fma3(shf(tq, src), shf3(tg, src), eta); });  // vorticity.glsl:72
+        const float s = coop_visit(i, stencil_centre(XP[i], c), c, cstart, cend, Q, pi, sm,
+                                   CoopVortB{});  // neighbourcells.glsl:57
+        float3 eta = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
         if ((threadIdx.x & 31u) == 0u) {
             if (eta_out) eta_out[i] = make_float4(eta.x, eta.y, eta.z, 0.0f);
             const float l = fsqrt(dot3(eta, eta));  // :76
