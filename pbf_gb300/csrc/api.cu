@@ -230,6 +230,16 @@ bool mixed_on(const pbf_sim* s) {
     const bool vort = s->params.vorticity_confinement != 0;
     return pass_mixed(s, s->pass_solver) || (vort && pass_mixed(s, s->pass_vort));
 }
+// Whether some sweep of the substep reads the stencil rows: the direct sweeps
+// alone walk the cells themselves.
+bool rows_on(const pbf_sim* s) {
+    auto reads = [&](uint32_t pass) {
+        const PassModes m = modes_of(s, pass);
+        return m.first != 0 || m.second != 0;
+    };
+    return mixed_on(s) || reads(s->pass_solver) ||
+           (s->params.vorticity_confinement != 0 && reads(s->pass_vort));
+}
 uint32_t heavy_threshold(const pbf_sim* s) {
     return s->tuning.coop_candidates ? s->tuning.coop_candidates : kMixedCandidates;
 }
@@ -313,7 +323,7 @@ void free_sim(pbf_sim* s) {
                     s->cstart, s->cend, s->status, s->sort_mem, s->nbr_idx, s->nbr_cnt,
                     s->guard, s->d_consts, s->sid, s->sid_sorted, s->pair_idx, s->pair_cnt,
                     s->scan_xy, s->scan_z, s->heavy, s->heavy_list, s->heavy_count,
-                    s->runs};
+                    s->runs, s->rows};
     for (void* b : bufs)
         if (b) cudaFree(b);
     if (s->h_status) cudaFreeHost(s->h_status);
@@ -342,9 +352,9 @@ uint32_t kernels_per_substep(const pbf_sim* s) {
         if (!lists) k += iters * (a.second == 0 ? 1u : 0u);
         if (!lists && vort) k += (b.first == 0 ? 1u : 0u) + (b.second == 0 ? 1u : 0u);
     }
-    if (mixed_on(s)) {  // the flag pass and a cooperative launch after each one-thread sweep
+    if (rows_on(s)) k += 1u;
+    if (mixed_on(s)) {  // a cooperative launch after each one-thread sweep
         const PassModes a = modes_of(s, s->pass_solver), b = modes_of(s, s->pass_vort);
-        k += 1u;
         if (pass_mixed(s, s->pass_solver)) k += iters * ((a.first != 3) + (a.second != 3));
         if (vort && pass_mixed(s, s->pass_vort)) k += (uint32_t)((b.first != 3) + (b.second != 3));
     }
@@ -496,21 +506,24 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
     if (e != cudaSuccess) return e;
     mark(2);
     // 3 cell ranges (NeighbourCellFinder::FindNeighbourCells)
-    const size_t half = ((size_t)n + 1) / 2;
-    auto scan_set = [&](int k) { return ScanPos{s->scan_xy + k * half, s->scan_z + k * half}; };
+    const size_t pairs = scan_pairs(n);
+    auto scan_set = [&](int k) { return ScanPos{s->scan_xy + k * pairs, s->scan_z + k * pairs}; };
     // (over n + 1 threads: the run-start bits end with a terminator at n)
     k_find_cells<<<grid_for(n + 1), kBlock, 0, st>>>(s->skeys, s->perm, s->xstar, s->XP, n,
                                                      s->ncells, s->cstart, s->cend, s->status + 1,
                                                      s->sid, s->sid_sorted, scan_set(0), s->runs,
                                                      s->status);
-    // mixed sweeps: flag the particles with more than coop_candidates stencil
-    // candidates; the cooperative kernels sweep those, the others skip them
+    // the stencil rows the masked and cooperative sweeps read; with mixed
+    // sweeps also the particles with more than coop_candidates stencil
+    // candidates: the cooperative kernels sweep those, the others skip them
     const bool mixed = mixed_on(s);
-    if (mixed) {
-        cudaError_t me = cudaMemsetAsync(s->heavy_count, 0, sizeof(uint32_t), st);
-        if (me != cudaSuccess) return me;
-        launch_heavy_scan(g, st, s->XP, s->cstart, s->cend, heavy_threshold(s), n, cps,
-                          s->heavy, s->heavy_list, s->heavy_count);
+    if (rows_on(s)) {
+        if (mixed) {
+            cudaError_t me = cudaMemsetAsync(s->heavy_count, 0, sizeof(uint32_t), st);
+            if (me != cudaSuccess) return me;
+        }
+        launch_stencil_rows(g, st, s->XP, s->cstart, s->cend, heavy_threshold(s), n, cps, s->rows,
+                            mixed ? s->heavy : nullptr, s->heavy_list, s->heavy_count);
     }
     mark(3);
     // 4 solver iterations (calclambda / updatepos).  The first lambda sweep
@@ -531,7 +544,7 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
     const bool mix_v = mixed && pass_mixed(s, s->pass_vort);
     const PairLists pl{s->pair_idx, s->pair_cnt, s->pair_cap, n, mix_s ? s->heavy : nullptr,
                        s->heavy_list, s->heavy_count,
-                       runs_solver || runs_vort ? s->runs : nullptr};
+                       runs_solver || runs_vort ? s->runs : nullptr, s->rows};
     PairLists pl_v = pl;
     pl_v.heavy = mix_v ? s->heavy : nullptr;
     cudaError_t ge = cudaMemsetAsync(s->guard, 0, sizeof(uint32_t) * (2 + iters), st);
@@ -699,8 +712,9 @@ pbf_status pbf_create_batch(const pbf_params* scene_params, const uint32_t* scen
     ALLOC(x, n) ALLOC(v, n) ALLOC(xstar, n) ALLOC(XP, n) ALLOC(Pa, n) ALLOC(Pb, n) ALLOC(L, n)
     ALLOC(VS, n) ALLOC(VX, n) ALLOC(OM, n) ALLOC(Q, n) ALLOC(keys, n) ALLOC(skeys, n)
     ALLOC(perm, n) ALLOC(cstart, s->ncells) ALLOC(cend, s->ncells) ALLOC(status, 2)
-    ALLOC(scan_xy, 3 * (((size_t)n + 1) / 2)) ALLOC(scan_z, 3 * (((size_t)n + 1) / 2))
+    ALLOC(scan_xy, 3 * scan_pairs(n)) ALLOC(scan_z, 3 * scan_pairs(n))
     ALLOC(heavy, n) ALLOC(heavy_list, n) ALLOC(heavy_count, 1) ALLOC(runs, (size_t)n / 32 + 2)
+    ALLOC(rows, 9 * (size_t)n)
     if (num_scenes > 1) {
         ALLOC(d_consts, num_scenes) ALLOC(sid, n) ALLOC(sid_sorted, n)
     }

@@ -93,16 +93,21 @@ struct PairLists {
     // run-start bits of the sweep's position set (neighbours.cuh: runs), read
     // by the direct sweeps' coincident runs; NULL: no run path
     const uint32_t* runs = nullptr;
+    // the substep's stencil rows (k_stencil_rows): row o (0..8) of particle i
+    // at rows[o * n + i], read by the masked and the cooperative sweeps
+    const int2* rows = nullptr;
 };
 
 // Scan copy of a sorted position array, read by the masked stencil scans two
 // candidates at a time with packed (float2) arithmetic: x and y of the
 // particle pair (2q, 2q+1) interleaved in xy[q] = (x0, x1, y0, y1), z as a
-// plain array read as the float2 z[q] = (z0, z1).  (n + 1) / 2 entries each.
+// plain array read as the float2 z[q] = (z0, z1).  scan_pairs(n) entries each:
+// a scan reads two pairs at a time, so one pair past the last is allocated.
 struct ScanPos {
     float4* xy;
     float2* z;
 };
+inline size_t scan_pairs(uint32_t n) { return ((size_t)n + 1) / 2 + 1; }
 
 __device__ __forceinline__ void scanpos_store(const ScanPos& sp, uint32_t i, float x, float y,
                                               float z) {

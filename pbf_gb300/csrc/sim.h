@@ -61,11 +61,12 @@ struct pbf_sim {
     uint8_t* heavy = nullptr;
     uint32_t* heavy_list = nullptr;
     uint32_t* heavy_count = nullptr;
+    int2* rows = nullptr;  // [9][n] the substep's stencil rows (k_stencil_rows)
     // run-start bits of the position set the direct sweeps read (k_find_cells,
     // k_run_flags), n / 32 + 2 words
     uint32_t* runs = nullptr;
     // scan copies (ScanPos) of the predicted positions (set 0) and of the
-    // solver iterates (sets 1 and 2, alternating), (n + 1) / 2 pairs per set
+    // solver iterates (sets 1 and 2, alternating), scan_pairs(n) pairs per set
     float4* scan_xy = nullptr;
     float2* scan_z = nullptr;
     uint32_t* h_status = nullptr;

@@ -263,10 +263,10 @@ __device__ __forceinline__ void warp_max_to(uint32_t* slot, float v) {
 template <bool MASKED, class Ctr, class F>
 __device__ __forceinline__ void sweep_visit(uint32_t i, Ctr&& ctr, const DevConsts& c,
                                             const int32_t* __restrict__ cstart,
-                                            const int32_t* __restrict__ cend, const ScanPos& X,
-                                            float3 pi, F&& body) {
+                                            const int32_t* __restrict__ cend, const PairLists& pl,
+                                            const ScanPos& X, float3 pi, F&& body) {
     if constexpr (MASKED)
-        visit_masked<false>(i, ctr, c, cstart, cend, X, pi, [](int32_t, uint32_t) {}, body);
+        visit_masked<false>(i, c, pl.rows, pl.n, X, pi, [](int32_t, uint32_t) {}, body);
     else
         visit_full(i, ctr, c, cstart, cend, body);
 }
@@ -278,17 +278,16 @@ __device__ __forceinline__ void sweep_visit(uint32_t i, Ctr&& ctr, const DevCons
 // together over their own list positions (the same shape as the replaying
 // sweeps) instead of chunk by chunk.  A list longer than its capacity keeps
 // its first `cap` entries (and is marked -1 for the replaying sweep); the
-// candidates past them are found by a second scan and evaluated in order.
-template <bool LIST, class Ctr, class S, class F>
-__device__ __forceinline__ void scan_then_eval(uint32_t i, Ctr&& ctr, const DevConsts& c,
-                                               const int32_t* __restrict__ cstart,
-                                               const int32_t* __restrict__ cend,
-                                               const ScanPos& X, float3 pi, const PairLists& pw,
-                                               S&& list, F&& eval) {
+// candidates past them are found by walking the rows again, `near(j)` being
+// the in-range test, and evaluated in order.
+template <bool LIST, class S, class N, class F>
+__device__ __forceinline__ void scan_then_eval(uint32_t i, const DevConsts& c, const ScanPos& X,
+                                               float3 pi, const PairLists& pw, S&& list, N&& near,
+                                               F&& eval) {
     uint32_t* const out = pw.idx + i;
     const size_t stride = pw.n;
     uint32_t tot = 0;
-    visit_masked<LIST>(i, ctr, c, cstart, cend, X, pi, list, [&](uint32_t j) {
+    visit_masked<LIST>(i, c, pw.rows, pw.n, X, pi, list, [&](uint32_t j) {
         if (tot < pw.cap) out[(size_t)tot * stride] = j;
         ++tot;
     });
@@ -305,10 +304,13 @@ __device__ __forceinline__ void scan_then_eval(uint32_t i, Ctr&& ctr, const DevC
     }
     if (tot > pw.cap) {
         uint32_t rank = 0;
-        visit_masked<false>(i, ctr, c, cstart, cend, X, pi, [](int32_t, uint32_t) {},
-                            [&](uint32_t j) {
-                                if (rank++ >= pw.cap) eval(j);
-                            });
+#pragma unroll 1
+        for (int o = 0; o < 9; ++o) {
+            const int2 be = __ldg(pw.rows + (size_t)o * pw.n + i);
+#pragma unroll 1
+            for (int32_t j = be.x; j < be.y; ++j)
+                if ((uint32_t)j != i && near((uint32_t)j) && rank++ >= pw.cap) eval((uint32_t)j);
+        }
     }
 }
 
@@ -411,18 +413,20 @@ k_lambda_build(const float4* __restrict__ XP, const uint32_t* __restrict__ skeys
             const float3 d = sub3(pi, xyz(__ldg(XP + j)));
             lambda_pair(c, d, dot3(d, d), a);
         };
+        auto near = [&](uint32_t j) {
+            const float3 d = sub3(pi, xyz(__ldg(XP + j)));
+            return !(dot3(d, d) > c.r2cut);
+        };
         if constexpr (MODE == kPairs) {
             if (LISTS && cap)
-                scan_then_eval<true>(i, ctr, c, cstart, cend, sx, pi, pw, list_rec, eval);
+                scan_then_eval<true>(i, c, sx, pi, pw, list_rec, near, eval);
             else
-                scan_then_eval<false>(i, ctr, c, cstart, cend, sx, pi, pw,
-                                      [](int32_t, uint32_t) {}, eval);
+                scan_then_eval<false>(i, c, sx, pi, pw, [](int32_t, uint32_t) {}, near, eval);
         } else if constexpr (MODE == kMasked) {
             if (LISTS && cap)
-                visit_masked<true>(i, ctr, c, cstart, cend, sx, pi, list_rec, eval);
+                visit_masked<true>(i, c, pw.rows, n, sx, pi, list_rec, eval);
             else
-                visit_masked<false>(i, ctr, c, cstart, cend, sx, pi,
-                                    [](int32_t, uint32_t) {}, eval);
+                visit_masked<false>(i, c, pw.rows, n, sx, pi, [](int32_t, uint32_t) {}, eval);
         } else {
             bool piles = false;
             if constexpr (!LISTS) {
@@ -486,6 +490,10 @@ k_lambda(const float4* __restrict__ P, const float4* __restrict__ XP,
         const float3 d = sub3(pi, xyz(__ldg(P + j)));
         lambda_pair(c, d, dot3(d, d), a);
     };
+    auto near = [&](uint32_t j) {
+        const float3 d = sub3(pi, xyz(__ldg(P + j)));
+        return !(dot3(d, d) > c.r2cut);
+    };
     auto eval = [&](uint32_t j) {
         const float3 d = sub3(pi, xyz(__ldg(P + j)));
         const float r2 = dot3(d, d);
@@ -512,10 +520,9 @@ k_lambda(const float4* __restrict__ P, const float4* __restrict__ XP,
     }
     if (!listed) {
         if constexpr (MODE == kPairs)
-            scan_then_eval<false>(i, ctr, c, cstart, cend, sx, pi, pw, [](int32_t, uint32_t) {},
-                                  eval_in);
+            scan_then_eval<false>(i, c, sx, pi, pw, [](int32_t, uint32_t) {}, near, eval_in);
         else if constexpr (MODE == kMasked)
-            sweep_visit<true>(i, ctr, c, cstart, cend, sx, pi, eval_in);
+            sweep_visit<true>(i, ctr, c, cstart, cend, pw, sx, pi, eval_in);
         else if (!LISTS && pw.runs)
             visit_direct_piles(
                 i, ctr, c, cstart, cend, pw.runs,
@@ -525,7 +532,7 @@ k_lambda(const float4* __restrict__ P, const float4* __restrict__ XP,
                     lambda_pair_run(c, d, r2, r - j0, a);
                 });
         else
-            sweep_visit<false>(i, ctr, c, cstart, cend, sx, pi, eval);
+            sweep_visit<false>(i, ctr, c, cstart, cend, pw, sx, pi, eval);
     }
     L[i] = make_float4(pi.x, pi.y, pi.z, lambda_finish(c, a));
     if (aux) aux[i] = lambda_aux(a);
@@ -596,7 +603,7 @@ k_delta_p(const float4* __restrict__ L, const float4* __restrict__ XP,
                             dp = repeat_fma3(coef, g, dp, r - j0);
                         });
                 else
-                    sweep_visit<MODE != kDirect>(i, ctr, c, cstart, cend, sx, pi, body);
+                    sweep_visit<MODE != kDirect>(i, ctr, c, cstart, cend, pr, sx, pi, body);
             }
         }
         float3 q = fma3(c.oorho, dp, pi);  // :85
@@ -775,18 +782,17 @@ struct CoopVortB {
     }
 };
 
-// Sweeps particle i's stencil around `ctr` with one warp (every lane calls);
+// Sweeps particle i's stencil with one warp (every lane calls);
 // lane c < Op::kSums returns sum c, the other lanes sum 0.
 template <class Op>
-__device__ __forceinline__ float coop_visit(uint32_t i, int3 ctr, const DevConsts& c,
-                                            const int32_t* __restrict__ cstart,
-                                            const int32_t* __restrict__ cend,
+__device__ __forceinline__ float coop_visit(uint32_t i, const DevConsts& c,
+                                            const int2* __restrict__ rows, uint32_t n,
                                             const float4* __restrict__ X, float3 pi,
                                             CoopShared& sm, const Op& op) {
     const int lane = (int)(threadIdx.x & 31u);
     const uint32_t before = (1u << lane) - 1u;
     int2 mine = make_int2(0, lane == 9 ? 0x7FFFFFFF : 0);  // row 9 ends the sequence
-    if (lane < 9) mine = run_of_row(lane, ctr, c, cstart, cend);
+    if (lane < 9) mine = __ldg(rows + (size_t)lane * n + i);
     if (lane < 10) sm.run[lane] = mine;
     const bool look = __reduce_add_sync(kFull, lane < 9 ? (uint32_t)(mine.y - mine.x) : 0u) >=
                       kCoopRunsFrom;
@@ -906,6 +912,7 @@ __device__ __forceinline__ float coop_visit(uint32_t i, int3 ctr, const DevConst
 struct CoopWork {
     const uint32_t* list;
     const uint32_t* count;
+    const int2* rows;  // PairLists::rows
 };
 
 #define PBF_COOP_FOR_EACH(i)                                                                  \
@@ -919,14 +926,12 @@ struct CoopWork {
 
 template <class CP>
 __global__ void __launch_bounds__(kBlock)
-k_lambda_coop(const float4* __restrict__ P, const float4* __restrict__ XP,
-              const int32_t* __restrict__ cstart, const int32_t* __restrict__ cend,
-              float4* __restrict__ L, float4* __restrict__ aux, uint32_t n, CP cp, CoopWork wk) {
+k_lambda_coop(const float4* __restrict__ P, float4* __restrict__ L, float4* __restrict__ aux,
+              uint32_t n, CP cp, CoopWork wk) {
     PBF_COOP_FOR_EACH(i) {
         const auto& c = cp.at(i);
         const float3 pi = xyz(P[i]);
-        const float s = coop_visit(i, stencil_centre(XP[i], c), c, cstart, cend, P, pi, sm,
-                                   CoopLambda{});  // neighbourcells.glsl:57
+        const float s = coop_visit(i, c, wk.rows, n, P, pi, sm, CoopLambda{});
         const LambdaAcc a{shf(s, 0), shf(s, 1), make_float3(shf(s, 2), shf(s, 3), shf(s, 4))};
         if ((threadIdx.x & 31u) == 0u) {
             L[i] = make_float4(pi.x, pi.y, pi.z, lambda_finish(c, a));
@@ -937,16 +942,13 @@ k_lambda_coop(const float4* __restrict__ P, const float4* __restrict__ XP,
 
 template <class CP>
 __global__ void __launch_bounds__(kBlock)
-k_delta_p_coop(const float4* __restrict__ L, const float4* __restrict__ XP,
-               const int32_t* __restrict__ cstart, const int32_t* __restrict__ cend,
-               float4* __restrict__ Pn, ScanPos sx_out, uint32_t n, CP cp, uint32_t* status,
-               CoopWork wk) {
+k_delta_p_coop(const float4* __restrict__ L, float4* __restrict__ Pn, ScanPos sx_out, uint32_t n,
+               CP cp, uint32_t* status, CoopWork wk) {
     PBF_COOP_FOR_EACH(i) {
         const auto& c = cp.at(i);
         const float4 Li = L[i];
         const float3 pi = xyz(Li);
-        const float s = coop_visit(i, stencil_centre(XP[i], c), c, cstart, cend, L, pi, sm,
-                                   CoopDeltaP{Li.w});  // neighbourcells.glsl:57
+        const float s = coop_visit(i, c, wk.rows, n, L, pi, sm, CoopDeltaP{Li.w});
         const float3 dp = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
         if ((threadIdx.x & 31u) == 0u) {
             float3 q = fma3(c.oorho, dp, pi);  // :85
@@ -966,16 +968,13 @@ k_delta_p_coop(const float4* __restrict__ L, const float4* __restrict__ XP,
 template <class CP>
 __global__ void __launch_bounds__(kBlock)
 k_vorticity_a_coop(const float4* __restrict__ P, const float4* __restrict__ VS,
-                   const float4* __restrict__ XP, const int32_t* __restrict__ cstart,
-                   const int32_t* __restrict__ cend, float4* __restrict__ VX,
-                   float4* __restrict__ OM, float4* __restrict__ Q, uint32_t n, CP cp,
-                   CoopWork wk) {
+                   float4* __restrict__ VX, float4* __restrict__ OM, float4* __restrict__ Q,
+                   uint32_t n, CP cp, CoopWork wk) {
     PBF_COOP_FOR_EACH(i) {
         const auto& c = cp.at(i);
         const float3 pi = xyz(P[i]);
         const float3 vi = xyz(VS[i]);
-        const float s = coop_visit(i, stencil_centre(XP[i], c), c, cstart, cend, P, pi, sm,
-                                   CoopVortA{VS, vi});  // neighbourcells.glsl:57
+        const float s = coop_visit(i, c, wk.rows, n, P, pi, sm, CoopVortA{VS, vi});
         const float3 acc = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
         const float3 w = make_float3(shf(s, 3), shf(s, 4), shf(s, 5));
         if ((threadIdx.x & 31u) == 0u) {
@@ -990,15 +989,13 @@ k_vorticity_a_coop(const float4* __restrict__ P, const float4* __restrict__ VS,
 template <class CP>
 __global__ void __launch_bounds__(kBlock)
 k_vorticity_b_coop(const float4* __restrict__ Q, const float4* __restrict__ VX,
-                   const float4* __restrict__ OM, const float4* __restrict__ XP,
-                   const uint32_t* __restrict__ perm, const int32_t* __restrict__ cstart,
-                   const int32_t* __restrict__ cend, float4* __restrict__ v,
-                   float4* __restrict__ eta_out, uint32_t n, CP cp, CoopWork wk) {
+                   const float4* __restrict__ OM, const uint32_t* __restrict__ perm,
+                   float4* __restrict__ v, float4* __restrict__ eta_out, uint32_t n, CP cp,
+                   CoopWork wk) {
     PBF_COOP_FOR_EACH(i) {
         const auto& c = cp.at(i);
         const float3 pi = xyz(Q[i]);
-        const float s = coop_visit(i, stencil_centre(XP[i], c), c, cstart, cend, Q, pi, sm,
-                                   CoopVortB{});  // neighbourcells.glsl:57
+        const float s = coop_visit(i, c, wk.rows, n, Q, pi, sm, CoopVortB{});
         float3 eta = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
         if ((threadIdx.x & 31u) == 0u) {
             if (eta_out) eta_out[i] = make_float4(eta.x, eta.y, eta.z, 0.0f);
@@ -1010,31 +1007,42 @@ k_vorticity_b_coop(const float4* __restrict__ Q, const float4* __restrict__ VX,
     }
 }
 
-// Mixed sweeps: the heavy particles (more than `threshold` stencil
-// candidates) go to the cooperative kernels, listed once per substep after
-// the cell pass (the set depends on the cell tables only, so every sweep of
-// the substep agrees on it); the one-thread kernels skip them.  A block
-// appends its heavy particles in ascending order (one atomic per block), so
-// consecutive warps of a cooperative launch work on neighbouring particles.
+// The substep's stencil rows: row o of sorted particle i, [x, y), at
+// rows[o * n + i].  They depend on the cell tables and the predicted positions
+// only, so they are found once after the cell pass and every sweep of the
+// substep reads them (9 coalesced 8-byte loads) instead of repeating the 27
+// cell lookups, the bounds tests and the merging (~500 instructions, and a
+// 72-byte local array) in each of its scanning sweeps.
+// Mixed sweeps (heavy != nullptr): the particles with more than `threshold`
+// stencil candidates go to the cooperative kernels and are listed here; the
+// one-thread kernels skip them.  A block appends its heavy particles in
+// ascending order (one atomic per block), so consecutive warps of a
+// cooperative launch work on neighbouring particles.
 template <class CP>
 __global__ void __launch_bounds__(kBlock)
-k_heavy_scan(const float4* __restrict__ XP, const int32_t* __restrict__ cstart,
-             const int32_t* __restrict__ cend, uint32_t threshold, uint32_t n, CP cp,
-             uint8_t* __restrict__ heavy, uint32_t* __restrict__ list, uint32_t* __restrict__ count) {
+k_stencil_rows(const float4* __restrict__ XP, const int32_t* __restrict__ cstart,
+               const int32_t* __restrict__ cend, uint32_t threshold, uint32_t n, CP cp,
+               int2* __restrict__ rows, uint8_t* __restrict__ heavy, uint32_t* __restrict__ list,
+               uint32_t* __restrict__ count) {
     __shared__ uint32_t warp_off[kBlock / 32];
     __shared__ uint32_t base;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     bool h = false;
     if (i < n) {
-        Runs r;
-        runs_of(stencil_centre(XP[i], cp.at(i)), cp.at(i), cstart, cend, r);
+        const auto& c = cp.at(i);
+        const int3 ctr = stencil_centre(XP[i], c);  // neighbourcells.glsl:57
         uint32_t cand = 0;
 #pragma unroll
-        for (int o = 0; o < 9; ++o) cand += (uint32_t)(r.e[o] - r.b[o]);
+        for (int o = 0; o < 9; ++o) {
+            const int2 be = run_of_row(o, ctr, c, cstart, cend);
+            rows[(size_t)o * n + i] = be;
+            cand += (uint32_t)(be.y - be.x);
+        }
         h = cand > threshold;
-        heavy[i] = h ? 1 : 0;
+        if (heavy) heavy[i] = h ? 1 : 0;
     }
+    if (!heavy) return;
     const uint32_t m = __ballot_sync(0xffffffffu, h);
     if (lane == 0) warp_off[wid] = __popc(m);
     __syncthreads();
@@ -1110,6 +1118,10 @@ k_vorticity_a(const float4* __restrict__ P, const float4* __restrict__ XP,
     };
     auto eval = [&](uint32_t j) { body(j, std::false_type{}); };
     auto eval_in = [&](uint32_t j) { body(j, std::true_type{}); };
+    auto near = [&](uint32_t j) {
+        const float3 d = sub3(pi, xyz(__ldg(P + j)));
+        return !(dot3(d, d) > c.r2cut);
+    };
     bool listed = false;
     if constexpr (LISTS) {
         const int32_t cnt = nl.cnt[i];
@@ -1130,10 +1142,9 @@ k_vorticity_a(const float4* __restrict__ P, const float4* __restrict__ XP,
     }
     if (!listed) {
         if constexpr (MODE == kPairs)
-            scan_then_eval<false>(i, ctr, c, cstart, cend, sx, pi, pw, [](int32_t, uint32_t) {},
-                                  eval_in);
+            scan_then_eval<false>(i, c, sx, pi, pw, [](int32_t, uint32_t) {}, near, eval_in);
         else if constexpr (MODE == kMasked)
-            sweep_visit<true>(i, ctr, c, cstart, cend, sx, pi, eval_in);
+            sweep_visit<true>(i, ctr, c, cstart, cend, pw, sx, pi, eval_in);
         else if (!LISTS && pw.runs)
             visit_direct_piles(
                 i, ctr, c, cstart, cend, pw.runs,
@@ -1152,7 +1163,7 @@ k_vorticity_a(const float4* __restrict__ P, const float4* __restrict__ XP,
                     w = repeat_add3(cross3(vij, g), w, r - j0);            // :55
                 });
         else
-            sweep_visit<false>(i, ctr, c, cstart, cend, sx, pi, eval);
+            sweep_visit<false>(i, ctr, c, cstart, cend, pw, sx, pi, eval);
     }
     const float3 vx = fma3(c.cx, acc, vi);  // :58
     VX[i] = make_float4(vx.x, vx.y, vx.z, 0.0f);
@@ -1209,7 +1220,7 @@ k_vorticity_b(const float4* __restrict__ Q, const float4* __restrict__ XP,
                         eta = repeat_fma3(__ldg(&Q[j0].w), g, eta, r - j0);  // :72
                     });
             else
-                sweep_visit<MODE != kDirect>(i, ctr, c, cstart, cend, sx, pi, body);
+                sweep_visit<MODE != kDirect>(i, ctr, c, cstart, cend, pr, sx, pi, body);
         }
     }
     if (eta_out) eta_out[i] = make_float4(eta.x, eta.y, eta.z, 0.0f);
@@ -1320,14 +1331,14 @@ void launch_lambda_build(SweepCfg sw, cudaStream_t st, const float4* XP, const u
                          const int32_t* cstart, const int32_t* cend, float4* L, float4* aux,
                          NbrLists nl, PairLists pw, ScanPos sx, uint32_t n, CP cp) {
     if (sw.mode == kCoop) {
-        k_lambda_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(XP, XP, cstart, cend, L, aux, n, cp,
-                                                           CoopWork{nullptr, nullptr});
+        k_lambda_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(XP, L, aux, n, cp,
+                                                           CoopWork{nullptr, nullptr, pw.rows});
         return;
     }
     PBF_SWEEP_LAUNCH(k_lambda_build, XP, skeys, cstart, cend, L, aux, nl, pw, sx, n, cp);
     if (pw.heavy)
-        k_lambda_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(XP, XP, cstart, cend, L, aux, n, cp,
-                                                         CoopWork{pw.heavy_list, pw.heavy_count});
+        k_lambda_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(XP, L, aux, n, cp,
+                                                         CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
 }
 template <class CP>
 void launch_lambda(SweepCfg sw, cudaStream_t st, const float4* P, const float4* XP,
@@ -1335,14 +1346,14 @@ void launch_lambda(SweepCfg sw, cudaStream_t st, const float4* P, const float4* 
                    float4* aux, NbrLists nl, PairLists pw, ScanPos sx, int dmax_slot, uint32_t n,
                    CP cp) {
     if (sw.mode == kCoop) {
-        k_lambda_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(P, XP, cstart, cend, L, aux, n, cp,
-                                                           CoopWork{nullptr, nullptr});
+        k_lambda_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(P, L, aux, n, cp,
+                                                           CoopWork{nullptr, nullptr, pw.rows});
         return;
     }
     PBF_SWEEP_LAUNCH(k_lambda, P, XP, skeys, cstart, cend, L, aux, nl, pw, sx, dmax_slot, n, cp);
     if (pw.heavy)
-        k_lambda_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(P, XP, cstart, cend, L, aux, n, cp,
-                                                         CoopWork{pw.heavy_list, pw.heavy_count});
+        k_lambda_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(P, L, aux, n, cp,
+                                                         CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
 }
 template <class CP>
 void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4* XP,
@@ -1350,23 +1361,23 @@ void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4*
                     NbrLists nl, PairLists pr, ScanPos sx, ScanPos sx_out, int dmax_slot,
                     int out_slot, uint32_t n, CP cp, uint32_t* status) {
     if (sw.mode == kCoop) {
-        k_delta_p_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(L, XP, cstart, cend, Pn,
-                                                            ScanPos{nullptr, nullptr}, n, cp, status,
-                                                            CoopWork{nullptr, nullptr});
+        k_delta_p_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(L, Pn, ScanPos{nullptr, nullptr}, n, cp, status,
+                                                            CoopWork{nullptr, nullptr, pr.rows});
         return;
     }
     PBF_SWEEP_LAUNCH(k_delta_p, L, XP, skeys, cstart, cend, Pn, nl, pr, sx, sx_out, dmax_slot,
                      out_slot, n, cp, status);
     if (pr.heavy)
-        k_delta_p_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(L, XP, cstart, cend, Pn, sx_out, n, cp,
+        k_delta_p_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(L, Pn, sx_out, n, cp,
                                                           status,
-                                                          CoopWork{pr.heavy_list, pr.heavy_count});
+                                                          CoopWork{pr.heavy_list, pr.heavy_count, pr.rows});
 }
 template <class CP>
-void launch_heavy_scan(unsigned g, cudaStream_t st, const float4* XP, const int32_t* cstart,
-                       const int32_t* cend, uint32_t threshold, uint32_t n, CP cp, uint8_t* heavy,
-                       uint32_t* list, uint32_t* count) {
-    k_heavy_scan<CP><<<g, kBlock, 0, st>>>(XP, cstart, cend, threshold, n, cp, heavy, list, count);
+void launch_stencil_rows(unsigned g, cudaStream_t st, const float4* XP, const int32_t* cstart,
+                         const int32_t* cend, uint32_t threshold, uint32_t n, CP cp, int2* rows,
+                         uint8_t* heavy, uint32_t* list, uint32_t* count) {
+    k_stencil_rows<CP><<<g, kBlock, 0, st>>>(XP, cstart, cend, threshold, n, cp, rows, heavy, list,
+                                             count);
 }
 template <class CP>
 void launch_commit(unsigned g, cudaStream_t st, const float4* P, const uint32_t* perm, float4* x,
@@ -1379,15 +1390,15 @@ void launch_vorticity_a(SweepCfg sw, cudaStream_t st, const float4* P, const flo
                         const int32_t* cend, float4* VX, float4* OM, float4* Q, NbrLists nl,
                         PairLists pw, ScanPos sx, int dmax_slot, uint32_t n, CP cp) {
     if (sw.mode == kCoop) {
-        k_vorticity_a_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(P, VS, XP, cstart, cend, VX, OM, Q,
-                                                               n, cp, CoopWork{nullptr, nullptr});
+        k_vorticity_a_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(P, VS, VX, OM, Q,
+                                                               n, cp, CoopWork{nullptr, nullptr, pw.rows});
         return;
     }
     PBF_SWEEP_LAUNCH(k_vorticity_a, P, XP, VS, skeys, cstart, cend, VX, OM, Q, nl, pw, sx, dmax_slot,
                      n, cp);
     if (pw.heavy)
         k_vorticity_a_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(
-            P, VS, XP, cstart, cend, VX, OM, Q, n, cp, CoopWork{pw.heavy_list, pw.heavy_count});
+            P, VS, VX, OM, Q, n, cp, CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
 }
 template <class CP>
 void launch_vorticity_b(SweepCfg sw, cudaStream_t st, const float4* Q, const float4* XP,
@@ -1396,16 +1407,16 @@ void launch_vorticity_b(SweepCfg sw, cudaStream_t st, const float4* Q, const flo
                         float4* v, float4* eta_out, NbrLists nl, PairLists pr, ScanPos sx,
                         int dmax_slot, uint32_t n, CP cp) {
     if (sw.mode == kCoop) {
-        k_vorticity_b_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(Q, VX, OM, XP, perm, cstart, cend, v,
-                                                               eta_out, n, cp, CoopWork{nullptr, nullptr});
+        k_vorticity_b_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(Q, VX, OM, perm, v,
+                                                               eta_out, n, cp, CoopWork{nullptr, nullptr, pr.rows});
         return;
     }
     PBF_SWEEP_LAUNCH(k_vorticity_b, Q, XP, VX, OM, skeys, perm, cstart, cend, v, eta_out, nl, pr, sx,
                      dmax_slot, n, cp);
     if (pr.heavy)
         k_vorticity_b_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(
-            Q, VX, OM, XP, perm, cstart, cend, v, eta_out, n, cp,
-            CoopWork{pr.heavy_list, pr.heavy_count});
+            Q, VX, OM, perm, v, eta_out, n, cp,
+            CoopWork{pr.heavy_list, pr.heavy_count, pr.rows});
 }
 template <class CP>
 void launch_diagnostics(unsigned g, cudaStream_t st, const float4* P, const float4* v,
@@ -1429,9 +1440,9 @@ void launch_diagnostics(unsigned g, cudaStream_t st, const float4* P, const floa
                                      const uint32_t*, const int32_t*, const int32_t*, float4*,  \
                                      NbrLists, PairLists, ScanPos, ScanPos, int, int, uint32_t, \
                                      CP, uint32_t*);                                            \
-    template void launch_heavy_scan<CP>(unsigned, cudaStream_t, const float4*, const int32_t*,    \
-                                        const int32_t*, uint32_t, uint32_t, CP, uint8_t*,          \
-                                        uint32_t*, uint32_t*);                                     \
+    template void launch_stencil_rows<CP>(unsigned, cudaStream_t, const float4*, const int32_t*, \
+                                          const int32_t*, uint32_t, uint32_t, CP, int2*,         \
+                                          uint8_t*, uint32_t*, uint32_t*);                       \
     template void launch_commit<CP>(unsigned, cudaStream_t, const float4*, const uint32_t*,     \
                                     float4*, float4*, float4*, uint32_t, CP);                   \
     template void launch_vorticity_a<CP>(SweepCfg, cudaStream_t, const float4*, const float4*,  \
@@ -1479,6 +1490,7 @@ cudaError_t preload_sweeps() {
     load((const void*)k_delta_p_coop<CP>);
     load((const void*)k_vorticity_a_coop<CP>);
     load((const void*)k_vorticity_b_coop<CP>);
+    load((const void*)k_stencil_rows<CP>);
     load((const void*)k_run_flags);
     load((const void*)k_run_flags_vals);
     return e;
