@@ -216,7 +216,8 @@ __device__ __forceinline__ void visit_direct_piles(uint32_t i, Ctr&& ctr, const 
 // past it: the scan copies are padded by a pair) and i itself are masked out
 // once per chunk.  With LIST, `list(base, mask)` also receives, per chunk, the
 // candidates base + t (bit t) with r2 <= c.r2list, before f runs on the chunk.
-// Measured, 2,097,152 particles at rest: PBF_T_SCAN.
+// Measured (2,097,152 particles, 20 substeps of the dam break; with the rows read
+// from k_stencil_rows): lambda 535 -> 464 us per launch, vorticity 607 -> 538.
 template <bool LIST, class S, class F>
 __device__ __forceinline__ void visit_masked(uint32_t i, const DevConsts& c,
                                              const int2* __restrict__ rows, uint32_t n,
