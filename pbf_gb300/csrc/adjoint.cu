@@ -53,17 +53,27 @@ namespace pbf {
 constexpr int kAdjBlock = 256;
 constexpr int kParams = 4;  // epsilon, tensile k, XSPH c, vorticity epsilon
 
+// Buffers and bookkeeping of a recorded run.  The buffers are one allocation,
+// kept with the handle and reused by the next pbf_forward_record of the same
+// shape (a training step records again and again: allocating and freeing them
+// in pieces cost 4 ms of a 21 ms step with 32,768 particles and 14 ms of 165 ms
+// with 1.2 million); pbf_release_record and the handle's end give them back.
 struct Tape {
     uint32_t substeps = 0, every = 0, iters = 0, nslots = 0;
     bool vort = false;
+    bool valid = false;    // holds a complete recorded run
+    uint32_t held = kNone; // the segment whose substeps the slots hold
+    static constexpr uint32_t kNone = 0xFFFFFFFFu;
     std::vector<float4*> ckpt_x, ckpt_v;  // states at substeps 0, every, 2 every, ... (id order)
     float4 *final_x = nullptr, *final_v = nullptr;
     struct Slot {
         uint32_t* perm = nullptr;
-        int32_t *cstart = nullptr, *cend = nullptr;
+        int2* rows = nullptr;  // [9][n] stencil rows around each particle's key cell
         std::vector<float4*> L, AUX;
         float4 *PF = nullptr, *VS = nullptr, *OM = nullptr, *Q = nullptr, *ETA = nullptr;
-        float4* X0 = nullptr;  // positions at the start of the substep (id order)
+        // the forward sweeps' pair lists, one per solver iteration and the
+        // vorticity passes' last (cap 0: not recorded)
+        std::vector<PairLists> lists;
     };
     std::vector<Slot> slots;
     // adjoint work buffers
@@ -78,7 +88,11 @@ struct Tape {
     uint8_t* heavy = nullptr;               // [n] swept by a warp (sorted), per substep
     uint32_t* heavy_list = nullptr;         // [n] those particles
     uint32_t warp_above = 0;                // candidates above which a particle gets a warp
-    std::vector<void*> owned;
+    double* sums = nullptr;                 // [scenes][kParams] parameter gradients
+    uint32_t* scene_first = nullptr;        // [scenes + 1] first particle of each scene
+    uint32_t list_cap = 0;                  // capacity of the recorded pair lists (0: none)
+    uint32_t list_pairs = 0;                // the handle's pair-list capacity at allocation
+    void* mem = nullptr;                    // holds all of the above
 };
 
 namespace {
@@ -171,55 +185,78 @@ struct PairDirs {
 // ---- neighbour visits of the reverse sweeps -----------------------------------
 //
 // Two reverse sweeps read each position set (delta-p then lambda at an
-// iterate, vorticity pass B then pass A at the final positions), so the first
-// scans the stencil once, writing each particle's in-range candidates (visit
-// order) to a list in the handle's pair-list buffer, and runs its pair terms
-// from that list; the second replays the list.  The lanes of a warp then run
-// their (heavy) pair terms together instead of each at its own point of the
-// stencil.  A particle whose list would overflow, or a handle without pair
-// lists, uses the direct stencil visit; results are the same either way (the
-// pair terms test r2 themselves, in the same order).
+// iterate, vorticity pass B then pass A at the final positions), the sets
+// whose in-range candidates the forward sweeps listed: the recorded run keeps
+// those lists, and both reverse sweeps replay them.  The lanes of a warp then
+// run their (heavy) pair terms together instead of each at its own point of
+// the stencil, and nothing is scanned.  (1.2 million particles, per launch:
+// the delta-p sweep took 562 us when it scanned the stencil itself, 318 us now.)
+//
+// A particle without a recorded list (longer than its capacity, swept by a
+// warp in the forward run, or every one in a substep with particles predicted
+// outside the grid, whose one-way candidates the forward lists lack) scans its
+// stencil in the first of the two sweeps, writing its candidates to the
+// handle's own pair-list buffer, and replays those in the second; without
+// room there it visits the stencil both times.  Results are the same either
+// way (the pair terms test r2 themselves, in the same order).
 struct AdjLists {
-    uint32_t* idx;
-    int32_t* cnt;
-    uint32_t cap, n;
+    PairLists rec;         // the forward run's list of this position set (cap 0: none)
+    PairLists own;         // scratch list (cap 0: none)
+    const int2* rows;      // [9][n] the key-cell stencil rows
+    const uint32_t* any;   // nonzero when the substep has irregular particles
+    __device__ __forceinline__ bool recorded(uint32_t i) const {
+        return rec.cap && !__ldg(any) && __ldg(rec.cnt + i) >= 0;
+    }
 };
 
 template <class F>
-__device__ __forceinline__ void adj_replay(uint32_t i, const DevConsts& c, const AdjLists& al,
+__device__ __forceinline__ void adj_replay(uint32_t i, const DevConsts& c, const PairLists& pl,
                                            F&& f) {
-    const int32_t cnt = al.cnt[i];
-    const uint32_t* p = al.idx + i;
+    const int32_t cnt = pl.cnt[i];
+    const uint32_t* p = pl.idx + i;
     if (cnt > 0) {  // the next index is loaded one entry ahead
         uint32_t jn = p[0];
 #pragma unroll 1
         for (int32_t k = 0; k < cnt; ++k) {
             const uint32_t j = jn;
-            if (k + 1 < cnt) jn = p[(size_t)(k + 1) * al.n];
+            if (k + 1 < cnt) jn = p[(size_t)(k + 1) * pl.n];
             if (check_ok(c, j < c.n_total)) f(j);
         }
     }
 }
 
-template <class Ctr, class F>
-__device__ __forceinline__ void adj_scan_eval(uint32_t i, Ctr&& ctr, const DevConsts& c,
-                                              const int32_t* __restrict__ cstart,
-                                              const int32_t* __restrict__ cend,
-                                              const float4* __restrict__ X, float3 pi,
-                                              const AdjLists& al, F&& f) {
-    if (!al.cap) {
-        visit_full(i, ctr, c, cstart, cend, f);
-        return;
-    }
-    Runs r;
-    runs_of(ctr(), c, cstart, cend, r);
-    uint32_t tot = 0;
-    uint32_t* const out = al.idx + i;
+template <class F>
+__device__ __forceinline__ void adj_visit_rows(uint32_t i, const AdjLists& al, F&& f) {
 #pragma unroll 1
     for (int o = 0; o < 9; ++o) {
-        const int32_t e = r.e[o];
+        const int2 be = __ldg(al.rows + (size_t)o * al.own.n + i);
+        for (int32_t j = be.x; j < be.y; ++j)
+            if ((uint32_t)j != i) f((uint32_t)j);
+    }
+}
+
+// The first of the two sweeps over a position set.
+template <class F>
+__device__ __forceinline__ void adj_visit_first(uint32_t i, const DevConsts& c,
+                                                const float4* __restrict__ X, float3 pi,
+                                                const AdjLists& al, F&& f) {
+    if (al.recorded(i)) {
+        adj_replay(i, c, al.rec, f);
+        return;
+    }
+    const PairLists& own = al.own;
+    if (!own.cap) {
+        adj_visit_rows(i, al, f);
+        return;
+    }
+    uint32_t tot = 0;
+    uint32_t* const out = own.idx + i;
 #pragma unroll 1
-        for (int32_t base = r.b[o]; base < e; base += 32) {
+    for (int o = 0; o < 9; ++o) {
+        const int2 be = __ldg(al.rows + (size_t)o * own.n + i);
+        const int32_t e = be.y;
+#pragma unroll 1
+        for (int32_t base = be.x; base < e; base += 32) {
             const float4* __restrict__ p = X + base;
             const float4* const pe = p + min(e - base, 32);
             uint32_t m = 0, bit = 1;
@@ -235,29 +272,30 @@ __device__ __forceinline__ void adj_scan_eval(uint32_t i, Ctr&& ctr, const DevCo
             while (m) {
                 const int t = __ffs(m) - 1;
                 m &= m - 1;
-                if (tot < al.cap) out[(size_t)tot * al.n] = (uint32_t)(base + t);
+                if (tot < own.cap) out[(size_t)tot * own.n] = (uint32_t)(base + t);
                 ++tot;
             }
         }
     }
-    if (tot <= al.cap) {
-        al.cnt[i] = (int32_t)tot;
-        adj_replay(i, c, al, f);
+    if (tot <= own.cap) {
+        own.cnt[i] = (int32_t)tot;
+        adj_replay(i, c, own, f);
     } else {
-        al.cnt[i] = -1;
-        visit_full(i, ctr, c, cstart, cend, f);
+        own.cnt[i] = -1;
+        adj_visit_rows(i, al, f);
     }
 }
 
-template <class Ctr, class F>
-__device__ __forceinline__ void adj_visit_again(uint32_t i, Ctr&& ctr, const DevConsts& c,
-                                                const int32_t* __restrict__ cstart,
-                                                const int32_t* __restrict__ cend,
+// The second one.
+template <class F>
+__device__ __forceinline__ void adj_visit_again(uint32_t i, const DevConsts& c,
                                                 const AdjLists& al, F&& f) {
-    if (al.cap && al.cnt[i] >= 0)
-        adj_replay(i, c, al, f);
+    if (al.recorded(i))
+        adj_replay(i, c, al.rec, f);
+    else if (al.own.cap && al.own.cnt[i] >= 0)
+        adj_replay(i, c, al.own, f);
     else
-        visit_full(i, ctr, c, cstart, cend, f);
+        adj_visit_rows(i, al, f);
 }
 
 // ---- a warp per particle for dense stencils ---------------------------------------
@@ -274,18 +312,15 @@ __device__ __forceinline__ void adj_visit_again(uint32_t i, Ctr&& ctr, const Dev
 // the thread's, so the two agree to rounding, not bitwise; both are
 // deterministic.
 
-template <class Ctr, class F>
-__device__ __forceinline__ void warp_visit(uint32_t i, Ctr&& ctr, const DevConsts& c,
-                                           const int32_t* __restrict__ cstart,
-                                           const int32_t* __restrict__ cend, uint32_t lane,
-                                           F&& f) {
-    Runs r;
-    runs_of(ctr(), c, cstart, cend, r);
+template <class F>
+__device__ __forceinline__ void warp_visit(uint32_t i, const AdjLists& al, uint32_t lane, F&& f) {
 #pragma unroll 1
-    for (int o = 0; o < 9; ++o)
+    for (int o = 0; o < 9; ++o) {
+        const int2 be = __ldg(al.rows + (size_t)o * al.own.n + i);
 #pragma unroll 1
-        for (int32_t j = r.b[o] + (int32_t)lane; j < r.e[o]; j += 32)
+        for (int32_t j = be.x + (int32_t)lane; j < be.y; j += 32)
             if ((uint32_t)j != i) f((uint32_t)j);
+    }
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -318,6 +353,23 @@ __device__ __forceinline__ const DevConsts& consts_of(const CP& cp, uint32_t id)
 
 // ---- reverse kernels --------------------------------------------------------------
 
+// Stencil rows around the key cell of every particle, from the cell tables of
+// the substep just recorded (the reverse sweeps read the rows, so the tables
+// need not be kept).
+template <class CP>
+__global__ void __launch_bounds__(kAdjBlock)
+k_adj_rows(const uint32_t* __restrict__ perm, const float4* __restrict__ XPc,
+           const int32_t* __restrict__ cstart, const int32_t* __restrict__ cend,
+           int2* __restrict__ rows, uint32_t n, CP cp) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const DevConsts& c = consts_of(cp, perm[i]);
+    const int3 cell = key_cell(XPc[i], c);
+#pragma unroll
+    for (int o = 0; o < 9; ++o)
+        rows[(size_t)o * n + i] = run_of_row(o, cell, c, cstart, cend);
+}
+
 // Per substep: irr[i] = 1 when particle i's stencil centre is not its key
 // cell (predicted outside the grid), and word[0] set when some particle is;
 // with `above` != kAdjNoWarps, heavy[i] = 1 when i's key-cell stencil holds
@@ -326,9 +378,9 @@ __device__ __forceinline__ const DevConsts& consts_of(const CP& cp, uint32_t id)
 template <class CP>
 __global__ void __launch_bounds__(kAdjBlock)
 k_adj_flags(const uint32_t* __restrict__ perm, const float4* __restrict__ XPc,
-            const int32_t* __restrict__ cstart, const int32_t* __restrict__ cend,
-            uint32_t above, uint8_t* __restrict__ irr, uint8_t* __restrict__ heavy,
-            uint32_t* __restrict__ list, uint32_t* __restrict__ word, uint32_t n, CP cp) {
+            const int2* __restrict__ rows, uint32_t above, uint8_t* __restrict__ irr,
+            uint8_t* __restrict__ heavy, uint32_t* __restrict__ list, uint32_t* __restrict__ word,
+            uint32_t n, CP cp) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const DevConsts& c = consts_of(cp, perm[i]);
@@ -338,11 +390,12 @@ k_adj_flags(const uint32_t* __restrict__ perm, const float4* __restrict__ XPc,
     irr[i] = odd ? 1 : 0;
     if (odd) atomicOr(word, 1u);
     if (above == kAdjNoWarps) return;
-    Runs r;
-    runs_of(b, c, cstart, cend, r);
     uint32_t cand = 0;
 #pragma unroll
-    for (int o = 0; o < 9; ++o) cand += (uint32_t)(r.e[o] - r.b[o]);
+    for (int o = 0; o < 9; ++o) {
+        const int2 be = rows[(size_t)o * n + i];
+        cand += (uint32_t)(be.y - be.x);
+    }
     const bool h = cand > above;
     heavy[i] = h ? 1 : 0;
     if (h) {
@@ -406,9 +459,6 @@ k_adj_vort_b1(const uint32_t* __restrict__ perm, const float4* __restrict__ VB,
 template <class CP>
 struct AdjVortB2 {
     const uint32_t* __restrict__ perm;
-    const float4* __restrict__ XPc;
-    const int32_t* __restrict__ cstart;
-    const int32_t* __restrict__ cend;
     const float4* __restrict__ Q;
     const float4* __restrict__ OM;
     const float4* __restrict__ ETB;
@@ -427,7 +477,6 @@ struct AdjVortB2 {
         const float3 ebi = f3(ETB[i]);
         float mb = 0.0f;
         float3 pb = make_float3(0.0f, 0.0f, 0.0f);
-        auto ctr = [&] { return key_cell(XPc[i], c); };
         auto pair = [&](uint32_t j) {
             const float4 Qj = __ldg(Q + j);
             const float3 d = pi - f3(Qj);
@@ -441,12 +490,12 @@ struct AdjVortB2 {
             pb = pb + sp.H(d, (own * Qj.w) * ebi - mi * ebj);
         };
         if constexpr (W) {
-            warp_visit(i, ctr, c, cstart, cend, lane, pair);
+            warp_visit(i, al, lane, pair);
             mb = warp_sum(mb);
             pb = warp_sum(pb);
             if (lane) return;
         } else {
-            adj_scan_eval(i, ctr, c, cstart, cend, Q, pi, al, pair);
+            adj_visit_first(i, c, Q, pi, al, pair);
         }
         float3 wb = f3(OMB[i]);
         if (mi > 0.0f) wb = wb + (mb / mi) * f3(OM[i]);
@@ -460,9 +509,6 @@ struct AdjVortB2 {
 template <class CP>
 struct AdjVortA {
     const uint32_t* __restrict__ perm;
-    const float4* __restrict__ XPc;
-    const int32_t* __restrict__ cstart;
-    const int32_t* __restrict__ cend;
     const float4* __restrict__ PF;
     const float4* __restrict__ VS;
     const float4* __restrict__ VSB;
@@ -485,7 +531,6 @@ struct AdjVortA {
         float3 vb = W ? zero : sbi;
         float3 pb = W ? zero : f3(PA[i]);
         float3 wsum = zero;
-        auto ctr = [&] { return key_cell(XPc[i], c); };
         auto pair = [&](uint32_t j) {
             const float3 d = pi - f3(__ldg(PF + j));
             const float r2 = dotf(d, d);
@@ -506,13 +551,13 @@ struct AdjVortA {
             pb = pb + sp.H(d, crossf(wbs, vji));
         };
         if constexpr (W) {
-            warp_visit(i, ctr, c, cstart, cend, lane, pair);
+            warp_visit(i, al, lane, pair);
             vb = sbi + warp_sum(vb);
             pb = f3(PA[i]) + warp_sum(pb);
             wsum = warp_sum(wsum);
             if (lane) return;
         } else {
-            adj_visit_again(i, ctr, c, cstart, cend, al, pair);
+            adj_visit_again(i, c, al, pair);
         }
         acc_c[id] += (double)dotf(sbi, wsum);
         VCB[i] = make_float4(vb.x, vb.y, vb.z, 0.0f);
@@ -553,9 +598,6 @@ k_adj_commit(const uint32_t* __restrict__ perm, const float4* __restrict__ XB,
 template <class CP>
 struct AdjDeltaP {
     const uint32_t* __restrict__ perm;
-    const float4* __restrict__ XPc;
-    const int32_t* __restrict__ cstart;
-    const int32_t* __restrict__ cend;
     const float4* __restrict__ L;
     const float4* __restrict__ AUX;
     const float4* __restrict__ QB;
@@ -577,7 +619,6 @@ struct AdjDeltaP {
         float lb = 0.0f, kb = 0.0f;
         float3 pb = W ? make_float3(0.0f, 0.0f, 0.0f) : qbi;
         const float sc4 = c.scale * c.scale * c.scale * c.scale;
-        auto ctr = [&] { return key_cell(XPc[i], c); };
         auto pair = [&](uint32_t j) {
             const float4 Lj = __ldg(L + j);
             const float3 d = pi - f3(Lj);
@@ -601,13 +642,13 @@ struct AdjDeltaP {
             kb -= own * c.oorho * dotf(qbi, G) * sc4 * W3 * W6;
         };
         if constexpr (W) {
-            warp_visit(i, ctr, c, cstart, cend, lane, pair);
+            warp_visit(i, al, lane, pair);
             lb = warp_sum(lb);
             kb = warp_sum(kb);
             pb = qbi + warp_sum(pb);
             if (lane) return;
         } else {
-            adj_scan_eval(i, ctr, c, cstart, cend, L, pi, al, pair);
+            adj_visit_first(i, c, L, pi, al, pair);
         }
         const float4 aux = AUX[i];
         const float D = aux.w + c.eps;
@@ -626,9 +667,6 @@ struct AdjDeltaP {
 template <class CP>
 struct AdjLambda {
     const uint32_t* __restrict__ perm;
-    const float4* __restrict__ XPc;
-    const int32_t* __restrict__ cstart;
-    const int32_t* __restrict__ cend;
     const float4* __restrict__ L;
     const float4* __restrict__ AUX;
     const float4* __restrict__ RS;
@@ -647,7 +685,6 @@ struct AdjLambda {
         const float4 RSi = RS[i];
         const float3 gi = f3(AUX[i]);
         float3 pb = W ? make_float3(0.0f, 0.0f, 0.0f) : f3(PDB[i]);
-        auto ctr = [&] { return key_cell(XPc[i], c); };
         auto pair = [&](uint32_t j) {
             const float3 d = pi - f3(__ldg(L + j));
             const float r2 = dotf(d, d);
@@ -664,11 +701,11 @@ struct AdjLambda {
             pb = pb + (2.0f * c.oorho) * sp.H(d, u);
         };
         if constexpr (W) {
-            warp_visit(i, ctr, c, cstart, cend, lane, pair);
+            warp_visit(i, al, lane, pair);
             pb = f3(PDB[i]) + warp_sum(pb);
             if (lane) return;
         } else {
-            adj_visit_again(i, ctr, c, cstart, cend, al, pair);
+            adj_visit_again(i, c, al, pair);
         }
         if (first) {
             XSB[id] = make_float4(pb.x, pb.y, pb.z, 0.0f);
@@ -694,55 +731,118 @@ k_adj_predict(const float4* __restrict__ XSB, const float4* __restrict__ XOB,
     VB[id] = make_float4(vb.x, vb.y, vb.z, 0.0f);
 }
 
-// ---- host side ------------------------------------------------------------------
-
-template <class T>
-cudaError_t talloc(Tape* t, T** p, size_t count) {
-    cudaError_t e = cudaMalloc((void**)p, sizeof(T) * (count ? count : 1));
-    if (e == cudaSuccess) t->owned.push_back(*p);
-    return e;
+// Parameter gradients of each scene: sums the per-particle gradients acc
+// [kParams][n] over the scene's particles, one block per (scene, parameter),
+// in a fixed order (a strided partial sum per thread, then a tree).
+__global__ void __launch_bounds__(kAdjBlock)
+k_adj_param_sums(const double* __restrict__ acc, const uint32_t* __restrict__ first, uint32_t n,
+                 double* __restrict__ sums) {
+    __shared__ double part[kAdjBlock];
+    const uint32_t scene = blockIdx.x / kParams, p = blockIdx.x % kParams;
+    const uint32_t e = first[scene + 1];
+    const double* __restrict__ a = acc + (size_t)p * n;
+    double s = 0.0;
+    for (uint32_t i = first[scene] + threadIdx.x; i < e; i += kAdjBlock) s += a[i];
+    part[threadIdx.x] = s;
+    for (uint32_t h = kAdjBlock / 2; h > 0; h >>= 1) {
+        __syncthreads();
+        if (threadIdx.x < h) part[threadIdx.x] += part[threadIdx.x + h];
+    }
+    if (threadIdx.x == 0) sums[blockIdx.x] = part[0];
 }
 
-cudaError_t alloc_tape(pbf_sim* s, Tape* t) {
+// ---- host side ------------------------------------------------------------------
+
+// Hands out 256-byte aligned pieces of one allocation (base null: only counts).
+struct Carver {
+    uint8_t* base;
+    size_t used = 0;
+    template <class T>
+    void take(T** p, size_t count) {
+        if (base) *p = reinterpret_cast<T*>(base + used);
+        used += (sizeof(T) * (count ? count : 1) + 255) & ~size_t(255);
+    }
+};
+
+void carve_tape(const pbf_sim* s, Tape* t, Carver& a) {
     const size_t n = s->n;
     const uint32_t nck = (t->substeps + t->every - 1) / t->every;
-    cudaError_t e = cudaSuccess;
-    t->ckpt_x.assign(nck, nullptr);
-    t->ckpt_v.assign(nck, nullptr);
-    for (uint32_t k = 0; k < nck && e == cudaSuccess; ++k) {
-        e = talloc(t, &t->ckpt_x[k], n);
-        if (e == cudaSuccess) e = talloc(t, &t->ckpt_v[k], n);
+    t->ckpt_x.resize(nck);
+    t->ckpt_v.resize(nck);
+    for (uint32_t k = 0; k < nck; ++k) {
+        a.take(&t->ckpt_x[k], n);
+        a.take(&t->ckpt_v[k], n);
     }
-    if (e == cudaSuccess) e = talloc(t, &t->final_x, n);
-    if (e == cudaSuccess) e = talloc(t, &t->final_v, n);
+    a.take(&t->final_x, n);
+    a.take(&t->final_v, n);
     t->slots.resize(t->nslots);
     for (auto& sl : t->slots) {
-        if (e == cudaSuccess) e = talloc(t, &sl.perm, n);
-        if (e == cudaSuccess) e = talloc(t, &sl.cstart, s->ncells);
-        if (e == cudaSuccess) e = talloc(t, &sl.cend, s->ncells);
-        sl.L.assign(t->iters, nullptr);
-        sl.AUX.assign(t->iters, nullptr);
-        for (uint32_t k = 0; k < t->iters && e == cudaSuccess; ++k) {
-            e = talloc(t, &sl.L[k], n);
-            if (e == cudaSuccess) e = talloc(t, &sl.AUX[k], n);
+        a.take(&sl.perm, n);
+        a.take(&sl.rows, 9 * n);
+        sl.L.resize(t->iters);
+        sl.AUX.resize(t->iters);
+        for (uint32_t k = 0; k < t->iters; ++k) {
+            a.take(&sl.L[k], n);
+            a.take(&sl.AUX[k], n);
         }
-        if (e == cudaSuccess) e = talloc(t, &sl.PF, n);
-        if (e == cudaSuccess) e = talloc(t, &sl.VS, n);
-        if (e == cudaSuccess) e = talloc(t, &sl.OM, n);
-        if (e == cudaSuccess) e = talloc(t, &sl.Q, n);
-        if (e == cudaSuccess) e = talloc(t, &sl.ETA, n);
-        if (e == cudaSuccess) e = talloc(t, &sl.X0, n);
+        float4** one[] = {&sl.PF, &sl.VS, &sl.OM, &sl.Q, &sl.ETA};
+        for (float4** w : one) a.take(w, n);
+        sl.lists.assign(t->iters + 1, PairLists{nullptr, nullptr, 0, s->n});
+        if (t->list_cap)
+            for (uint32_t k = 0; k < t->iters + (t->vort ? 1u : 0u); ++k) {
+                sl.lists[k].cap = t->list_cap;
+                a.take(&sl.lists[k].idx, (size_t)t->list_cap * n);
+                a.take(&sl.lists[k].cnt, n);
+            }
     }
     float4** work[] = {&t->XB, &t->VB, &t->XB2, &t->VB2, &t->QB, &t->PDB, &t->RS, &t->PA,
                        &t->VSB, &t->ETB, &t->OMB, &t->VCB, &t->XSB, &t->XOB};
-    for (float4** w : work)
-        if (e == cudaSuccess) e = talloc(t, w, n);
-    if (e == cudaSuccess) e = talloc(t, &t->acc, (size_t)kParams * n);
-    if (e == cudaSuccess) e = talloc(t, &t->irr, n);
-    if (e == cudaSuccess) e = talloc(t, &t->words, 2);
-    if (e == cudaSuccess) e = talloc(t, &t->heavy, n);
-    if (e == cudaSuccess) e = talloc(t, &t->heavy_list, n);
-    return e;
+    for (float4** w : work) a.take(w, n);
+    a.take(&t->acc, (size_t)kParams * n);
+    a.take(&t->irr, n);
+    a.take(&t->words, 2);
+    a.take(&t->heavy, n);
+    a.take(&t->heavy_list, n);
+    a.take(&t->sums, (size_t)s->nscenes * kParams);
+    a.take(&t->scene_first, (size_t)s->nscenes + 1);
+}
+
+// Capacity of the recorded pair lists: the handle's while the tape then stays
+// below kAdjListBytes; otherwise kAdjListCap entries per particle (a fluid at
+// its rest density has about 33 neighbours; a longer list is not kept), and
+// none where that would take more than half of the free memory.
+constexpr size_t kAdjListBytes = size_t(4) << 30;
+constexpr uint32_t kAdjListCap = 48;
+
+cudaError_t alloc_tape(pbf_sim* s, Tape* t) {
+    auto bytes = [&](uint32_t cap) {
+        t->list_cap = cap;
+        Carver a{nullptr};
+        carve_tape(s, t, a);
+        return a.used;
+    };
+    size_t need = bytes(s->pair_cap);
+    if (need > kAdjListBytes) need = bytes(std::min(s->pair_cap, kAdjListCap));
+    if (t->list_cap && need > kAdjListBytes) {
+        size_t free_b = 0, total_b = 0;
+        const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+        if (e != cudaSuccess) return e;
+        if (need > free_b / 2) need = bytes(0);
+    }
+    cudaError_t e = cudaMalloc(&t->mem, need);
+    if (e == cudaErrorMemoryAllocation && t->list_cap) {
+        cudaGetLastError();
+        need = bytes(0);
+        e = cudaMalloc(&t->mem, need);
+    }
+    if (e != cudaSuccess) {
+        t->mem = nullptr;
+        return e;
+    }
+    Carver a{(uint8_t*)t->mem};
+    carve_tape(s, t, a);
+    return cudaMemcpy(t->scene_first, s->offsets.data(), sizeof(uint32_t) * (s->nscenes + 1),
+                      cudaMemcpyHostToDevice);
 }
 
 template <class CP>
@@ -755,15 +855,16 @@ cudaError_t reverse_substep(pbf_sim* s, Tape* t, const Tape::Slot& sl, const CP&
     double* acc_k = t->acc + n;
     double* acc_c = t->acc + 2 * (size_t)n;
     double* acc_ev = t->acc + 3 * (size_t)n;
-    const AdjLists al{s->pair_idx, s->pair_cnt, s->pair_cap, n};
+    const PairLists own{s->pair_idx, s->pair_cnt, s->pair_cap, n};
+    auto lists = [&](int k) { return AdjLists{sl.lists[k], own, sl.rows, t->words}; };
     // the substep's predicted positions (sorted), where every stencil is
     // centred (neighbourcells.glsl:57): the first lambda sweep's L holds them,
     // and PF does when there is no solver iteration
     const float4* XPc = iters > 0 ? sl.L[0] : sl.PF;
     cudaError_t fe = cudaMemsetAsync(t->words, 0, 2 * sizeof(uint32_t), st);
     if (fe != cudaSuccess) return fe;
-    k_adj_flags<<<g, kAdjBlock, 0, st>>>(sl.perm, XPc, sl.cstart, sl.cend, t->warp_above, t->irr,
-                                         t->heavy, t->heavy_list, t->words, n, cp);
+    k_adj_flags<<<g, kAdjBlock, 0, st>>>(sl.perm, XPc, sl.rows, t->warp_above, t->irr, t->heavy,
+                                         t->heavy_list, t->words, n, cp);
     const PairDirs dirs{t->irr, XPc, t->words};
     // the particles with dense stencils get a warp each
     const bool warps = t->warp_above != kAdjNoWarps;
@@ -774,18 +875,19 @@ cudaError_t reverse_substep(pbf_sim* s, Tape* t, const Tape::Slot& sl, const CP&
     if (t->vort) {
         k_adj_vort_b1<<<g, kAdjBlock, 0, st>>>(sl.perm, t->VB, sl.OM, sl.ETA, t->VSB, t->ETB,
                                                t->OMB, acc_ev, n, cp);
-        sweep(AdjVortB2<CP>{sl.perm, XPc, sl.cstart, sl.cend, sl.Q, sl.OM, t->ETB, t->OMB, t->PA,
-                            al, dirs, cp});
-        sweep(AdjVortA<CP>{sl.perm, XPc, sl.cstart, sl.cend, sl.PF, sl.VS, t->VSB, t->OMB,
-                           t->VCB, t->PA, acc_c, al, dirs, cp});
+        const AdjLists al = lists(iters);
+        sweep(AdjVortB2<CP>{sl.perm, sl.Q, sl.OM, t->ETB, t->OMB, t->PA, al, dirs, cp});
+        sweep(AdjVortA<CP>{sl.perm, sl.PF, sl.VS, t->VSB, t->OMB, t->VCB, t->PA, acc_c, al, dirs,
+                           cp});
     }
     k_adj_commit<<<g, kAdjBlock, 0, st>>>(sl.perm, t->XB, t->VB, t->VCB, t->PA, sl.PF, t->QB,
                                           t->XOB, t->XSB, t->vort ? 1 : 0, iters, n, cp);
     for (int k = iters - 1; k >= 0; --k) {
-        sweep(AdjDeltaP<CP>{sl.perm, XPc, sl.cstart, sl.cend, sl.L[k], sl.AUX[k], t->QB, t->PDB,
-                            t->RS, acc_eps, acc_k, al, dirs, cp});
-        sweep(AdjLambda<CP>{sl.perm, XPc, sl.cstart, sl.cend, sl.L[k], sl.AUX[k], t->RS, t->PDB,
-                            t->QB, t->XSB, k == 0 ? 1 : 0, al, dirs, cp});
+        const AdjLists al = lists(k);
+        sweep(AdjDeltaP<CP>{sl.perm, sl.L[k], sl.AUX[k], t->QB, t->PDB, t->RS, acc_eps, acc_k, al,
+                            dirs, cp});
+        sweep(AdjLambda<CP>{sl.perm, sl.L[k], sl.AUX[k], t->RS, t->PDB, t->QB, t->XSB,
+                            k == 0 ? 1 : 0, al, dirs, cp});
     }
     k_adj_predict<<<g, kAdjBlock, 0, st>>>(t->XSB, t->XOB, t->XB2, t->VB2, n, cp);
     std::swap(t->XB, t->XB2);
@@ -798,14 +900,15 @@ cudaError_t reverse_dispatch(pbf_sim* s, Tape* t, const Tape::Slot& sl) {
     return reverse_substep(s, t, sl, ManyScenes{s->d_consts, s->sid});
 }
 
-// Runs `count` substeps from the current state, recording each into a slot.
-cudaError_t record_segment(pbf_sim* s, Tape* t, uint32_t count) {
+// Runs segment `seg` (`count` substeps) from the current state, recording each
+// substep into a slot.
+cudaError_t record_segment(pbf_sim* s, Tape* t, uint32_t seg, uint32_t count) {
     cudaStream_t st = s->stream;
     const size_t n = s->n;
+    const unsigned g = grid_for(s->n, kAdjBlock);
+    t->held = Tape::kNone;
     for (uint32_t k = 0; k < count; ++k) {
         Tape::Slot& sl = t->slots[k];
-        cudaError_t e = cudaMemcpyAsync(sl.X0, s->x, sizeof(float4) * n, cudaMemcpyDeviceToDevice, st);
-        if (e != cudaSuccess) return e;
         Recording rec;
         rec.L = sl.L.data();
         rec.AUX = sl.AUX.data();
@@ -814,17 +917,30 @@ cudaError_t record_segment(pbf_sim* s, Tape* t, uint32_t count) {
         rec.OM = sl.OM;
         rec.Q = sl.Q;
         rec.ETA = sl.ETA;
+        cudaError_t e = cudaSuccess;
+        if (t->list_cap) {
+            rec.lists = sl.lists.data();
+            // particles that a cooperative sweep takes write no list
+            for (const PairLists& pl : sl.lists)
+                if (pl.cap && e == cudaSuccess)
+                    e = cudaMemsetAsync(pl.cnt, 0xFF, sizeof(int32_t) * n, st);
+            if (e != cudaSuccess) return e;
+        }
         e = enqueue_substep(s, nullptr, &rec);
         if (e != cudaSuccess) return e;
         e = cudaMemcpyAsync(sl.perm, s->perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(sl.cstart, s->cstart, sizeof(int32_t) * s->ncells,
-                                cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(sl.cend, s->cend, sizeof(int32_t) * s->ncells,
-                                cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) return e;
+        const float4* XPc = t->iters > 0 ? sl.L[0] : sl.PF;
+        if (s->nscenes == 1)
+            k_adj_rows<<<g, kAdjBlock, 0, st>>>(sl.perm, XPc, s->cstart, s->cend, sl.rows, s->n,
+                                                OneScene{s->dc});
+        else
+            k_adj_rows<<<g, kAdjBlock, 0, st>>>(sl.perm, XPc, s->cstart, s->cend, sl.rows, s->n,
+                                                ManyScenes{s->d_consts, s->sid});
+        e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
+    t->held = seg;
     return cudaSuccess;
 }
 
@@ -832,9 +948,20 @@ cudaError_t record_segment(pbf_sim* s, Tape* t, uint32_t count) {
 
 void free_tape(pbf_sim* s) {
     if (!s->tape) return;
-    for (void* p : s->tape->owned) cudaFree(p);
+    if (s->tape->mem) cudaFree(s->tape->mem);
     delete s->tape;
     s->tape = nullptr;
+}
+
+void invalidate_tape(pbf_sim* s) {
+    if (s->tape) s->tape->valid = false;
+}
+
+bool free_idle_tape(pbf_sim* s) {
+    if (!s->tape || s->tape->valid) return false;
+    cudaStreamSynchronize(s->stream);
+    free_tape(s);
+    return true;
 }
 
 }  // namespace pbf
@@ -850,30 +977,53 @@ pbf_status pbf_forward_record(pbf_sim* s, uint32_t substeps, uint32_t checkpoint
         return fail(s, PBF_ERR_INVALID_ARGUMENT, "substeps and checkpoint_every must be positive");
     DeviceGuard dg(s->device);
     PBF_CUDA(s, cudaStreamSynchronize(s->stream));
-    free_tape(s);
-    Tape* t = new Tape();
-    s->tape = t;
-    t->substeps = substeps;
-    t->every = std::min(checkpoint_every, substeps);
-    t->iters = s->params.num_solver_iterations;
-    t->nslots = t->every;
-    t->vort = s->params.vorticity_confinement != 0;
-    cudaError_t e = alloc_tape(s, t);
-    if (e != cudaSuccess) {
+    const uint32_t every = std::min(checkpoint_every, substeps);
+    const uint32_t iters = s->params.num_solver_iterations;
+    const bool vort = s->params.vorticity_confinement != 0;
+    Tape* t = s->tape;
+    // (the recorded lists' capacity follows the handle's)
+    if (t && !(t->substeps == substeps && t->every == every && t->iters == iters &&
+               t->vort == vort && t->list_pairs == s->pair_cap)) {
         free_tape(s);
-        return cuda_fail(s, e, "tape allocation");
+        t = nullptr;
     }
-    const size_t b = sizeof(float4) * s->n;
-    for (uint32_t k = 0; k < substeps; ++k) {
-        if (k % t->every == 0) {
-            PBF_CUDA(s, cudaMemcpyAsync(t->ckpt_x[k / t->every], s->x, b, cudaMemcpyDeviceToDevice, s->stream));
-            PBF_CUDA(s, cudaMemcpyAsync(t->ckpt_v[k / t->every], s->v, b, cudaMemcpyDeviceToDevice, s->stream));
+    if (!t) {
+        t = s->tape = new Tape();
+        t->substeps = substeps;
+        t->every = every;
+        t->iters = iters;
+        t->nslots = every;
+        t->vort = vort;
+        t->list_pairs = s->pair_cap;
+        cudaError_t e = alloc_tape(s, t);
+        if (e != cudaSuccess) {
+            free_tape(s);
+            return cuda_fail(s, e, "tape allocation");
         }
-        pbf_status r = pbf_step(s, 1);
-        if (r != PBF_OK) return r;
+    }
+    t->valid = false;
+    t->held = Tape::kNone;
+    const size_t b = sizeof(float4) * s->n;
+    // every segment but the last is stepped as usual and recorded when the
+    // reverse pass reaches it; the last is recorded at once (its slots are the
+    // first that the reverse pass reads)
+    const uint32_t last = (substeps - 1) / t->every;
+    for (uint32_t seg = 0; seg <= last; ++seg) {
+        PBF_CUDA(s, cudaMemcpyAsync(t->ckpt_x[seg], s->x, b, cudaMemcpyDeviceToDevice, s->stream));
+        PBF_CUDA(s, cudaMemcpyAsync(t->ckpt_v[seg], s->v, b, cudaMemcpyDeviceToDevice, s->stream));
+        const uint32_t cnt = std::min(t->every, substeps - seg * t->every);
+        if (seg < last || s->timing) {
+            pbf_status r = pbf_step(s, cnt);
+            if (r != PBF_OK) return r;
+        } else {
+            PBF_CUDA(s, record_segment(s, t, seg, cnt));
+            s->launched += (uint64_t)cnt * pbf_kernels_per_substep(s);
+            s->autop.count += cnt;
+        }
     }
     PBF_CUDA(s, cudaMemcpyAsync(t->final_x, s->x, b, cudaMemcpyDeviceToDevice, s->stream));
     PBF_CUDA(s, cudaMemcpyAsync(t->final_v, s->v, b, cudaMemcpyDeviceToDevice, s->stream));
+    t->valid = true;
     return check_status(s);
 }
 
@@ -881,7 +1031,8 @@ pbf_status pbf_backward(pbf_sim* s, const float* dL_dx4, const float* dL_dv4, in
                         float* dL_dx0_4, float* dL_dv0_4, pbf_param_grads* grads) {
     NvtxRange nvtx_("pbf_backward");
     if (!s) return fail(nullptr, PBF_ERR_INVALID_ARGUMENT, "sim is NULL");
-    if (!s->tape) return fail(s, PBF_ERR_INVALID_ARGUMENT, "no recorded forward run (pbf_forward_record)");
+    if (!s->tape || !s->tape->valid)
+        return fail(s, PBF_ERR_INVALID_ARGUMENT, "no recorded forward run (pbf_forward_record)");
     if (where != PBF_HOST && where != PBF_DEVICE) return fail(s, PBF_ERR_INVALID_ARGUMENT, "bad where");
     Tape* t = s->tape;
     if (t->iters != s->params.num_solver_iterations ||
@@ -910,9 +1061,11 @@ pbf_status pbf_backward(pbf_sim* s, const float* dL_dx4, const float* dL_dv4, in
     for (int seg = (int)nseg - 1; seg >= 0; --seg) {
         const uint32_t t0 = (uint32_t)seg * t->every;
         const uint32_t cnt = std::min(t->every, t->substeps - t0);
-        PBF_CUDA(s, cudaMemcpyAsync(s->x, t->ckpt_x[seg], b, cudaMemcpyDeviceToDevice, st));
-        PBF_CUDA(s, cudaMemcpyAsync(s->v, t->ckpt_v[seg], b, cudaMemcpyDeviceToDevice, st));
-        PBF_CUDA(s, record_segment(s, t, cnt));
+        if (t->held != (uint32_t)seg) {
+            PBF_CUDA(s, cudaMemcpyAsync(s->x, t->ckpt_x[seg], b, cudaMemcpyDeviceToDevice, st));
+            PBF_CUDA(s, cudaMemcpyAsync(s->v, t->ckpt_v[seg], b, cudaMemcpyDeviceToDevice, st));
+            PBF_CUDA(s, record_segment(s, t, (uint32_t)seg, cnt));
+        }
         for (int k = (int)cnt - 1; k >= 0; --k) PBF_CUDA(s, reverse_dispatch(s, t, t->slots[k]));
     }
     // the handle's state returns to the end of the recorded run
@@ -920,19 +1073,24 @@ pbf_status pbf_backward(pbf_sim* s, const float* dL_dx4, const float* dL_dv4, in
     PBF_CUDA(s, cudaMemcpyAsync(s->v, t->final_v, b, cudaMemcpyDeviceToDevice, st));
     if (dL_dx0_4) PBF_CUDA(s, cudaMemcpyAsync(dL_dx0_4, t->XB, b, out, st));
     if (dL_dv0_4) PBF_CUDA(s, cudaMemcpyAsync(dL_dv0_4, t->VB, b, out, st));
+    std::vector<double> sums;
+    if (grads) {
+        sums.resize((size_t)s->nscenes * kParams);
+        k_adj_param_sums<<<s->nscenes * kParams, kAdjBlock, 0, st>>>(t->acc, t->scene_first, s->n,
+                                                                     t->sums);
+        PBF_CUDA(s, cudaGetLastError());
+        PBF_CUDA(s, cudaMemcpyAsync(sums.data(), t->sums, sizeof(double) * sums.size(),
+                                    cudaMemcpyDeviceToHost, st));
+    }
     pbf_status r = check_status(s);
     if (r != PBF_OK) return r;
     if (grads) {
-        std::vector<double> acc((size_t)kParams * n);
-        PBF_CUDA(s, cudaMemcpy(acc.data(), t->acc, sizeof(double) * acc.size(), cudaMemcpyDeviceToHost));
         for (uint32_t sc = 0; sc < s->nscenes; ++sc) {
-            double sum[kParams] = {0, 0, 0, 0};
-            for (int p = 0; p < kParams; ++p)
-                for (uint32_t i = s->offsets[sc]; i < s->offsets[sc + 1]; ++i) sum[p] += acc[p * n + i];
-            grads[sc].epsilon = sum[0];
-            grads[sc].tensile_instability_k = sum[1];
-            grads[sc].xsph_viscosity_c = sum[2];
-            grads[sc].vorticity_epsilon = sum[3];
+            const double* v = &sums[(size_t)sc * kParams];
+            grads[sc].epsilon = v[0];
+            grads[sc].tensile_instability_k = v[1];
+            grads[sc].xsph_viscosity_c = v[2];
+            grads[sc].vorticity_epsilon = v[3];
         }
     }
     return PBF_OK;

@@ -250,7 +250,7 @@ uint32_t heavy_threshold(const pbf_sim* s) {
 std::atomic<int> g_fail_alloc_after{-1};
 
 template <typename T>
-cudaError_t dalloc(T** p, size_t count) {
+cudaError_t dalloc(T** p, size_t count, pbf_sim* s = nullptr) {
     int k = g_fail_alloc_after.load();
     while (k >= 0) {
         if (g_fail_alloc_after.compare_exchange_weak(k, k - 1)) {
@@ -261,7 +261,14 @@ cudaError_t dalloc(T** p, size_t count) {
             break;
         }
     }
-    return cudaMalloc((void**)p, sizeof(T) * (count > 0 ? count : 1));
+    const size_t bytes = sizeof(T) * (count > 0 ? count : 1);
+    cudaError_t e = cudaMalloc((void**)p, bytes);
+    // a tape that holds no recorded run gives its memory back first
+    if (e == cudaErrorMemoryAllocation && s && free_idle_tape(s)) {
+        cudaGetLastError();
+        e = cudaMalloc((void**)p, bytes);
+    }
+    return e;
 }
 
 // (Re)allocates the neighbour-list and guard buffers for the current
@@ -274,8 +281,8 @@ cudaError_t ensure_lists(pbf_sim* s) {
         s->nbr_idx = nullptr;
         s->nbr_cnt = nullptr;
         s->nbr_cap = 0;
-        cudaError_t e = dalloc(&s->nbr_idx, (size_t)(cap > 0 ? cap : 1) * s->n);
-        if (e == cudaSuccess) e = dalloc(&s->nbr_cnt, s->n);
+        cudaError_t e = dalloc(&s->nbr_idx, (size_t)(cap > 0 ? cap : 1) * s->n, s);
+        if (e == cudaSuccess) e = dalloc(&s->nbr_cnt, s->n, s);
         if (e != cudaSuccess) return e;
         s->nbr_cap = cap;
     }
@@ -287,8 +294,8 @@ cudaError_t ensure_lists(pbf_sim* s) {
         s->pair_cnt = nullptr;
         s->pair_cap = 0;
         if (pcap > 0) {
-            cudaError_t e = dalloc(&s->pair_idx, (size_t)pcap * s->n);
-            if (e == cudaSuccess) e = dalloc(&s->pair_cnt, s->n);
+            cudaError_t e = dalloc(&s->pair_idx, (size_t)pcap * s->n, s);
+            if (e == cudaSuccess) e = dalloc(&s->pair_cnt, s->n, s);
             if (e != cudaSuccess) return e;
             s->pair_cap = pcap;
         }
@@ -298,7 +305,7 @@ cudaError_t ensure_lists(pbf_sim* s) {
         if (s->guard) cudaFree(s->guard);
         s->guard = nullptr;
         s->guard_slots = 0;
-        cudaError_t e = dalloc(&s->guard, slots);
+        cudaError_t e = dalloc(&s->guard, slots, s);
         if (e != cudaSuccess) return e;
         s->guard_slots = slots;
     }
@@ -547,6 +554,16 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
                        runs_solver || runs_vort ? s->runs : nullptr, s->rows};
     PairLists pl_v = pl;
     pl_v.heavy = mix_v ? s->heavy : nullptr;
+    // a recorded substep lists its pairs in the recording's buffers
+    auto lists_of = [&](PairLists l, uint32_t k) {
+        if (rec && rec->lists && rec->lists[k].cap) {
+            l.idx = rec->lists[k].idx;
+            l.cnt = rec->lists[k].cnt;
+            l.cap = rec->lists[k].cap;
+        }
+        return l;
+    };
+    pl_v = lists_of(pl_v, iters);
     cudaError_t ge = cudaMemsetAsync(s->guard, 0, sizeof(uint32_t) * (2 + iters), st);
     if (ge != cudaSuccess) return ge;
     const float4* cur = s->XP;
@@ -558,18 +575,19 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
         float4* Lk = rec ? rec->L[it] : s->L;
         float4* aux = rec ? rec->AUX[it] : nullptr;
         const int in_slot = it == 0 ? -1 : (int)it;  // displacement of `cur` from XP
+        const PairLists pk = lists_of(pl, it);
         if (it == 0)
-            launch_lambda_build(s_lam, st, s->XP, s->skeys, s->cstart, s->cend, Lk, aux, nl, pl,
+            launch_lambda_build(s_lam, st, s->XP, s->skeys, s->cstart, s->cend, Lk, aux, nl, pk,
                                 scan_set(0), n, cps);
         else
-            launch_lambda(s_lam, st, cur, s->XP, s->skeys, s->cstart, s->cend, Lk, aux, nl, pl,
+            launch_lambda(s_lam, st, cur, s->XP, s->skeys, s->cstart, s->cend, Lk, aux, nl, pk,
                           scan_set(cur_set), in_slot, n, cps);
         if (dp_direct)
             k_run_flags_vals<<<grid_for(n + 1), kBlock, 0, st>>>(Lk, nullptr, 1, n, s->runs);
         mark(4 + 2 * it);
         // delta-p replays the pair lists the lambda sweep just recorded
         const bool write_scan = it + 1 < iters ? solver_scans : vort_scans;
-        launch_delta_p(s_dp, st, Lk, s->XP, s->skeys, s->cstart, s->cend, nxt, nl, pl,
+        launch_delta_p(s_dp, st, Lk, s->XP, s->skeys, s->cstart, s->cend, nxt, nl, pk,
                        scan_set(cur_set), write_scan ? scan_set(nxt_set) : ScanPos{nullptr, nullptr},
                        in_slot, (int)it + 1, n, cps, s->status);
         if (it + 1 < iters && lam_direct)
@@ -787,6 +805,13 @@ pbf_status pbf_set_scene_params(pbf_sim* s, uint32_t scene, const pbf_params* p)
          (p->vorticity_confinement != 0) != (s->params.vorticity_confinement != 0)))
         return fail(s, PBF_ERR_INVALID_ARGUMENT,
                     "all scenes share the iteration count and the vorticity flag");
+    if (std::memcmp(p, &s->sparams[scene], sizeof *p) == 0) {
+        // nothing changes but the recorded run, which ends with any call
+        // (a training step sets every scene's parameters, mostly the same)
+        invalidate_tape(s);
+        s->auto_trial = -1;
+        return PBF_OK;
+    }
     DeviceGuard dg(s->device);
     PBF_CUDA(s, cudaStreamSynchronize(s->stream));
     const uint32_t base = s->sdc[scene].cell_base;
@@ -800,7 +825,7 @@ pbf_status pbf_set_scene_params(pbf_sim* s, uint32_t scene, const pbf_params* p)
         PBF_CUDA(s, cudaMemcpy(s->d_consts + scene, &s->sdc[scene], sizeof(DevConsts),
                                cudaMemcpyHostToDevice));
     invalidate_graph(s);
-    free_tape(s);  // a recorded run is only valid for the parameters it ran with
+    invalidate_tape(s);  // a recorded run is only valid for the parameters it ran with
     s->auto_trial = -1;  // a running trial's events may not match the new iteration count
     PBF_CUDA(s, ensure_lists(s));
     return PBF_OK;

@@ -112,6 +112,9 @@ struct Recording {
     float4* OM = nullptr;
     float4* Q = nullptr;
     float4* ETA = nullptr;
+    // the pair lists the sweeps write and replay instead of the handle's, one
+    // per iteration and the vorticity passes' last (NULL: the handle's)
+    const PairLists* lists = nullptr;
 };
 
 pbf_status fail(pbf_sim* s, pbf_status st, const std::string& msg);
@@ -122,6 +125,10 @@ pbf_status check_status(pbf_sim* s);
 cudaError_t enqueue_substep(pbf_sim* s, cudaEvent_t* ev, const Recording* rec = nullptr);
 void invalidate_graph(pbf_sim* s);
 void free_tape(pbf_sim* s);
+// Drops the recorded run but keeps its buffers for the next one.
+void invalidate_tape(pbf_sim* s);
+// Frees the buffers when they hold no recorded run; whether it freed any.
+bool free_idle_tape(pbf_sim* s);
 
 struct DeviceGuard {
     int prev = -1;
