@@ -214,7 +214,7 @@ __device__ __forceinline__ void adj_replay(uint32_t i, const DevConsts& c, const
                                            F&& f) {
     const int32_t cnt = pl.cnt[i];
     const uint32_t* p = pl.idx + i;
-    if (cnt > 0) {  // the next index is loaded one entry ahead
+    if (cnt > 0 && check_ok(c, (uint32_t)cnt <= pl.cap)) {  // the next index is loaded one entry ahead
         uint32_t jn = p[0];
 #pragma unroll 1
         for (int32_t k = 0; k < cnt; ++k) {
@@ -225,11 +225,21 @@ __device__ __forceinline__ void adj_replay(uint32_t i, const DevConsts& c, const
     }
 }
 
+// Row o of particle i's key-cell stencil.
+__device__ __forceinline__ int2 adj_row(int o, uint32_t i, const DevConsts& c,
+                                        const AdjLists& al) {
+    const int2 be = __ldg(al.rows + (size_t)o * al.own.n + i);
+    if (!check_ok(c, be.x >= 0 && be.x <= be.y && (uint32_t)be.y <= c.n_total))
+        return make_int2(0, 0);
+    return be;
+}
+
 template <class F>
-__device__ __forceinline__ void adj_visit_rows(uint32_t i, const AdjLists& al, F&& f) {
+__device__ __forceinline__ void adj_visit_rows(uint32_t i, const DevConsts& c, const AdjLists& al,
+                                               F&& f) {
 #pragma unroll 1
     for (int o = 0; o < 9; ++o) {
-        const int2 be = __ldg(al.rows + (size_t)o * al.own.n + i);
+        const int2 be = adj_row(o, i, c, al);
         for (int32_t j = be.x; j < be.y; ++j)
             if ((uint32_t)j != i) f((uint32_t)j);
     }
@@ -246,14 +256,14 @@ __device__ __forceinline__ void adj_visit_first(uint32_t i, const DevConsts& c,
     }
     const PairLists& own = al.own;
     if (!own.cap) {
-        adj_visit_rows(i, al, f);
+        adj_visit_rows(i, c, al, f);
         return;
     }
     uint32_t tot = 0;
     uint32_t* const out = own.idx + i;
 #pragma unroll 1
     for (int o = 0; o < 9; ++o) {
-        const int2 be = __ldg(al.rows + (size_t)o * own.n + i);
+        const int2 be = adj_row(o, i, c, al);
         const int32_t e = be.y;
 #pragma unroll 1
         for (int32_t base = be.x; base < e; base += 32) {
@@ -282,7 +292,7 @@ __device__ __forceinline__ void adj_visit_first(uint32_t i, const DevConsts& c,
         adj_replay(i, c, own, f);
     } else {
         own.cnt[i] = -1;
-        adj_visit_rows(i, al, f);
+        adj_visit_rows(i, c, al, f);
     }
 }
 
@@ -295,7 +305,7 @@ __device__ __forceinline__ void adj_visit_again(uint32_t i, const DevConsts& c,
     else if (al.own.cap && al.own.cnt[i] >= 0)
         adj_replay(i, c, al.own, f);
     else
-        adj_visit_rows(i, al, f);
+        adj_visit_rows(i, c, al, f);
 }
 
 // ---- a warp per particle for dense stencils ---------------------------------------
@@ -313,10 +323,11 @@ __device__ __forceinline__ void adj_visit_again(uint32_t i, const DevConsts& c,
 // deterministic.
 
 template <class F>
-__device__ __forceinline__ void warp_visit(uint32_t i, const AdjLists& al, uint32_t lane, F&& f) {
+__device__ __forceinline__ void warp_visit(uint32_t i, const DevConsts& c, const AdjLists& al,
+                                           uint32_t lane, F&& f) {
 #pragma unroll 1
     for (int o = 0; o < 9; ++o) {
-        const int2 be = __ldg(al.rows + (size_t)o * al.own.n + i);
+        const int2 be = adj_row(o, i, c, al);
 #pragma unroll 1
         for (int32_t j = be.x + (int32_t)lane; j < be.y; j += 32)
             if ((uint32_t)j != i) f((uint32_t)j);
@@ -404,12 +415,15 @@ k_adj_flags(const uint32_t* __restrict__ perm, const float4* __restrict__ XPc,
     }
 }
 
+// Blocks per SM each body is compiled for (Body::kBlocksPerSM): 4 (64 registers)
+// fit every body without spills; the delta-p body alone would take 71 and run
+// 3.  Measured, 1.2 million particles: delta-p 318 -> 250 us per launch.
 // One neighbour reversal (Body::run<W>): blocks below `tblocks` take a
 // thread per unflagged particle, the blocks after them a warp per flagged
 // particle (in turn, from the list).
 template <class Body>
-__global__ void __launch_bounds__(kAdjBlock) k_adj_sweep(Body b, Heavy hv, uint32_t n,
-                                                         uint32_t tblocks) {
+__global__ void __launch_bounds__(kAdjBlock, Body::kBlocksPerSM)
+k_adj_sweep(Body b, Heavy hv, uint32_t n, uint32_t tblocks) {
     if (blockIdx.x < tblocks) {
         const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
         if (i >= n || (hv.flag && hv.flag[i])) return;
@@ -421,7 +435,10 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_sweep(Body b, Heavy hv, uint3
     const uint32_t nw = ((gridDim.x - tblocks) * blockDim.x) >> 5;
     const uint32_t cnt = min(*hv.count, n);
 #pragma unroll 1
-    for (uint32_t k = w; k < cnt; k += nw) b.template run<true>(hv.list[k], lane);
+    for (uint32_t k = w; k < cnt; k += nw) {
+        const uint32_t i = hv.list[k];
+        if (check_ok(b.cp.at(0), i < n)) b.template run<true>(i, lane);
+    }
 }
 
 // vorticity.glsl:76-85 reversed, pointwise: from vf-bar to vs-bar, eta-bar and
@@ -458,6 +475,7 @@ k_adj_vort_b1(const uint32_t* __restrict__ perm, const float4* __restrict__ VB,
 // and the position adjoint, then folds |w|-bar into w-bar.
 template <class CP>
 struct AdjVortB2 {
+    static constexpr int kBlocksPerSM = 4;
     const uint32_t* __restrict__ perm;
     const float4* __restrict__ Q;
     const float4* __restrict__ OM;
@@ -470,6 +488,7 @@ struct AdjVortB2 {
     template <bool W>
     __device__ __forceinline__ void run(uint32_t i, uint32_t lane) const {
         const uint32_t id = perm[i];
+        if (!check_ok(cp.at(0), id < cp.at(0).n_total)) return;
         const DevConsts& c = consts_of(cp, id);
         const float4 Qi = Q[i];
         const float3 pi = f3(Qi);
@@ -490,7 +509,7 @@ struct AdjVortB2 {
             pb = pb + sp.H(d, (own * Qj.w) * ebi - mi * ebj);
         };
         if constexpr (W) {
-            warp_visit(i, al, lane, pair);
+            warp_visit(i, c, al, lane, pair);
             mb = warp_sum(mb);
             pb = warp_sum(pb);
             if (lane) return;
@@ -508,6 +527,7 @@ struct AdjVortB2 {
 // committed-velocity adjoint and adds the position adjoint; accumulates d/dc.
 template <class CP>
 struct AdjVortA {
+    static constexpr int kBlocksPerSM = 4;
     const uint32_t* __restrict__ perm;
     const float4* __restrict__ PF;
     const float4* __restrict__ VS;
@@ -522,6 +542,7 @@ struct AdjVortA {
     template <bool W>
     __device__ __forceinline__ void run(uint32_t i, uint32_t lane) const {
         const uint32_t id = perm[i];
+        if (!check_ok(cp.at(0), id < cp.at(0).n_total)) return;
         const DevConsts& c = consts_of(cp, id);
         const float3 pi = f3(PF[i]);
         const float3 vi = f3(VS[i]);
@@ -551,7 +572,7 @@ struct AdjVortA {
             pb = pb + sp.H(d, crossf(wbs, vji));
         };
         if constexpr (W) {
-            warp_visit(i, al, lane, pair);
+            warp_visit(i, c, al, lane, pair);
             vb = sbi + warp_sum(vb);
             pb = f3(PA[i]) + warp_sum(pb);
             wsum = warp_sum(wsum);
@@ -597,6 +618,7 @@ k_adj_commit(const uint32_t* __restrict__ perm, const float4* __restrict__ XB,
 // accumulates d/d(eps) and d/dk.
 template <class CP>
 struct AdjDeltaP {
+    static constexpr int kBlocksPerSM = 4;
     const uint32_t* __restrict__ perm;
     const float4* __restrict__ L;
     const float4* __restrict__ AUX;
@@ -611,6 +633,7 @@ struct AdjDeltaP {
     template <bool W>
     __device__ __forceinline__ void run(uint32_t i, uint32_t lane) const {
         const uint32_t id = perm[i];
+        if (!check_ok(cp.at(0), id < cp.at(0).n_total)) return;
         const DevConsts& c = consts_of(cp, id);
         const float4 Li = L[i];
         const float3 pi = f3(Li);
@@ -642,7 +665,7 @@ struct AdjDeltaP {
             kb -= own * c.oorho * dotf(qbi, G) * sc4 * W3 * W6;
         };
         if constexpr (W) {
-            warp_visit(i, al, lane, pair);
+            warp_visit(i, c, al, lane, pair);
             lb = warp_sum(lb);
             kb = warp_sum(kb);
             pb = qbi + warp_sum(pb);
@@ -666,6 +689,7 @@ struct AdjDeltaP {
 // the predicted-position adjoint after the first iteration.
 template <class CP>
 struct AdjLambda {
+    static constexpr int kBlocksPerSM = 4;
     const uint32_t* __restrict__ perm;
     const float4* __restrict__ L;
     const float4* __restrict__ AUX;
@@ -680,6 +704,7 @@ struct AdjLambda {
     template <bool W>
     __device__ __forceinline__ void run(uint32_t i, uint32_t lane) const {
         const uint32_t id = perm[i];
+        if (!check_ok(cp.at(0), id < cp.at(0).n_total)) return;
         const DevConsts& c = consts_of(cp, id);
         const float3 pi = f3(L[i]);
         const float4 RSi = RS[i];
@@ -701,7 +726,7 @@ struct AdjLambda {
             pb = pb + (2.0f * c.oorho) * sp.H(d, u);
         };
         if constexpr (W) {
-            warp_visit(i, al, lane, pair);
+            warp_visit(i, c, al, lane, pair);
             pb = f3(PDB[i]) + warp_sum(pb);
             if (lane) return;
         } else {

@@ -239,7 +239,8 @@ __device__ __forceinline__ void visit_masked(uint32_t i, const DevConsts& c,
     };
 #pragma unroll 1
     for (int o = 0; o < 9; ++o) {
-        const int2 be = __ldg(rows + (size_t)o * n + i);
+        int2 be = __ldg(rows + (size_t)o * n + i);
+        if (!check_ok(c, be.x >= 0 && be.x <= be.y && (uint32_t)be.y <= n)) be = make_int2(0, 0);
         const int32_t b = be.x, e = be.y;
 #pragma unroll 1
         for (int32_t base = b & ~1; base < e; base += 32) {

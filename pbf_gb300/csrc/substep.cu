@@ -224,7 +224,7 @@ __device__ __forceinline__ bool visit_pairs(uint32_t i, const DevConsts& c, cons
                                             F&& f) {
     if (!pl.cap) return false;
     const int32_t cnt = pl.cnt[i];
-    if (cnt < 0) return false;
+    if (cnt < 0 || !check_ok(c, (uint32_t)cnt <= pl.cap)) return false;
     const uint32_t* __restrict__ p = pl.idx + i;
     if (cnt > 0) {  // the next index is loaded one entry ahead
         uint32_t jn = __ldg(p);
@@ -792,7 +792,11 @@ __device__ __forceinline__ float coop_visit(uint32_t i, const DevConsts& c,
     const int lane = (int)(threadIdx.x & 31u);
     const uint32_t before = (1u << lane) - 1u;
     int2 mine = make_int2(0, lane == 9 ? 0x7FFFFFFF : 0);  // row 9 ends the sequence
-    if (lane < 9) mine = __ldg(rows + (size_t)lane * n + i);
+    if (lane < 9) {
+        mine = __ldg(rows + (size_t)lane * n + i);
+        if (!check_ok(c, mine.x >= 0 && mine.x <= mine.y && (uint32_t)mine.y <= n))
+            mine = make_int2(0, 0);
+    }
     if (lane < 10) sm.run[lane] = mine;
     const bool look = __reduce_add_sync(kFull, lane < 9 ? (uint32_t)(mine.y - mine.x) : 0u) >=
                       kCoopRunsFrom;
@@ -922,7 +926,7 @@ struct CoopWork {
     const uint32_t nwarps_ = (gridDim.x * blockDim.x) >> 5;                                    \
     const uint32_t total_ = wk.list ? *wk.count : n;                                           \
     for (uint32_t w_ = warp0_; w_ < total_; w_ += nwarps_)                                     \
-        if (const uint32_t i = wk.list ? wk.list[w_] : w_; true)
+        if (const uint32_t i = wk.list ? wk.list[w_] : w_; check_ok(cp.at(0), i < n))
 
 template <class CP>
 __global__ void __launch_bounds__(kBlock)
