@@ -70,6 +70,26 @@ k_unmark_cells(const uint32_t* __restrict__ prev_sorted, uint32_t n, uint32_t nc
     if (k < ncells && (i == 0 || prev_sorted[i - 1] != k)) cstart[k] = -1;
 }
 
+// Marks every cell empty (-1 in both tables): one launch, 16-byte stores where
+// both tables are aligned for them.
+__global__ void __launch_bounds__(kBlock)
+k_empty_cells(int32_t* __restrict__ start, int32_t* __restrict__ end, uint32_t ncells, bool wide) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t c = 4u * i;
+    if (c >= ncells) return;
+    if (wide && ncells - c >= 4u) {
+        const int4 none = make_int4(-1, -1, -1, -1);
+        reinterpret_cast<int4*>(start)[i] = none;
+        reinterpret_cast<int4*>(end)[i] = none;
+    } else {
+        for (uint32_t k = c; k < ncells && k < c + 4u; ++k) start[k] = end[k] = -1;
+    }
+}
+void launch_empty_cells(cudaStream_t st, int32_t* start, int32_t* end, uint32_t ncells) {
+    const bool wide = (((uintptr_t)start | (uintptr_t)end) & 15u) == 0u;
+    k_empty_cells<<<grid_for(ncells / 4u + 1u), kBlock, 0, st>>>(start, end, ncells, wide);
+}
+
 // The run-start bit of sorted particle j (neighbours.cuh: runs) from its
 // position p and the previous particle's q, with the warp's 32 bits stored
 // by its first lane.  Call with every lane of the warp.
