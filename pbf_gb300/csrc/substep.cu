@@ -1385,7 +1385,9 @@ void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4*
                     NbrLists nl, PairLists pr, ScanPos sx, ScanPos sx_out, int dmax_slot,
                     int out_slot, uint32_t n, CP cp, uint32_t* status) {
     if (sw.mode == kCoop) {
-        k_delta_p_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(L, Pn, ScanPos{nullptr, nullptr}, n, cp, status,
+        // (with its scan copy where the vorticity passes scan it: they may run
+        // under another configuration than the solver)
+        k_delta_p_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(L, Pn, sx_out, n, cp, status,
                                                             CoopWork{nullptr, nullptr, pr.rows});
         return;
     }
