@@ -367,18 +367,36 @@ __device__ __forceinline__ const DevConsts& consts_of(const CP& cp, uint32_t id)
 // Stencil rows around the key cell of every particle, from the cell tables of
 // the substep just recorded (the reverse sweeps read the rows, so the tables
 // need not be kept).
-template <class CP>
-__global__ void __launch_bounds__(kAdjBlock)
+// kWide: one thread per particle and row, a warp per row of 32 particles (as in
+// k_stencil_rows: where threads are few).
+constexpr int kAdjRowsBlock = 9 * 32;
+constexpr uint32_t kAdjWideRowsBelow = 131072;
+template <bool kWide, class CP>
+__global__ void __launch_bounds__(kAdjRowsBlock)
 k_adj_rows(const uint32_t* __restrict__ perm, const float4* __restrict__ XPc,
            const int32_t* __restrict__ cstart, const int32_t* __restrict__ cend,
            int2* __restrict__ rows, uint32_t n, CP cp) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = kWide ? blockIdx.x * 32u + (threadIdx.x & 31u)
+                             : blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const DevConsts& c = consts_of(cp, perm[i]);
     const int3 cell = key_cell(XPc[i], c);
 #pragma unroll
-    for (int o = 0; o < 9; ++o)
+    for (int r = 0; r < (kWide ? 1 : 9); ++r) {
+        const int o = kWide ? (int)(threadIdx.x >> 5) : r;
         rows[(size_t)o * n + i] = run_of_row(o, cell, c, cstart, cend);
+    }
+}
+template <class CP>
+void launch_adj_rows(cudaStream_t st, const uint32_t* perm, const float4* XPc,
+                     const int32_t* cstart, const int32_t* cend, int2* rows, uint32_t n,
+                     const CP& cp) {
+    if (n < kAdjWideRowsBelow)
+        k_adj_rows<true><<<grid_for(n, 32), kAdjRowsBlock, 0, st>>>(perm, XPc, cstart, cend, rows,
+                                                                    n, cp);
+    else
+        k_adj_rows<false><<<grid_for(n, kAdjBlock), kAdjBlock, 0, st>>>(perm, XPc, cstart, cend,
+                                                                        rows, n, cp);
 }
 
 // Per substep: irr[i] = 1 when particle i's stencil centre is not its key
@@ -930,7 +948,6 @@ cudaError_t reverse_dispatch(pbf_sim* s, Tape* t, const Tape::Slot& sl) {
 cudaError_t record_segment(pbf_sim* s, Tape* t, uint32_t seg, uint32_t count) {
     cudaStream_t st = s->stream;
     const size_t n = s->n;
-    const unsigned g = grid_for(s->n, kAdjBlock);
     t->held = Tape::kNone;
     for (uint32_t k = 0; k < count; ++k) {
         Tape::Slot& sl = t->slots[k];
@@ -957,11 +974,10 @@ cudaError_t record_segment(pbf_sim* s, Tape* t, uint32_t seg, uint32_t count) {
         if (e != cudaSuccess) return e;
         const float4* XPc = t->iters > 0 ? sl.L[0] : sl.PF;
         if (s->nscenes == 1)
-            k_adj_rows<<<g, kAdjBlock, 0, st>>>(sl.perm, XPc, s->cstart, s->cend, sl.rows, s->n,
-                                                OneScene{s->dc});
+            launch_adj_rows(st, sl.perm, XPc, s->cstart, s->cend, sl.rows, s->n, OneScene{s->dc});
         else
-            k_adj_rows<<<g, kAdjBlock, 0, st>>>(sl.perm, XPc, s->cstart, s->cend, sl.rows, s->n,
-                                                ManyScenes{s->d_consts, s->sid});
+            launch_adj_rows(st, sl.perm, XPc, s->cstart, s->cend, sl.rows, s->n,
+                            ManyScenes{s->d_consts, s->sid});
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

@@ -153,6 +153,12 @@ constexpr uint32_t kCoopBelow = 32768;
 // 5.7 masked, before the direct sweeps skipped pile runs) and loses once
 // every particle is over the threshold, so it is not a default.
 constexpr uint32_t kMixedCandidates = 256;
+static_assert(kMixedCandidates <= kQuadCandidates, "the quad sweeps take every light particle");
+
+// The cooperative and mixed configurations take the quad sweeps below this many
+// particles (from kQuadScanBelow the second sweeps only: substep.cu has the
+// figures; from here a thread per particle fills the GPU).
+constexpr uint32_t kQuadBelow = 131072;
 
 pbf_tuning default_tuning() {
     pbf_tuning t{};
@@ -197,7 +203,8 @@ void pick_trial_candidates(pbf_sim* s) {
                                         s->n >= kCoopBelow);
 }
 
-// SweepCfg modes (0 direct, 1 masked, 2 masked + pair lists, 3 cooperative)
+// SweepCfg modes (0 direct, 1 masked, 2 masked + pair lists, 3 cooperative; 4
+// quads, see pass_quads)
 // of a pass's first and second sweep.
 struct PassModes {
     int first, second;
@@ -226,9 +233,27 @@ bool pass_mixed(const pbf_sim* s, uint32_t pass) {
     const PassModes m = modes_of(s, pass);
     return m.first != 3 || m.second != 3;
 }
+uint32_t heavy_threshold(const pbf_sim* s) {
+    return s->tuning.coop_candidates ? s->tuning.coop_candidates : kMixedCandidates;
+}
+// Whether a pass gives its particles four lanes each (the quad sweeps,
+// substep.cu) instead of a thread or a warp, leaving the heavy ones to warps:
+// in scenes below kQuadBelow particles, the cooperative and the mixed
+// configurations; they need the pair lists, and at most 256 candidates of a
+// particle that is not heavy.
+bool pass_quads(const pbf_sim* s, uint32_t pass) {
+    if (s->n >= kQuadBelow || !s->pair_cap || skin_lists_on(s) ||
+        heavy_threshold(s) > kQuadCandidates)
+        return false;
+    return (pass == PBF_PASS_COOP && s->n < kQuadScanBelow) || pass == PBF_PASS_MIXED;
+}
+// Whether a pass leaves its heavy particles to warps.
+bool pass_splits(const pbf_sim* s, uint32_t pass) {
+    return pass_mixed(s, pass) || pass_quads(s, pass);
+}
 bool mixed_on(const pbf_sim* s) {
     const bool vort = s->params.vorticity_confinement != 0;
-    return pass_mixed(s, s->pass_solver) || (vort && pass_mixed(s, s->pass_vort));
+    return pass_splits(s, s->pass_solver) || (vort && pass_splits(s, s->pass_vort));
 }
 // Whether some sweep of the substep reads the stencil rows: the direct sweeps
 // alone walk the cells themselves.
@@ -239,9 +264,6 @@ bool rows_on(const pbf_sim* s) {
     };
     return mixed_on(s) || reads(s->pass_solver) ||
            (s->params.vorticity_confinement != 0 && reads(s->pass_vort));
-}
-uint32_t heavy_threshold(const pbf_sim* s) {
-    return s->tuning.coop_candidates ? s->tuning.coop_candidates : kMixedCandidates;
 }
 
 // Host-side fault injection (pbf_debug_fail_allocation): when armed, the
@@ -362,8 +384,12 @@ uint32_t kernels_per_substep(const pbf_sim* s) {
     if (rows_on(s)) k += 1u;
     if (mixed_on(s)) {  // a cooperative launch after each one-thread sweep
         const PassModes a = modes_of(s, s->pass_solver), b = modes_of(s, s->pass_vort);
-        if (pass_mixed(s, s->pass_solver)) k += iters * ((a.first != 3) + (a.second != 3));
-        if (vort && pass_mixed(s, s->pass_vort)) k += (uint32_t)((b.first != 3) + (b.second != 3));
+        auto extra = [&](uint32_t pass, const PassModes& m) {
+            if (pass_quads(s, pass)) return 2u;
+            return pass_mixed(s, pass) ? (uint32_t)((m.first != 3) + (m.second != 3)) : 0u;
+        };
+        k += iters * extra(s->pass_solver, a);
+        if (vort) k += extra(s->pass_vort, b);
     }
     return k;
 }
@@ -487,7 +513,11 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
     const unsigned g = grid_for(n);
     const unsigned blk = s->tuning.block_size ? s->tuning.block_size : (unsigned)kBlock;
     const bool lists = skin_lists_on(s);
-    const PassModes ms = modes_of(s, s->pass_solver), mv = modes_of(s, s->pass_vort);
+    auto modes = [&](uint32_t pass) {
+        return !pass_quads(s, pass) ? modes_of(s, pass)
+               : s->n < kQuadScanBelow ? PassModes{4, 4} : PassModes{2, 4};
+    };
+    const PassModes ms = modes(s->pass_solver), mv = modes(s->pass_vort);
     const SweepCfg s_lam{blk, ms.first, lists}, s_dp{blk, ms.second, lists},
         s_va{blk, mv.first, lists}, s_vb{blk, mv.second, lists};
     const bool vort = s->params.vorticity_confinement != 0;
@@ -529,7 +559,7 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
             cudaError_t me = cudaMemsetAsync(s->heavy_count, 0, sizeof(uint32_t), st);
             if (me != cudaSuccess) return me;
         }
-        launch_stencil_rows(g, st, s->XP, s->cstart, s->cend, heavy_threshold(s), n, cps, s->rows,
+        launch_stencil_rows(st, s->XP, s->cstart, s->cend, heavy_threshold(s), n, cps, s->rows,
                             mixed ? s->heavy : nullptr, s->heavy_list, s->heavy_count);
     }
     mark(3);
@@ -547,8 +577,8 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
     const bool runs_solver = lam_direct || dp_direct;
     const bool runs_vort = va_direct || vb_direct;
     // the heavy list goes only to the passes that leave heavy particles to warps
-    const bool mix_s = mixed && pass_mixed(s, s->pass_solver);
-    const bool mix_v = mixed && pass_mixed(s, s->pass_vort);
+    const bool mix_s = mixed && pass_splits(s, s->pass_solver);
+    const bool mix_v = mixed && pass_splits(s, s->pass_vort);
     const PairLists pl{s->pair_idx, s->pair_cnt, s->pair_cap, n, mix_s ? s->heavy : nullptr,
                        s->heavy_list, s->heavy_count,
                        runs_solver || runs_vort ? s->runs : nullptr, s->rows};

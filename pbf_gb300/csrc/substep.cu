@@ -948,6 +948,44 @@ struct CoopWork {
     for (uint32_t w_ = warp0_; w_ < total_; w_ += nwarps_)                                     \
         if (const uint32_t i = wk.list ? wk.list[w_] : w_; check_ok(cp.at(0), i < n))
 
+// What one lane does with a particle's sums.
+// updatepos.glsl:100: the clamp as min(max(q, lo), hi) with explicit selects,
+// so signed zeros and NaN behave like the oracle's std::min/std::max.
+__device__ __forceinline__ void store_position(uint32_t i, float3 q, const DevConsts& c,
+                                               float4* __restrict__ Pn, const ScanPos& sx_out,
+                                               uint32_t* status) {
+    q.x = (q.x < c.lo[0]) ? c.lo[0] : q.x;
+    q.x = (c.hi[0] < q.x) ? c.hi[0] : q.x;
+    q.y = (q.y < c.lo[1]) ? c.lo[1] : q.y;
+    q.y = (c.hi[1] < q.y) ? c.hi[1] : q.y;
+    q.z = (q.z < c.lo[2]) ? c.lo[2] : q.z;
+    q.z = (c.hi[2] < q.z) ? c.hi[2] : q.z;
+    if (!finite3(q)) atomicOr(status, kDevNonFinite);
+    Pn[i] = make_float4(q.x, q.y, q.z, 0.0f);
+    if (sx_out.xy) scanpos_store(sx_out, i, q.x, q.y, q.z);
+}
+__device__ __forceinline__ void store_vorticity(uint32_t i, float3 pi, float3 vi, float3 acc,
+                                                float3 w, const DevConsts& c,
+                                                float4* __restrict__ VX, float4* __restrict__ OM,
+                                                float4* __restrict__ Q) {
+    const float3 vx = fma3(c.cx, acc, vi);  // vorticity.glsl:58
+    VX[i] = make_float4(vx.x, vx.y, vx.z, 0.0f);
+    OM[i] = make_float4(w.x, w.y, w.z, 0.0f);
+    Q[i] = make_float4(pi.x, pi.y, pi.z, fsqrt(dot3(w, w)));  // :60
+}
+__device__ __forceinline__ void store_velocity(uint32_t i, float3 eta, const DevConsts& c,
+                                               const float4* __restrict__ VX,
+                                               const float4* __restrict__ OM,
+                                               const uint32_t* __restrict__ perm,
+                                               float4* __restrict__ v,
+                                               float4* __restrict__ eta_out) {
+    if (eta_out) eta_out[i] = make_float4(eta.x, eta.y, eta.z, 0.0f);
+    const float l = fsqrt(dot3(eta, eta));  // vorticity.glsl:76
+    if (l > 0.0f) eta = make_float3(fdiv(eta.x, l), fdiv(eta.y, l), fdiv(eta.z, l));  // :77-78
+    const float3 vf = fma3(c.dteps, cross3(eta, xyz(OM[i])), xyz(VX[i]));  // :82
+    if (check_ok(c, perm[i] < c.n_total)) v[perm[i]] = make_float4(vf.x, vf.y, vf.z, 0.0f);  // :85
+}
+
 template <class CP>
 __global__ void __launch_bounds__(kBlock)
 k_lambda_coop(const float4* __restrict__ P, float4* __restrict__ L, float4* __restrict__ aux,
@@ -974,18 +1012,8 @@ k_delta_p_coop(const float4* __restrict__ L, float4* __restrict__ Pn, ScanPos sx
         const float3 pi = xyz(Li);
         const float s = coop_visit(i, c, wk.rows, n, L, pi, sm, CoopDeltaP{Li.w});
         const float3 dp = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
-        if ((threadIdx.x & 31u) == 0u) {
-            float3 q = fma3(c.oorho, dp, pi);  // :85
-            q.x = (q.x < c.lo[0]) ? c.lo[0] : q.x;
-            q.x = (c.hi[0] < q.x) ? c.hi[0] : q.x;
-            q.y = (q.y < c.lo[1]) ? c.lo[1] : q.y;
-            q.y = (c.hi[1] < q.y) ? c.hi[1] : q.y;
-            q.z = (q.z < c.lo[2]) ? c.lo[2] : q.z;
-            q.z = (c.hi[2] < q.z) ? c.hi[2] : q.z;
-            if (!finite3(q)) atomicOr(status, kDevNonFinite);
-            Pn[i] = make_float4(q.x, q.y, q.z, 0.0f);
-            if (sx_out.xy) scanpos_store(sx_out, i, q.x, q.y, q.z);
-        }
+        if ((threadIdx.x & 31u) == 0u)
+            store_position(i, fma3(c.oorho, dp, pi), c, Pn, sx_out, status);  // :85
     }
 }
 
@@ -1001,12 +1029,7 @@ k_vorticity_a_coop(const float4* __restrict__ P, const float4* __restrict__ VS,
         const float s = coop_visit(i, c, wk.rows, n, P, pi, sm, CoopVortA{VS, vi});
         const float3 acc = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
         const float3 w = make_float3(shf(s, 3), shf(s, 4), shf(s, 5));
-        if ((threadIdx.x & 31u) == 0u) {
-            const float3 vx = fma3(c.cx, acc, vi);  // :58
-            VX[i] = make_float4(vx.x, vx.y, vx.z, 0.0f);
-            OM[i] = make_float4(w.x, w.y, w.z, 0.0f);
-            Q[i] = make_float4(pi.x, pi.y, pi.z, fsqrt(dot3(w, w)));  // :60
-        }
+        if ((threadIdx.x & 31u) == 0u) store_vorticity(i, pi, vi, acc, w, c, VX, OM, Q);
     }
 }
 
@@ -1020,15 +1043,332 @@ k_vorticity_b_coop(const float4* __restrict__ Q, const float4* __restrict__ VX,
         const auto& c = cp.at(i);
         const float3 pi = xyz(Q[i]);
         const float s = coop_visit(i, c, wk.rows, n, Q, pi, sm, CoopVortB{});
-        float3 eta = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
-        if ((threadIdx.x & 31u) == 0u) {
-            if (eta_out) eta_out[i] = make_float4(eta.x, eta.y, eta.z, 0.0f);
-            const float l = fsqrt(dot3(eta, eta));  // :76
-            if (l > 0.0f) eta = make_float3(fdiv(eta.x, l), fdiv(eta.y, l), fdiv(eta.z, l));  // :77-78
-            const float3 vf = fma3(c.dteps, cross3(eta, xyz(OM[i])), xyz(VX[i]));  // :82
-            v[perm[i]] = make_float4(vf.x, vf.y, vf.z, 0.0f);                     // :85
+        const float3 eta = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
+        if ((threadIdx.x & 31u) == 0u) store_velocity(i, eta, c, VX, OM, perm, v, eta_out);
+    }
+}
+
+// ---- quad sweeps: four or eight lanes per particle ------------------------------------------
+//
+// For scenes between the two: a thread per particle leaves each SM a few warps
+// whose every step waits for the one before it (at 32,768 particles, 7 warps
+// per SM and 26 us per lambda launch of 8 us worth of instructions), a warp per
+// particle spends five times the instructions.  A group of G lanes shares a
+// particle of at most kQuadCandidates stencil candidates; the scene's others are
+// listed (k_stencil_rows) and take a warp each.  Lane q tests the q-th part of
+// the particle's flattened candidate sequence, eight candidates at a time, and
+// keeps those in range in its column of shared memory; the columns in turn are
+// the particle's pair list.  The pair terms are evaluated G entries at a time,
+// one per lane, and folded in list order by lane c (sums c and c + G), as in the
+// cooperative sweeps: the same terms in the same order, so the same bits.  The
+// second sweep over a position set replays the list the same way.
+//
+// Measured, us per launch, before and after (lambda / delta-p / vorticity A /
+// B): 16,384 particles (a warp each before) 17.9 -> 13.6, 18.2 -> 5.1, 22.2 ->
+// 14.5, 19.4 -> 5.2; 32,768 (a thread each) 26.0 -> 18.5, 14.8 -> 6.9, 29.7 ->
+// 21.0, 15.1 -> 7.0; 65,536 (two blocks, 32 candidates per particle) delta-p
+// 11.9 -> 10.0, but lambda 19.2 -> 23.9: there only the second sweeps are quads.
+// What bounds it now: latency (scan of 16,384: 5.8 of 13.6 us, the pairs 4.4).
+constexpr int kQuad = 4;  // SweepCfg mode
+constexpr int kQuadBlock = 64;
+// A lane's share of a particle's candidates.
+template <int G>
+constexpr int kQuadShare = (int)kQuadCandidates / G;
+template <int G>
+struct QuadTerms {
+    // term rows of G entries, two rounds in turn (padded against bank conflicts)
+    float t[2][32 / G][8 * G + 4];
+};
+template <int G>
+struct QuadScan {
+    uint16_t found[kQuadShare<G>][32];  // each lane's candidates in range, a column per lane
+    int2 run[32 / G][10];               // the rows; the tenth ends the sequence
+};
+static_assert(kQuadScanBelow <= 65536, "QuadScan::found holds 16-bit indices");
+
+// One of a few registers by index.
+template <int N>
+__device__ __forceinline__ float pick(const float (&t)[N], int k) {
+    float v = t[0];
+#pragma unroll
+    for (int i = 1; i < N; ++i) v = k == i ? t[i] : v;
+    return v;
+}
+
+// The sums of a group's particle: lane q keeps sum q in `a` and sum q + G in `b`.
+template <int G>
+struct QuadSums {
+    float a = 0.0f, b = 0.0f;
+    __device__ __forceinline__ float get(int k) const {  // every lane of the warp calls
+        return __shfl_sync(kFull, k < G ? a : b, k & (G - 1), G);
+    }
+};
+
+template <class Op, int G>
+__device__ __forceinline__ float quad_fold(float acc, const float* t, int c, uint32_t valid) {
+#pragma unroll
+    for (int k = 0; k < G; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(t + G * Op::a_row(c) + k);
+        const uint32_t v = valid >> k;
+        if constexpr (Op::kAdd) {
+            if (v & 1u) acc = fadd(acc, a.x);
+            if (v & 2u) acc = fadd(acc, a.y);
+            if (v & 4u) acc = fadd(acc, a.z);
+            if (v & 8u) acc = fadd(acc, a.w);
+        } else {
+            const float4 s = *reinterpret_cast<const float4*>(t + G * Op::s_row(c) + k);
+            if (v & 1u) acc = ffma(s.x, a.x, acc);
+            if (v & 2u) acc = ffma(s.y, a.y, acc);
+            if (v & 4u) acc = ffma(s.z, a.z, acc);
+            if (v & 8u) acc = ffma(s.w, a.w, acc);
         }
     }
+    return acc;
+}
+
+// Adds the pairs of the first m list entries (entry(k) is the candidate of
+// entry k < m) to the particle's sums.  Every lane of the warp calls; m is the
+// same on the lanes of a group.  The next round's record and the entry after it
+// are loaded ahead: with a few warps per SM a round otherwise waits for both.
+template <class Op, int G, class E>
+__device__ __forceinline__ void quad_pairs(uint32_t m, const DevConsts& c,
+                                           const float4* __restrict__ X, float3 pi,
+                                           QuadTerms<G>& sm, const Op& op, QuadSums<G>& sums,
+                                           E&& entry) {
+    const uint32_t q = threadIdx.x & (G - 1), part = (threadIdx.x & 31u) / G;
+    const uint32_t most = __reduce_max_sync(kFull, m);
+    uint32_t j1 = 0u, j2 = 0u;
+    float4 x1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (q < m) j1 = entry(q);
+    if (!check_ok(c, j1 < c.n_total)) j1 = 0u;
+    if (q < m) x1 = __ldg(X + j1);
+    if (q + G < m) j2 = entry(q + G);
+    int turn = 0;
+#pragma unroll 1
+    for (uint32_t k = q; k - q < most; k += G, turn ^= 1) {
+        const uint32_t j = j1;
+        const float4 xj = x1;
+        j1 = check_ok(c, j2 < c.n_total) ? j2 : 0u;
+        if (k + G < m) x1 = __ldg(X + j1);
+        if (k + 2 * G < m) j2 = entry(k + 2 * G);
+        bool has = k < m;
+        if (has) {
+            const float3 d = sub3(pi, xyz(xj));
+            const float r2 = dot3(d, d);
+            has = !(r2 > c.r2cut) && !(Op::kSkipCoincident && r2 == 0.0f);
+            if (has) {
+                float t[Op::kRows];
+                op.terms(c, d, r2, op.payload(j, xj), t);
+#pragma unroll
+                for (int r = 0; r < Op::kRows; ++r) sm.t[turn][part][G * r + q] = t[r];
+            }
+        }
+        const uint32_t valid = __ballot_sync(kFull, has) >> (threadIdx.x & 31u & ~(G - 1u));
+        __syncwarp();
+        const float* const t = sm.t[turn][part];
+        if (q < Op::kSums) sums.a = quad_fold<Op, G>(sums.a, t, (int)q, valid);
+        if (q + G < Op::kSums) sums.b = quad_fold<Op, G>(sums.b, t, (int)q + G, valid);
+    }
+    __syncwarp();
+}
+
+// The pairs in visit order, one after the other on all lanes of the group: for a
+// particle whose pair list was too short.
+template <class Op, int G>
+__device__ __forceinline__ void quad_walk(uint32_t i, const DevConsts& c,
+                                          const PairLists& pl, const float4* __restrict__ X,
+                                          float3 pi, const Op& op, QuadSums<G>& sums) {
+    const int q = (int)(threadIdx.x & (G - 1));
+#pragma unroll 1
+    for (int o = 0; o < 9; ++o) {
+        const int2 be = __ldg(pl.rows + (size_t)o * pl.n + i);
+#pragma unroll 1
+        for (int32_t j = be.x; j < be.y; ++j) {
+            const float4 xj = __ldg(X + j);
+            const float3 d = sub3(pi, xyz(xj));
+            const float r2 = dot3(d, d);
+            if ((uint32_t)j == i || r2 > c.r2cut) continue;
+            if (Op::kSkipCoincident && r2 == 0.0f) continue;
+            float t[Op::kRows];
+            op.terms(c, d, r2, op.payload((uint32_t)j, xj), t);
+            auto add = [&](float acc, int k) {
+                const float a = pick(t, Op::a_row(k));
+                return Op::kAdd ? fadd(acc, a) : ffma(pick(t, Op::s_row(k)), a, acc);
+            };
+            if (q < Op::kSums) sums.a = add(sums.a, q);
+            if (q + G < Op::kSums) sums.b = add(sums.b, q + G);
+        }
+    }
+}
+
+// First sweep over a position set X: scans, records particle
+// i's pair list and sums its pairs.  Every lane of the warp calls.
+template <int G, class Op>
+__device__ __forceinline__ QuadSums<G> quad_scan(uint32_t i, bool live, const DevConsts& c,
+                                                 const PairLists& pl,
+                                                 const float4* __restrict__ X, float3 pi,
+                                                 QuadTerms<G>& sm, QuadScan<G>& sc,
+                                                 const Op& op) {
+    const int lane = (int)(threadIdx.x & 31u), q = lane & (G - 1), part = lane / G;
+    for (int o = q; o < 9; o += G) {
+        int2 be = make_int2(0, 0);
+        if (live) be = __ldg(pl.rows + (size_t)o * pl.n + i);
+        if (!check_ok(c, be.x >= 0 && be.x <= be.y && (uint32_t)be.y <= pl.n))
+            be = make_int2(0, 0);
+        sc.run[part][o] = be;
+    }
+    if (q == 0) sc.run[part][9] = make_int2(0, 0x7FFFFFFF);
+    __syncwarp();
+    int total = 0;
+#pragma unroll
+    for (int o = 0; o < 9; ++o) total += sc.run[part][o].y - sc.run[part][o].x;
+    if (!check_ok(c, total <= (int)kQuadCandidates)) total = 0;
+    // this lane's share: `left` candidates from position `at` of row o
+    int at = total * q / G, o = 0;
+    int left = total * (q + 1) / G - at;
+    int2 be = sc.run[part][0];
+    while (at >= be.y - be.x) {
+        at -= be.y - be.x;
+        be = sc.run[part][++o];
+    }
+    int j = be.x + at;
+    uint32_t count = 0;
+    // eight candidates at a time, across rows: a scene this small waits for the
+    // first touch of every line, so eight loads are in flight
+#pragma unroll 1
+    for (; left > 0; left -= 8) {
+        int js[8];
+        float4 x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            js[k] = k < left ? j : -1;
+            ++j;
+            while (j >= be.y && o < 9) {  // into the next row that is not empty
+                be = sc.run[part][++o];
+                j = be.x;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = __ldg(X + max(js[k], 0));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float3 d = sub3(pi, xyz(x[k]));
+            if (js[k] >= 0 && !(dot3(d, d) > c.r2cut) && (uint32_t)js[k] != i)
+                sc.found[count++][lane] = (uint16_t)js[k];
+        }
+    }
+    // the group's entries in visit order: lane q's follow those of the lanes before
+    uint32_t upto = count;
+#pragma unroll
+    for (int d = 1; d < G; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, upto, d, G);
+        if (q >= d) upto += v;
+    }
+    const uint32_t tot = __shfl_sync(kFull, upto, G - 1, G);
+    uint32_t ends[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) ends[g] = __shfl_sync(kFull, upto, g, G);
+    uint32_t* const out = pl.idx + i;
+    for (uint32_t k = 0, rank = upto - count; k < count && rank < pl.cap; ++k, ++rank)
+        out[(size_t)rank * pl.n] = sc.found[k][lane];
+    if (live && q == 0) pl.cnt[i] = tot <= pl.cap ? (int32_t)tot : -1;
+    __syncwarp();
+    QuadSums<G> sums;
+    quad_pairs(tot, c, X, pi, sm, op, sums, [&](uint32_t k) {
+        uint32_t before = 0u;
+        int who = 0;
+#pragma unroll
+        for (int g = 0; g + 1 < G; ++g)
+            if (k >= ends[g]) {
+                before = ends[g];
+                who = g + 1;
+            }
+        return (uint32_t)sc.found[k - before][part * G + who];
+    });
+    return sums;
+}
+
+// Second sweep: replays the list.  Every lane of the warp calls.
+template <int G, class Op>
+__device__ __forceinline__ QuadSums<G> quad_replay(uint32_t i, bool live, const DevConsts& c,
+                                                   const PairLists& pl,
+                                                   const float4* __restrict__ X, float3 pi,
+                                                   QuadTerms<G>& sm, const Op& op) {
+    const int32_t cnt = live ? pl.cnt[i] : 0;
+    const uint32_t m = cnt > 0 && check_ok(c, (uint32_t)cnt <= pl.cap) ? (uint32_t)cnt : 0u;
+    const uint32_t* const in = pl.idx + i;
+    QuadSums<G> sums;
+    quad_pairs(m, c, X, pi, sm, op, sums,
+               [&](uint32_t k) { return __ldg(in + (size_t)k * pl.n); });
+    if (cnt < 0) quad_walk(i, c, pl, X, pi, op, sums);
+    __syncwarp();
+    return sums;
+}
+
+// Particle, liveness and constants of a quad; the lanes past the end and those
+// of listed (heavy) particles run along with nothing to do.
+#define PBF_QUAD_PARTICLE(pl)                                                                 \
+    __shared__ QuadTerms<G> terms_[kQuadBlock / 32];                                          \
+    QuadTerms<G>& sm = terms_[threadIdx.x >> 5];                                              \
+    const uint32_t own_ = (blockIdx.x * blockDim.x + threadIdx.x) / G;                        \
+    const bool live = own_ < n && !(pl.heavy && pl.heavy[own_]);                              \
+    const uint32_t i = live ? own_ : 0u;                                                      \
+    const auto& c = cp.at(i);                                                                 \
+    const bool writes = live && (threadIdx.x & (G - 1)) == 0u
+
+template <class CP, int G>
+__global__ void __launch_bounds__(kQuadBlock)
+k_lambda_quad(const float4* __restrict__ P, float4* __restrict__ L, float4* __restrict__ aux,
+              PairLists pw, uint32_t n, CP cp) {
+    PBF_QUAD_PARTICLE(pw);
+    __shared__ QuadScan<G> scan_[kQuadBlock / 32];
+    const float3 pi = xyz(P[i]);
+    const QuadSums<G> s = quad_scan<G>(i, live, c, pw, P, pi, sm, scan_[threadIdx.x >> 5], CoopLambda{});
+    const LambdaAcc a{s.get(0), s.get(1), make_float3(s.get(2), s.get(3), s.get(4))};
+    if (writes) {
+        L[i] = make_float4(pi.x, pi.y, pi.z, lambda_finish(c, a));
+        if (aux) aux[i] = lambda_aux(a);
+    }
+}
+
+template <class CP, int G>
+__global__ void __launch_bounds__(kQuadBlock)
+k_delta_p_quad(const float4* __restrict__ L, float4* __restrict__ Pn, PairLists pr, ScanPos sx_out,
+               uint32_t n, CP cp, uint32_t* status) {
+    PBF_QUAD_PARTICLE(pr);
+    const float4 Li = L[i];
+    const float3 pi = xyz(Li);
+    const QuadSums<G> s = quad_replay<G>(i, live, c, pr, L, pi, sm, CoopDeltaP{Li.w});
+    const float3 dp = make_float3(s.get(0), s.get(1), s.get(2));
+    if (writes) store_position(i, fma3(c.oorho, dp, pi), c, Pn, sx_out, status);  // :85
+}
+
+template <class CP, int G>
+__global__ void __launch_bounds__(kQuadBlock)
+k_vorticity_a_quad(const float4* __restrict__ P, const float4* __restrict__ VS,
+                   float4* __restrict__ VX, float4* __restrict__ OM, float4* __restrict__ Q,
+                   PairLists pw, uint32_t n, CP cp) {
+    PBF_QUAD_PARTICLE(pw);
+    __shared__ QuadScan<G> scan_[kQuadBlock / 32];
+    const float3 pi = xyz(P[i]);
+    const float3 vi = xyz(VS[i]);
+    const QuadSums<G> s = quad_scan<G>(i, live, c, pw, P, pi, sm, scan_[threadIdx.x >> 5], CoopVortA{VS, vi});
+    const float3 acc = make_float3(s.get(0), s.get(1), s.get(2));
+    const float3 w = make_float3(s.get(3), s.get(4), s.get(5));
+    if (writes) store_vorticity(i, pi, vi, acc, w, c, VX, OM, Q);
+}
+
+template <class CP, int G>
+__global__ void __launch_bounds__(kQuadBlock)
+k_vorticity_b_quad(const float4* __restrict__ Q, const float4* __restrict__ VX,
+                   const float4* __restrict__ OM, const uint32_t* __restrict__ perm,
+                   float4* __restrict__ v, float4* __restrict__ eta_out, PairLists pr, uint32_t n,
+                   CP cp) {
+    PBF_QUAD_PARTICLE(pr);
+    const float3 pi = xyz(Q[i]);
+    const QuadSums<G> s = quad_replay<G>(i, live, c, pr, Q, pi, sm, CoopVortB{});
+    const float3 eta = make_float3(s.get(0), s.get(1), s.get(2));
+    if (writes) store_velocity(i, eta, c, VX, OM, perm, v, eta_out);
 }
 
 // The substep's stencil rows: row o of sorted particle i, [x, y), at
@@ -1037,50 +1377,56 @@ k_vorticity_b_coop(const float4* __restrict__ Q, const float4* __restrict__ VX,
 // substep reads them (9 coalesced 8-byte loads) instead of repeating the 27
 // cell lookups, the bounds tests and the merging (~500 instructions, and a
 // 72-byte local array) in each of its scanning sweeps.
-// Mixed sweeps (heavy != nullptr): the particles with more than `threshold`
-// stencil candidates go to the cooperative kernels and are listed here; the
-// one-thread kernels skip them.  A block appends its heavy particles in
-// ascending order (one atomic per block), so consecutive warps of a
-// cooperative launch work on neighbouring particles.
-template <class CP>
-__global__ void __launch_bounds__(kBlock)
+// kWide: one thread per particle and row, a warp per row of 32 particles.  The
+// three cell lookups of a row wait for each other, so nine rows in one thread
+// are slow where threads are few; where they are many, the nine-fold particle
+// reads cost more.  Measured, us, a thread per particle / per row: 16,384
+// particles 8.9 / 3.1, 65,536 8.5 / 5.9, 2,097,152 72 / 143.
+// Mixed and quad sweeps (heavy != nullptr): the particles with more than
+// `threshold` stencil candidates go to the cooperative kernels and are listed
+// here; the other kernels skip them.  A warp appends its heavy particles in
+// ascending order (one atomic), so consecutive warps of a cooperative launch
+// work on neighbouring particles.
+constexpr int kRowsBlock = 9 * 32;
+constexpr uint32_t kWideRowsBelow = 131072;
+template <class CP, bool kWide>
+__global__ void __launch_bounds__(kRowsBlock)
 k_stencil_rows(const float4* __restrict__ XP, const int32_t* __restrict__ cstart,
                const int32_t* __restrict__ cend, uint32_t threshold, uint32_t n, CP cp,
                int2* __restrict__ rows, uint8_t* __restrict__ heavy, uint32_t* __restrict__ list,
                uint32_t* __restrict__ count) {
-    __shared__ uint32_t warp_off[kBlock / 32];
-    __shared__ uint32_t base;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    bool h = false;
+    __shared__ uint32_t cand[kWide ? 9 : 1][32];
+    const uint32_t lane = threadIdx.x & 31u, o = threadIdx.x >> 5;
+    const uint32_t i = kWide ? blockIdx.x * 32u + lane : blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t total = 0;
     if (i < n) {
         const auto& c = cp.at(i);
         const int3 ctr = stencil_centre(XP[i], c);  // neighbourcells.glsl:57
-        uint32_t cand = 0;
 #pragma unroll
-        for (int o = 0; o < 9; ++o) {
-            const int2 be = run_of_row(o, ctr, c, cstart, cend);
-            rows[(size_t)o * n + i] = be;
-            cand += (uint32_t)(be.y - be.x);
+        for (int r = 0; r < (kWide ? 1 : 9); ++r) {
+            const int row = kWide ? (int)o : r;
+            const int2 be = run_of_row(row, ctr, c, cstart, cend);
+            rows[(size_t)row * n + i] = be;
+            total += (uint32_t)(be.y - be.x);
         }
-        h = cand > threshold;
-        if (heavy) heavy[i] = h ? 1 : 0;
     }
     if (!heavy) return;
-    const uint32_t m = __ballot_sync(0xffffffffu, h);
-    if (lane == 0) warp_off[wid] = __popc(m);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
-            const uint32_t c = warp_off[w];
-            warp_off[w] = t;
-            t += c;
-        }
-        base = t ? atomicAdd(count, t) : 0u;
+    if constexpr (kWide) {
+        cand[o][lane] = total;
+        __syncthreads();
+        if (o != 0u) return;
+        total = 0;
+#pragma unroll
+        for (int r = 0; r < 9; ++r) total += cand[r][lane];
     }
-    __syncthreads();
-    if (h) list[base + warp_off[wid] + __popc(m & ((1u << lane) - 1u))] = i;
+    const bool h = total > threshold;
+    if (i < n) heavy[i] = h ? 1 : 0;
+    const uint32_t m = __ballot_sync(0xffffffffu, h);
+    if (m == 0u) return;
+    uint32_t base = 0;
+    if (lane == 0u) base = atomicAdd(count, (uint32_t)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (h) list[base + __popc(m & ((1u << lane) - 1u))] = i;
 }
 
 // Grid of the cooperative kernels of a mixed sweep (the heavy list's length is
@@ -1088,6 +1434,19 @@ k_stencil_rows(const float4* __restrict__ XP, const int32_t* __restrict__ cstart
 constexpr unsigned kHeavyGrid = 152 * 8;
 
 // Grid of warps, one per particle.
+// Grid and launch of a quad sweep: eight lanes per particle below kOctsBelow
+// particles (shorter chains), four above (fewer instructions).  Four / eight
+// lanes, us: 16,384 particles lambda 13.7 / 13.6, delta-p 6.2 / 5.1; 32,768
+// lambda 18.5 / 27.6, delta-p 6.9 / 8.8.
+constexpr uint32_t kOctsBelow = 24576;
+inline unsigned quad_grid(uint32_t n, uint32_t lanes) { return grid_for(lanes * n, kQuadBlock); }
+#define PBF_QUAD_LAUNCH(KERNEL, ...)                                                     \
+    do {                                                                                 \
+        if (n < kOctsBelow)                                                              \
+            KERNEL<CP, 8><<<quad_grid(n, 8), kQuadBlock, 0, st>>>(__VA_ARGS__);          \
+        else                                                                             \
+            KERNEL<CP, 4><<<quad_grid(n, 4), kQuadBlock, 0, st>>>(__VA_ARGS__);          \
+    } while (0)
 inline unsigned coop_grid(uint32_t n) { return (unsigned)(((size_t)n * 32 + kBlock - 1) / kBlock); }
 
 // update.glsl:16-28: v = (x* - x_old) / dt, x = x*, scattered back to id order.
@@ -1359,7 +1718,10 @@ void launch_lambda_build(SweepCfg sw, cudaStream_t st, const float4* XP, const u
                                                            CoopWork{nullptr, nullptr, pw.rows});
         return;
     }
-    PBF_SWEEP_LAUNCH(k_lambda_build, XP, skeys, cstart, cend, L, aux, nl, pw, sx, n, cp);
+    if (sw.mode == kQuad)
+        PBF_QUAD_LAUNCH(k_lambda_quad, XP, L, aux, pw, n, cp);
+    else
+        PBF_SWEEP_LAUNCH(k_lambda_build, XP, skeys, cstart, cend, L, aux, nl, pw, sx, n, cp);
     if (pw.heavy)
         k_lambda_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(XP, L, aux, n, cp,
                                                          CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
@@ -1374,7 +1736,10 @@ void launch_lambda(SweepCfg sw, cudaStream_t st, const float4* P, const float4* 
                                                            CoopWork{nullptr, nullptr, pw.rows});
         return;
     }
-    PBF_SWEEP_LAUNCH(k_lambda, P, XP, skeys, cstart, cend, L, aux, nl, pw, sx, dmax_slot, n, cp);
+    if (sw.mode == kQuad)
+        PBF_QUAD_LAUNCH(k_lambda_quad, P, L, aux, pw, n, cp);
+    else
+        PBF_SWEEP_LAUNCH(k_lambda, P, XP, skeys, cstart, cend, L, aux, nl, pw, sx, dmax_slot, n, cp);
     if (pw.heavy)
         k_lambda_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(P, L, aux, n, cp,
                                                          CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
@@ -1391,7 +1756,10 @@ void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4*
                                                             CoopWork{nullptr, nullptr, pr.rows});
         return;
     }
-    PBF_SWEEP_LAUNCH(k_delta_p, L, XP, skeys, cstart, cend, Pn, nl, pr, sx, sx_out, dmax_slot,
+    if (sw.mode == kQuad)
+        PBF_QUAD_LAUNCH(k_delta_p_quad, L, Pn, pr, sx_out, n, cp, status);
+    else
+        PBF_SWEEP_LAUNCH(k_delta_p, L, XP, skeys, cstart, cend, Pn, nl, pr, sx, sx_out, dmax_slot,
                      out_slot, n, cp, status);
     if (pr.heavy)
         k_delta_p_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(L, Pn, sx_out, n, cp,
@@ -1399,11 +1767,15 @@ void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4*
                                                           CoopWork{pr.heavy_list, pr.heavy_count, pr.rows});
 }
 template <class CP>
-void launch_stencil_rows(unsigned g, cudaStream_t st, const float4* XP, const int32_t* cstart,
+void launch_stencil_rows(cudaStream_t st, const float4* XP, const int32_t* cstart,
                          const int32_t* cend, uint32_t threshold, uint32_t n, CP cp, int2* rows,
                          uint8_t* heavy, uint32_t* list, uint32_t* count) {
-    k_stencil_rows<CP><<<g, kBlock, 0, st>>>(XP, cstart, cend, threshold, n, cp, rows, heavy, list,
-                                             count);
+    if (n < kWideRowsBelow)
+        k_stencil_rows<CP, true><<<grid_for(n, 32), kRowsBlock, 0, st>>>(
+            XP, cstart, cend, threshold, n, cp, rows, heavy, list, count);
+    else
+        k_stencil_rows<CP, false><<<grid_for(n, kBlock), kBlock, 0, st>>>(
+            XP, cstart, cend, threshold, n, cp, rows, heavy, list, count);
 }
 template <class CP>
 void launch_commit(unsigned g, cudaStream_t st, const float4* P, const uint32_t* perm, float4* x,
@@ -1420,7 +1792,10 @@ void launch_vorticity_a(SweepCfg sw, cudaStream_t st, const float4* P, const flo
                                                                n, cp, CoopWork{nullptr, nullptr, pw.rows});
         return;
     }
-    PBF_SWEEP_LAUNCH(k_vorticity_a, P, XP, VS, skeys, cstart, cend, VX, OM, Q, nl, pw, sx, dmax_slot,
+    if (sw.mode == kQuad)
+        PBF_QUAD_LAUNCH(k_vorticity_a_quad, P, VS, VX, OM, Q, pw, n, cp);
+    else
+        PBF_SWEEP_LAUNCH(k_vorticity_a, P, XP, VS, skeys, cstart, cend, VX, OM, Q, nl, pw, sx, dmax_slot,
                      n, cp);
     if (pw.heavy)
         k_vorticity_a_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(
@@ -1437,7 +1812,10 @@ void launch_vorticity_b(SweepCfg sw, cudaStream_t st, const float4* Q, const flo
                                                                eta_out, n, cp, CoopWork{nullptr, nullptr, pr.rows});
         return;
     }
-    PBF_SWEEP_LAUNCH(k_vorticity_b, Q, XP, VX, OM, skeys, perm, cstart, cend, v, eta_out, nl, pr, sx,
+    if (sw.mode == kQuad)
+        PBF_QUAD_LAUNCH(k_vorticity_b_quad, Q, VX, OM, perm, v, eta_out, pr, n, cp);
+    else
+        PBF_SWEEP_LAUNCH(k_vorticity_b, Q, XP, VX, OM, skeys, perm, cstart, cend, v, eta_out, nl, pr, sx,
                      dmax_slot, n, cp);
     if (pr.heavy)
         k_vorticity_b_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(
@@ -1466,7 +1844,7 @@ void launch_diagnostics(unsigned g, cudaStream_t st, const float4* P, const floa
                                      const uint32_t*, const int32_t*, const int32_t*, float4*,  \
                                      NbrLists, PairLists, ScanPos, ScanPos, int, int, uint32_t, \
                                      CP, uint32_t*);                                            \
-    template void launch_stencil_rows<CP>(unsigned, cudaStream_t, const float4*, const int32_t*, \
+    template void launch_stencil_rows<CP>(cudaStream_t, const float4*, const int32_t*,         \
                                           const int32_t*, uint32_t, uint32_t, CP, int2*,         \
                                           uint8_t*, uint32_t*, uint32_t*);                       \
     template void launch_commit<CP>(unsigned, cudaStream_t, const float4*, const uint32_t*,     \
@@ -1516,7 +1894,16 @@ cudaError_t preload_sweeps() {
     load((const void*)k_delta_p_coop<CP>);
     load((const void*)k_vorticity_a_coop<CP>);
     load((const void*)k_vorticity_b_coop<CP>);
-    load((const void*)k_stencil_rows<CP>);
+    load((const void*)k_lambda_quad<CP, 4>);
+    load((const void*)k_lambda_quad<CP, 8>);
+    load((const void*)k_delta_p_quad<CP, 4>);
+    load((const void*)k_delta_p_quad<CP, 8>);
+    load((const void*)k_vorticity_a_quad<CP, 4>);
+    load((const void*)k_vorticity_a_quad<CP, 8>);
+    load((const void*)k_vorticity_b_quad<CP, 4>);
+    load((const void*)k_vorticity_b_quad<CP, 8>);
+    load((const void*)k_stencil_rows<CP, true>);
+    load((const void*)k_stencil_rows<CP, false>);
     load((const void*)k_run_flags);
     load((const void*)k_run_flags_vals);
     return e;

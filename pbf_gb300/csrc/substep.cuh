@@ -26,6 +26,11 @@ __global__ void k_find_cells(const uint32_t* __restrict__ skeys, const uint32_t*
 // (0: the reference's loop shape, visit_full; 1: masked scans, visit_masked;
 // 2: masked scans that record the exact pair lists the next sweep replays);
 // whether the skin-radius neighbour lists are used.
+// The quad sweeps (substep.cu) take particles of at most this many stencil
+// candidates, and as first sweeps (which scan) scenes below this many particles.
+constexpr uint32_t kQuadCandidates = 256;
+constexpr uint32_t kQuadScanBelow = 49152;
+
 struct SweepCfg {
     unsigned block;
     int mode;
@@ -57,7 +62,7 @@ void launch_empty_cells(cudaStream_t st, int32_t* start, int32_t* end, uint32_t 
 template <class CP>
 cudaError_t preload_sweeps();
 template <class CP>
-void launch_stencil_rows(unsigned g, cudaStream_t st, const float4* XP, const int32_t* cstart,
+void launch_stencil_rows(cudaStream_t st, const float4* XP, const int32_t* cstart,
                          const int32_t* cend, uint32_t threshold, uint32_t n, CP cp, int2* rows,
                          uint8_t* heavy, uint32_t* list, uint32_t* count);
 template <class CP>
