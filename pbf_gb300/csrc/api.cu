@@ -233,6 +233,23 @@ bool pass_mixed(const pbf_sim* s, uint32_t pass) {
     const PassModes m = modes_of(s, pass);
     return m.first != 3 || m.second != 3;
 }
+// Threads per block of the scanning sweeps under the default block size.  The
+// blocks that share an SM come from all over the particle order, so a larger
+// block means fewer places whose records and lists have to fit in the SM's L1;
+// it also waits longer for its slowest warp.  Measured at 256 / 512 / 1024
+// threads, us per launch: 9.3 million particles in 256 scenes lambda 2,410 /
+// 2,159 / 1,976, vorticity A (at most 512: registers) 2,570 / 2,328; 2,097,152
+// lambda 466 / 454 / 464, vorticity A 541 / 537; 1.2 million lambda 259 / 263 /
+// 278; 250,000 lambda 57.5 / 62.3 / 61.6.
+constexpr uint32_t kMidScene = 1572864, kLargeScene = 4194304;
+unsigned lam_block(const pbf_sim* s, unsigned blk) {
+    if (blk != (unsigned)kBlock) return blk;
+    return s->n < kMidScene ? blk : s->n < kLargeScene ? 512u : 1024u;
+}
+unsigned vort_block(const pbf_sim* s, unsigned blk) {
+    if (blk != (unsigned)kBlock) return blk;
+    return s->n < kMidScene ? blk : 512u;
+}
 uint32_t heavy_threshold(const pbf_sim* s) {
     return s->tuning.coop_candidates ? s->tuning.coop_candidates : kMixedCandidates;
 }
@@ -518,8 +535,8 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
                : s->n < kQuadScanBelow ? PassModes{4, 4} : PassModes{2, 4};
     };
     const PassModes ms = modes(s->pass_solver), mv = modes(s->pass_vort);
-    const SweepCfg s_lam{blk, ms.first, lists}, s_dp{blk, ms.second, lists},
-        s_va{blk, mv.first, lists}, s_vb{blk, mv.second, lists};
+    const SweepCfg s_lam{lam_block(s, blk), ms.first, lists}, s_dp{blk, ms.second, lists},
+        s_va{vort_block(s, blk), mv.first, lists}, s_vb{blk, mv.second, lists};
     const bool vort = s->params.vorticity_confinement != 0;
     // delta-p writes the scan copy of its output when a sweep reading that
     // position set scans through it (masked modes; a pair-list replay falls

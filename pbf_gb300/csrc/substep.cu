@@ -392,7 +392,11 @@ constexpr int kSweepBlocksPerSM = 8;
 // XSPH and vorticity sums, the velocity, the run path's repeated steps): 6
 // blocks per SM (40 registers) keep it from spilling; measured 10% faster
 // than 8 blocks with spills on the 2M window.
-constexpr int kVortBlocksPerSM = 6;
+constexpr int kVortThreadsPerSM = 1536;
+
+// Largest blocks the scanning sweeps are launched with (api.cu: lam_block,
+// vort_block), at the same registers per thread.
+constexpr int kLambdaMaxBlock = 1024, kVortMaxBlock = 512;
 
 // Instantiations of the sweep kernels (pbf_tuning): MODE is the stencil scan
 // (kDirect: the reference's loop shape; kMasked: masked scans; kPairs: masked
@@ -406,7 +410,7 @@ constexpr int kDirect = 0, kMasked = 1, kPairs = 2;
 // candidate within h + skin (the neighbour list of the later sweeps) and the
 // largest coordinate magnitude (for the guard's rounding margin).
 template <class CP, int MODE, bool LISTS>
-__global__ void __launch_bounds__(kBlock, kSweepBlocksPerSM)
+__global__ void __launch_bounds__(kLambdaMaxBlock, 2048 / kLambdaMaxBlock)
 k_lambda_build(const float4* __restrict__ XP, const uint32_t* __restrict__ skeys,
                const int32_t* __restrict__ cstart, const int32_t* __restrict__ cend,
                float4* __restrict__ L, float4* __restrict__ aux, NbrLists nl, PairLists pw,
@@ -493,7 +497,7 @@ k_lambda_build(const float4* __restrict__ XP, const uint32_t* __restrict__ skeys
 // calclambda.glsl:66-102 at positions P (iterations after the first).
 // dmax_slot: guard slot holding the largest displacement of P from XP.
 template <class CP, int MODE, bool LISTS>
-__global__ void __launch_bounds__(kBlock, kSweepBlocksPerSM)
+__global__ void __launch_bounds__(kLambdaMaxBlock, 2048 / kLambdaMaxBlock)
 k_lambda(const float4* __restrict__ P, const float4* __restrict__ XP,
          const uint32_t* __restrict__ skeys, const int32_t* __restrict__ cstart,
          const int32_t* __restrict__ cend, float4* __restrict__ L, float4* __restrict__ aux,
@@ -1430,8 +1434,12 @@ k_stencil_rows(const float4* __restrict__ XP, const int32_t* __restrict__ cstart
 }
 
 // Grid of the cooperative kernels of a mixed sweep (the heavy list's length is
-// only known on the device): 8 blocks of 8 warps per SM.
-constexpr unsigned kHeavyGrid = 152 * 8;
+// only known on the device): 8 blocks of 8 warps per SM, and 20 for large scenes,
+// whose listed particles differ more in work (the blocks that find no more than
+// one entry each even it out; 2,097,152 particles, per launch: lambda 79 -> 71
+// us, delta-p 58.5 -> 53.5).  An empty launch takes 1.7 and 2.6 us.  A ticket
+// counter per launch instead was slower (lambda 87 us, 5.2 us empty).
+inline unsigned heavy_grid(uint32_t n) { return 152u * (n < 1048576u ? 8u : 20u); }
 
 // Grid of warps, one per particle.
 // Grid and launch of a quad sweep: eight lanes per particle below kOctsBelow
@@ -1473,7 +1481,7 @@ k_commit(const float4* __restrict__ P, const uint32_t* __restrict__ perm, float4
 // vorticity.glsl:34-60: XSPH velocity and the vorticity vector, Jacobi
 // (every read sees the committed velocities).
 template <class CP, int MODE, bool LISTS>
-__global__ void __launch_bounds__(kBlock, kVortBlocksPerSM)
+__global__ void __launch_bounds__(kVortMaxBlock, kVortThreadsPerSM / kVortMaxBlock)
 k_vorticity_a(const float4* __restrict__ P, const float4* __restrict__ XP,
               const float4* __restrict__ VS, const uint32_t* __restrict__ skeys,
               const int32_t* __restrict__ cstart, const int32_t* __restrict__ cend,
@@ -1723,7 +1731,7 @@ void launch_lambda_build(SweepCfg sw, cudaStream_t st, const float4* XP, const u
     else
         PBF_SWEEP_LAUNCH(k_lambda_build, XP, skeys, cstart, cend, L, aux, nl, pw, sx, n, cp);
     if (pw.heavy)
-        k_lambda_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(XP, L, aux, n, cp,
+        k_lambda_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(XP, L, aux, n, cp,
                                                          CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
 }
 template <class CP>
@@ -1741,7 +1749,7 @@ void launch_lambda(SweepCfg sw, cudaStream_t st, const float4* P, const float4* 
     else
         PBF_SWEEP_LAUNCH(k_lambda, P, XP, skeys, cstart, cend, L, aux, nl, pw, sx, dmax_slot, n, cp);
     if (pw.heavy)
-        k_lambda_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(P, L, aux, n, cp,
+        k_lambda_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(P, L, aux, n, cp,
                                                          CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
 }
 template <class CP>
@@ -1762,7 +1770,7 @@ void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4*
         PBF_SWEEP_LAUNCH(k_delta_p, L, XP, skeys, cstart, cend, Pn, nl, pr, sx, sx_out, dmax_slot,
                      out_slot, n, cp, status);
     if (pr.heavy)
-        k_delta_p_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(L, Pn, sx_out, n, cp,
+        k_delta_p_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(L, Pn, sx_out, n, cp,
                                                           status,
                                                           CoopWork{pr.heavy_list, pr.heavy_count, pr.rows});
 }
@@ -1798,7 +1806,7 @@ void launch_vorticity_a(SweepCfg sw, cudaStream_t st, const float4* P, const flo
         PBF_SWEEP_LAUNCH(k_vorticity_a, P, XP, VS, skeys, cstart, cend, VX, OM, Q, nl, pw, sx, dmax_slot,
                      n, cp);
     if (pw.heavy)
-        k_vorticity_a_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(
+        k_vorticity_a_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(
             P, VS, VX, OM, Q, n, cp, CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
 }
 template <class CP>
@@ -1818,7 +1826,7 @@ void launch_vorticity_b(SweepCfg sw, cudaStream_t st, const float4* Q, const flo
         PBF_SWEEP_LAUNCH(k_vorticity_b, Q, XP, VX, OM, skeys, perm, cstart, cend, v, eta_out, nl, pr, sx,
                      dmax_slot, n, cp);
     if (pr.heavy)
-        k_vorticity_b_coop<CP><<<kHeavyGrid, kBlock, 0, st>>>(
+        k_vorticity_b_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(
             Q, VX, OM, perm, v, eta_out, n, cp,
             CoopWork{pr.heavy_list, pr.heavy_count, pr.rows});
 }
