@@ -812,10 +812,14 @@ pbf_status pbf_create_batch(const pbf_params* scene_params, const uint32_t* scen
     if (e == cudaSuccess) e = cudaMemsetAsync(s->v, 0, sizeof(float4) * n, s->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->status, 0, 2 * sizeof(uint32_t), s->stream);
     if (e == cudaSuccess && num_scenes > 1) {
-        std::vector<uint32_t> sid(n);
-        for (uint32_t k = 0; k < num_scenes; ++k)
-            for (uint32_t i = s->offsets[k]; i < s->offsets[k + 1]; ++i) sid[i] = k;
-        e = cudaMemcpy(s->sid, sid.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice);
+        // (the offsets go through a buffer that the first substep overwrites)
+        e = cudaMemcpyAsync(s->skeys, s->offsets.data(), sizeof(uint32_t) * num_scenes,
+                            cudaMemcpyHostToDevice, s->stream);
+        if (e == cudaSuccess) {
+            launch_scene_ids(s->stream, s->skeys, num_scenes, n, s->sid);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaMemsetAsync(s->skeys, 0, sizeof(uint32_t) * n, s->stream);
         if (e == cudaSuccess)
             e = cudaMemcpy(s->d_consts, s->sdc.data(), sizeof(DevConsts) * num_scenes,
                            cudaMemcpyHostToDevice);

@@ -9,10 +9,20 @@ namespace pbf {
 
 constexpr uint32_t kMaxPasses = 4;     // 8-bit digits, 32-bit keys
 constexpr uint32_t kSortTile = 4096;   // keys per onesweep tile
+constexpr uint32_t kSortSmallTile = 1024;      // and below kSortSmallBelow keys
+constexpr uint32_t kSortSmallBelow = 131072;
+
+// Tiles of a sort of at most n keys (the most that any smaller count takes too).
+constexpr uint32_t sort_tiles(uint32_t n) {
+    const uint32_t small = n < kSortSmallBelow ? n : kSortSmallBelow - 1;
+    const uint32_t a = (uint32_t)(((uint64_t)n + kSortTile - 1) / kSortTile);
+    const uint32_t b = (small + kSortSmallTile - 1) / kSortSmallTile;
+    return a > b ? a : b;
+}
 
 // Bytes of the workspace SortWorkspace::carve lays out for up to n keys.
 constexpr size_t sort_ws_bytes(uint32_t n) {
-    const size_t tiles = ((size_t)n + kSortTile - 1) / kSortTile;
+    const size_t tiles = sort_tiles(n);
     size_t b = sizeof(uint32_t) * kMaxPasses * 256        // hist / digit base
                + sizeof(uint32_t) * kMaxPasses * 32       // tile counters (padded)
                + sizeof(uint32_t) * kMaxPasses * 256 * tiles;  // lookback status

@@ -70,6 +70,28 @@ k_unmark_cells(const uint32_t* __restrict__ prev_sorted, uint32_t n, uint32_t nc
     if (k < ncells && (i == 0 || prev_sorted[i - 1] != k)) cstart[k] = -1;
 }
 
+// The scene of every particle (id order): the last whose first particle is not
+// after it.
+__global__ void __launch_bounds__(kBlock)
+k_scene_ids(const uint32_t* __restrict__ first, uint32_t scenes, uint32_t n,
+            uint32_t* __restrict__ sid) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t lo = 0, hi = scenes;  // first[lo] <= i, and i < first[hi] or hi == scenes
+    while (hi - lo > 1u) {
+        const uint32_t mid = lo + (hi - lo) / 2u;
+        if (__ldg(first + mid) <= i)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    sid[i] = lo;
+}
+void launch_scene_ids(cudaStream_t st, const uint32_t* first, uint32_t scenes, uint32_t n,
+                      uint32_t* sid) {
+    k_scene_ids<<<grid_for(n), kBlock, 0, st>>>(first, scenes, n, sid);
+}
+
 // Marks every cell empty (-1 in both tables): one launch, 16-byte stores where
 // both tables are aligned for them.
 __global__ void __launch_bounds__(kBlock)

@@ -57,6 +57,8 @@ void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4*
                     const uint32_t* skeys, const int32_t* cstart, const int32_t* cend, float4* Pn,
                     NbrLists nl, PairLists pr, ScanPos sx, ScanPos sx_out, int dmax_slot,
                     int out_slot, uint32_t n, CP cp, uint32_t* status);
+void launch_scene_ids(cudaStream_t st, const uint32_t* first, uint32_t scenes, uint32_t n,
+                      uint32_t* sid);
 void launch_empty_cells(cudaStream_t st, int32_t* start, int32_t* end, uint32_t ncells);
 // Loads the sweep kernels the automatic configuration may launch.
 template <class CP>
