@@ -387,7 +387,7 @@ uint32_t kernels_per_substep(const pbf_sim* s) {
     const uint32_t passes = (s->numbits + 7) / 8;
     const uint32_t iters = s->params.num_solver_iterations;
     const bool vort = s->params.vorticity_confinement != 0;
-    uint32_t k = 1u /*predict*/ + 1u /*unmark*/ + 2u + passes /*sort*/ + 1u /*cells*/ +
+    uint32_t k = 1u /*predict*/ + 1u + passes /*sort*/ + 1u /*cells*/ +
                  2u * iters + 1u /*commit*/ + (vort ? 2u : 0u);
     {  // run-start bits before each direct sweep (enqueue_impl): the positions
        // of every lambda sweep after the first, (p, lambda) of every delta-p,
@@ -550,12 +550,12 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
         if (ev) cudaEventRecord(ev[idx], st);
     };
     mark(0);
-    // 1 predict (predictpos.glsl)
-    launch_predict(g, st, s->x, s->v, s->xstar, s->keys, n, cpi, s->status);
-    mark(1);
-    // 2 sort (RadixSort::Run); first clear the cell starts of the previous
+    // 1 predict (predictpos.glsl); first clears the cell starts of the previous
     // substep while its sorted keys are still there
-    k_unmark_cells<<<g, kBlock, 0, st>>>(s->skeys, n, s->ncells, s->cstart);
+    launch_predict(g, st, s->x, s->v, s->xstar, s->keys, n, cpi, s->status, s->skeys, s->ncells,
+                   s->cstart, s->heavy_count);
+    mark(1);
+    // 2 sort (RadixSort::Run)
     cudaError_t e = sort_pairs(s->sort, s->keys, s->skeys, s->perm, n, s->numbits, s->status, st);
     if (e != cudaSuccess) return e;
     mark(2);
@@ -572,10 +572,6 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
     // candidates: the cooperative kernels sweep those, the others skip them
     const bool mixed = mixed_on(s);
     if (rows_on(s)) {
-        if (mixed) {
-            cudaError_t me = cudaMemsetAsync(s->heavy_count, 0, sizeof(uint32_t), st);
-            if (me != cudaSuccess) return me;
-        }
         launch_stencil_rows(st, s->XP, s->cstart, s->cend, heavy_threshold(s), n, cps, s->rows,
                             mixed ? s->heavy : nullptr, s->heavy_list, s->heavy_count);
     }
@@ -611,8 +607,10 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
         return l;
     };
     pl_v = lists_of(pl_v, iters);
-    cudaError_t ge = cudaMemsetAsync(s->guard, 0, sizeof(uint32_t) * (2 + iters), st);
-    if (ge != cudaSuccess) return ge;
+    if (lists) {  // (only the skin lists read the guard)
+        cudaError_t ge = cudaMemsetAsync(s->guard, 0, sizeof(uint32_t) * (2 + iters), st);
+        if (ge != cudaSuccess) return ge;
+    }
     const float4* cur = s->XP;
     int cur_set = 0;  // scan copy of `cur`
     for (uint32_t it = 0; it < iters; ++it) {

@@ -91,32 +91,13 @@ k_sort_histogram(const uint32_t* __restrict__ keys, uint32_t n, uint32_t passes,
     }
 }
 
-// Exclusive scan of each pass's 256 digit counts; one CTA per pass.
-__global__ void __launch_bounds__(256) k_sort_digit_base(uint32_t* __restrict__ hist) {
-    __shared__ uint32_t s_warp[8];
-    uint32_t* h = hist + blockIdx.x * 256;
-    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    uint32_t v = h[t];
-    uint32_t inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= (uint32_t)o) inc += y;
-    }
-    if (lane == 31) s_warp[warp] = inc;
-    __syncthreads();
-    uint32_t wbase = 0;
-    for (uint32_t w = 0; w < warp; ++w) wbase += s_warp[w];
-    h[t] = wbase + inc - v;
-}
-
 // One onesweep pass over `n` keys, kItems per thread.  vin == nullptr means the
 // payload is the element index.
 template <int kItems>
 __global__ void __launch_bounds__(kSortThreads)
 k_onesweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
            uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n, uint32_t shift,
-           uint32_t dmask, const uint32_t* __restrict__ digit_base, uint32_t* tile_status, uint32_t* tile_counter,
+           uint32_t dmask, const uint32_t* __restrict__ hist, uint32_t* tile_status, uint32_t* tile_counter,
            uint32_t* status, const uint32_t* stall_word, uint32_t spin_limit) {
     constexpr uint32_t kTile = kSortThreads * kItems;
     __shared__ uint32_t s_k[kTile];
@@ -124,7 +105,7 @@ k_onesweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
     __shared__ uint32_t s_wh[kSortWarps][256];
     __shared__ uint32_t s_dstart[256];
     __shared__ uint32_t s_goff[256];
-    __shared__ uint32_t s_wsum[kSortWarps];
+    __shared__ uint32_t s_wsum[kSortWarps], s_hsum[kSortWarps];
     __shared__ uint32_t s_tile;
 
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -172,18 +153,32 @@ k_onesweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
     uint32_t* my_status = tile_status + (uint64_t)tile * 256 + d;
     store_volatile(my_status, (tile == 0 ? kFlagPrefix : kFlagAgg) | count);
 
-    // Tile-local digit starts: exclusive scan of the counts over digits.
-    uint32_t inc = count;
+    // Tile-local digit starts, and the digits' first places among all keys:
+    // exclusive scans over digits of the tile's counts and of the pass's
+    // histogram (a launch of its own for the latter took longer than each tile
+    // scanning it along).
+    const uint32_t in_all = hist[d];
+    uint32_t inc = count, hinc = in_all;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= (uint32_t)o) inc += y;
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        const uint32_t z = __shfl_up_sync(0xffffffffu, hinc, o);
+        if (lane >= (uint32_t)o) {
+            inc += y;
+            hinc += z;
+        }
     }
-    if (lane == 31) s_wsum[warp] = inc;
+    if (lane == 31) {
+        s_wsum[warp] = inc;
+        s_hsum[warp] = hinc;
+    }
     __syncthreads();
-    uint32_t wb = 0;
-    for (uint32_t w = 0; w < warp; ++w) wb += s_wsum[w];
-    const uint32_t dstart = wb + inc - count;
+    uint32_t wb = 0, hb = 0;
+    for (uint32_t w = 0; w < warp; ++w) {
+        wb += s_wsum[w];
+        hb += s_hsum[w];
+    }
+    const uint32_t dstart = wb + inc - count, digit_base = hb + hinc - in_all;
     s_dstart[d] = dstart;
 
     // Decoupled lookback over earlier tiles for digit d.
@@ -209,7 +204,7 @@ k_onesweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
         }
         store_volatile(my_status, kFlagPrefix | ((excl + count) & kValueMask));
     }
-    s_goff[d] = digit_base[d] + excl - dstart;
+    s_goff[d] = digit_base + excl - dstart;
     __syncthreads();
 
 #pragma unroll
@@ -278,7 +273,6 @@ cudaError_t sort_pairs(const SortWorkspace& ws, const uint32_t* keys_in, uint32_
     if (err != cudaSuccess) return err;
     const unsigned hgrid = std::min<unsigned>((n + kSortSmallTile - 1) / kSortSmallTile, 4u * 152u);
     k_sort_histogram<<<hgrid, kSortThreads, 0, stream>>>(keys_in, n, passes, numbits, ws.hist);
-    k_sort_digit_base<<<passes, 256, 0, stream>>>(ws.hist);
     // Pass p writes to the final buffers when (passes - 1 - p) is even, so the
     // last pass always lands in keys_out / vals_out and no pass reads the
     // buffer it writes.

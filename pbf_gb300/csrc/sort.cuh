@@ -23,7 +23,7 @@ constexpr uint32_t sort_tiles(uint32_t n) {
 // Bytes of the workspace SortWorkspace::carve lays out for up to n keys.
 constexpr size_t sort_ws_bytes(uint32_t n) {
     const size_t tiles = sort_tiles(n);
-    size_t b = sizeof(uint32_t) * kMaxPasses * 256        // hist / digit base
+    size_t b = sizeof(uint32_t) * kMaxPasses * 256        // digit histograms
                + sizeof(uint32_t) * kMaxPasses * 32       // tile counters (padded)
                + sizeof(uint32_t) * kMaxPasses * 256 * tiles;  // lookback status
     b = (b + 255) & ~size_t(255);
@@ -33,7 +33,7 @@ constexpr size_t sort_ws_bytes(uint32_t n) {
 // Device scratch of one sort: digit histograms, per-pass tile counters and
 // lookback status words (reset before every sort), and ping-pong buffers.
 struct SortWorkspace {
-    uint32_t* hist = nullptr;         // [kMaxPasses][256]; becomes digit bases
+    uint32_t* hist = nullptr;         // [kMaxPasses][256] digit counts of each pass
     uint32_t* counters = nullptr;     // [kMaxPasses][32]
     uint32_t* tile_status = nullptr;  // [kMaxPasses][tiles_max][256]
     uint32_t* ktmp = nullptr;         // [capacity]

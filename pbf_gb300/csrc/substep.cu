@@ -26,13 +26,28 @@
 
 namespace pbf {
 
-// predictpos.glsl:18-38 fused with the cell key of GetHash (counting.glsl:53-57).
+// Clears the cell-start entry that sorted particle i's cell got from the
+// previous sort, so the dense table never needs a full memset.
+__device__ __forceinline__ void unmark_cell(uint32_t i, const uint32_t* __restrict__ prev_sorted,
+                                            uint32_t ncells, int32_t* __restrict__ cstart) {
+    const uint32_t k = prev_sorted[i];
+    if (k < ncells && (i == 0 || prev_sorted[i - 1] != k)) cstart[k] = -1;
+}
+
+// predictpos.glsl:18-38 fused with the cell key of GetHash (counting.glsl:53-57),
+// and what the substep needs cleared: the previous sort's cells (its keys are
+// still in prev_sorted) and the count of heavy particles (k_stencil_rows).  In
+// launches of their own these took 2 to 3 us each of a small scene's substep.
 template <class CP>
 __global__ void __launch_bounds__(kBlock)
 k_predict(const float4* __restrict__ x, const float4* __restrict__ v, float4* __restrict__ xstar,
-          uint32_t* __restrict__ keys, uint32_t n, CP cp, uint32_t* status) {
+          uint32_t* __restrict__ keys, uint32_t n, CP cp, uint32_t* status,
+          const uint32_t* __restrict__ prev_sorted, uint32_t ncells, int32_t* __restrict__ cstart,
+          uint32_t* __restrict__ heavy_count) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *heavy_count = 0u;
     if (i >= n) return;
+    unmark_cell(i, prev_sorted, ncells, cstart);
     const auto& c = cp.at(i);
     const float4 q = x[i];
     const float4 w = v[i];
@@ -59,15 +74,12 @@ k_keys_of(const float4* __restrict__ x, float4* __restrict__ xstar, uint32_t* __
     keys[i] = cell_key(xyz(q), c);
 }
 
-// Clears the cell-start entries the previous sort set (its sorted keys are
-// still in `prev_sorted`), so the dense table never needs a full memset.
+// The same on its own, for the diagnostics.
 __global__ void __launch_bounds__(kBlock)
 k_unmark_cells(const uint32_t* __restrict__ prev_sorted, uint32_t n, uint32_t ncells,
                int32_t* __restrict__ cstart) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t k = prev_sorted[i];
-    if (k < ncells && (i == 0 || prev_sorted[i - 1] != k)) cstart[k] = -1;
+    if (i < n) unmark_cell(i, prev_sorted, ncells, cstart);
 }
 
 // The scene of every particle (id order): the last whose first particle is not
@@ -1717,8 +1729,11 @@ template void launch_highlight<ManyScenes>(unsigned, cudaStream_t, const float4*
 // (their host stubs are not visible to other translation units).
 template <class CP>
 void launch_predict(unsigned g, cudaStream_t st, const float4* x, const float4* v, float4* xstar,
-                    uint32_t* keys, uint32_t n, CP cp, uint32_t* status) {
-    k_predict<CP><<<g, kBlock, 0, st>>>(x, v, xstar, keys, n, cp, status);
+                    uint32_t* keys, uint32_t n, CP cp, uint32_t* status,
+                    const uint32_t* prev_sorted, uint32_t ncells, int32_t* cstart,
+                    uint32_t* heavy_count) {
+    k_predict<CP><<<g, kBlock, 0, st>>>(x, v, xstar, keys, n, cp, status, prev_sorted, ncells,
+                                        cstart, heavy_count);
 }
 template <class CP>
 void launch_keys_of(unsigned g, cudaStream_t st, const float4* x, float4* xstar, uint32_t* keys,
@@ -1861,7 +1876,8 @@ void launch_diagnostics(unsigned g, cudaStream_t st, const float4* P, const floa
 
 #define PBF_INSTANTIATE(CP)                                                                     \
     template void launch_predict<CP>(unsigned, cudaStream_t, const float4*, const float4*,      \
-                                     float4*, uint32_t*, uint32_t, CP, uint32_t*);              \
+                                     float4*, uint32_t*, uint32_t, CP, uint32_t*,               \
+                                     const uint32_t*, uint32_t, int32_t*, uint32_t*);           \
     template void launch_keys_of<CP>(unsigned, cudaStream_t, const float4*, float4*, uint32_t*, \
                                      uint32_t, CP);                                             \
     template void launch_lambda_build<CP>(SweepCfg, cudaStream_t, const float4*, const uint32_t*, \

@@ -39,7 +39,9 @@ struct SweepCfg {
 
 template <class CP>
 void launch_predict(unsigned g, cudaStream_t st, const float4* x, const float4* v, float4* xstar,
-                    uint32_t* keys, uint32_t n, CP cp, uint32_t* status);
+                    uint32_t* keys, uint32_t n, CP cp, uint32_t* status,
+                    const uint32_t* prev_sorted, uint32_t ncells, int32_t* cstart,
+                    uint32_t* heavy_count);
 template <class CP>
 void launch_keys_of(unsigned g, cudaStream_t st, const float4* x, float4* xstar, uint32_t* keys,
                     uint32_t n, CP cp);
