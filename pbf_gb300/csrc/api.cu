@@ -399,10 +399,11 @@ uint32_t kernels_per_substep(const pbf_sim* s) {
         if (!lists && vort) k += (b.first == 0 ? 1u : 0u) + (b.second == 0 ? 1u : 0u);
     }
     if (rows_on(s)) k += 1u;
-    if (mixed_on(s)) {  // a cooperative launch after each one-thread sweep
+    if (mixed_on(s)) {  // a cooperative launch after the one-thread sweeps
         const PassModes a = modes_of(s, s->pass_solver), b = modes_of(s, s->pass_vort);
         auto extra = [&](uint32_t pass, const PassModes& m) {
-            if (pass_quads(s, pass)) return 2u;
+            // (a quad sweep takes the listed particles in its own launch)
+            if (pass_quads(s, pass)) return s->n < kQuadScanBelow ? 0u : 1u;
             return pass_mixed(s, pass) ? (uint32_t)((m.first != 3) + (m.second != 3)) : 0u;
         };
         k += iters * extra(s->pass_solver, a);

@@ -974,17 +974,7 @@ __device__ __forceinline__ float coop_visit(uint32_t i, const DevConsts& c,
 struct CoopWork {
     const uint32_t* list;
     const uint32_t* count;
-    const int2* rows;  // PairLists::rows
 };
-
-#define PBF_COOP_FOR_EACH(i)                                                                  \
-    __shared__ CoopShared shared_[kBlock / 32];                                               \
-    CoopShared& sm = shared_[threadIdx.x >> 5];                                               \
-    const uint32_t warp0_ = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;                     \
-    const uint32_t nwarps_ = (gridDim.x * blockDim.x) >> 5;                                    \
-    const uint32_t total_ = wk.list ? *wk.count : n;                                           \
-    for (uint32_t w_ = warp0_; w_ < total_; w_ += nwarps_)                                     \
-        if (const uint32_t i = wk.list ? wk.list[w_] : w_; check_ok(cp.at(0), i < n))
 
 // What one lane does with a particle's sums.
 // updatepos.glsl:100: the clamp as min(max(q, lo), hi) with explicit selects,
@@ -1024,66 +1014,95 @@ __device__ __forceinline__ void store_velocity(uint32_t i, float3 eta, const Dev
     if (check_ok(c, perm[i] < c.n_total)) v[perm[i]] = make_float4(vf.x, vf.y, vf.z, 0.0f);  // :85
 }
 
-template <class CP>
-__global__ void __launch_bounds__(kBlock)
-k_lambda_coop(const float4* __restrict__ P, float4* __restrict__ L, float4* __restrict__ aux,
-              uint32_t n, CP cp, CoopWork wk) {
-    PBF_COOP_FOR_EACH(i) {
-        const auto& c = cp.at(i);
+// One particle by one warp (every lane calls).
+struct LambdaCoop {
+    const float4* __restrict__ P;
+    float4* __restrict__ L;
+    float4* __restrict__ aux;
+    const int2* __restrict__ rows;
+    uint32_t n;
+    __device__ __forceinline__ void operator()(uint32_t i, const DevConsts& c,
+                                               CoopShared& sm) const {
         const float3 pi = xyz(P[i]);
-        const float s = coop_visit(i, c, wk.rows, n, P, pi, sm, CoopLambda{});
+        const float s = coop_visit(i, c, rows, n, P, pi, sm, CoopLambda{});
         const LambdaAcc a{shf(s, 0), shf(s, 1), make_float3(shf(s, 2), shf(s, 3), shf(s, 4))};
         if ((threadIdx.x & 31u) == 0u) {
             L[i] = make_float4(pi.x, pi.y, pi.z, lambda_finish(c, a));
             if (aux) aux[i] = lambda_aux(a);
         }
     }
-}
-
-template <class CP>
-__global__ void __launch_bounds__(kBlock)
-k_delta_p_coop(const float4* __restrict__ L, float4* __restrict__ Pn, ScanPos sx_out, uint32_t n,
-               CP cp, uint32_t* status, CoopWork wk) {
-    PBF_COOP_FOR_EACH(i) {
-        const auto& c = cp.at(i);
+};
+struct DeltaPCoop {
+    const float4* __restrict__ L;
+    float4* __restrict__ Pn;
+    ScanPos sx_out;
+    const int2* __restrict__ rows;
+    uint32_t n;
+    uint32_t* status;
+    __device__ __forceinline__ void operator()(uint32_t i, const DevConsts& c,
+                                               CoopShared& sm) const {
         const float4 Li = L[i];
         const float3 pi = xyz(Li);
-        const float s = coop_visit(i, c, wk.rows, n, L, pi, sm, CoopDeltaP{Li.w});
+        const float s = coop_visit(i, c, rows, n, L, pi, sm, CoopDeltaP{Li.w});
         const float3 dp = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
         if ((threadIdx.x & 31u) == 0u)
             store_position(i, fma3(c.oorho, dp, pi), c, Pn, sx_out, status);  // :85
     }
-}
-
-template <class CP>
-__global__ void __launch_bounds__(kBlock)
-k_vorticity_a_coop(const float4* __restrict__ P, const float4* __restrict__ VS,
-                   float4* __restrict__ VX, float4* __restrict__ OM, float4* __restrict__ Q,
-                   uint32_t n, CP cp, CoopWork wk) {
-    PBF_COOP_FOR_EACH(i) {
-        const auto& c = cp.at(i);
+};
+struct VortACoop {
+    const float4* __restrict__ P;
+    const float4* __restrict__ VS;
+    float4* __restrict__ VX;
+    float4* __restrict__ OM;
+    float4* __restrict__ Q;
+    const int2* __restrict__ rows;
+    uint32_t n;
+    __device__ __forceinline__ void operator()(uint32_t i, const DevConsts& c,
+                                               CoopShared& sm) const {
         const float3 pi = xyz(P[i]);
         const float3 vi = xyz(VS[i]);
-        const float s = coop_visit(i, c, wk.rows, n, P, pi, sm, CoopVortA{VS, vi});
+        const float s = coop_visit(i, c, rows, n, P, pi, sm, CoopVortA{VS, vi});
         const float3 acc = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
         const float3 w = make_float3(shf(s, 3), shf(s, 4), shf(s, 5));
         if ((threadIdx.x & 31u) == 0u) store_vorticity(i, pi, vi, acc, w, c, VX, OM, Q);
     }
-}
-
-template <class CP>
-__global__ void __launch_bounds__(kBlock)
-k_vorticity_b_coop(const float4* __restrict__ Q, const float4* __restrict__ VX,
-                   const float4* __restrict__ OM, const uint32_t* __restrict__ perm,
-                   float4* __restrict__ v, float4* __restrict__ eta_out, uint32_t n, CP cp,
-                   CoopWork wk) {
-    PBF_COOP_FOR_EACH(i) {
-        const auto& c = cp.at(i);
+};
+struct VortBCoop {
+    const float4* __restrict__ Q;
+    const float4* __restrict__ VX;
+    const float4* __restrict__ OM;
+    const uint32_t* __restrict__ perm;
+    float4* __restrict__ v;
+    float4* __restrict__ eta_out;
+    const int2* __restrict__ rows;
+    uint32_t n;
+    __device__ __forceinline__ void operator()(uint32_t i, const DevConsts& c,
+                                               CoopShared& sm) const {
         const float3 pi = xyz(Q[i]);
-        const float s = coop_visit(i, c, wk.rows, n, Q, pi, sm, CoopVortB{});
+        const float s = coop_visit(i, c, rows, n, Q, pi, sm, CoopVortB{});
         const float3 eta = make_float3(shf(s, 0), shf(s, 1), shf(s, 2));
         if ((threadIdx.x & 31u) == 0u) store_velocity(i, eta, c, VX, OM, perm, v, eta_out);
     }
+};
+
+// The particles of `wk`, taken in turn by `warps` warps of which this is the
+// w-th: `body` on each.
+template <class CP, class Body>
+__device__ __forceinline__ void coop_each(uint32_t w, uint32_t warps, const CoopWork& wk,
+                                          uint32_t n, const CP& cp, CoopShared& sm,
+                                          const Body& body) {
+    const uint32_t total = wk.list ? *wk.count : n;
+    for (; w < total; w += warps) {
+        const uint32_t i = wk.list ? wk.list[w] : w;
+        if (check_ok(cp.at(0), i < n)) body(i, cp.at(i), sm);
+    }
+}
+
+template <class CP, class Body>
+__global__ void __launch_bounds__(kBlock) k_coop(Body body, uint32_t n, CP cp, CoopWork wk) {
+    __shared__ CoopShared shared[kBlock / 32];
+    coop_each((blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5, wk, n,
+              cp, shared[threadIdx.x >> 5], body);
 }
 
 // ---- quad sweeps: four or eight lanes per particle ------------------------------------------
@@ -1123,6 +1142,17 @@ struct QuadScan {
     int2 run[32 / G][10];               // the rows; the tenth ends the sequence
 };
 static_assert(kQuadScanBelow <= 65536, "QuadScan::found holds 16-bit indices");
+template <int G>
+struct QuadFirst {  // a first sweep's shared memory per warp; a second sweep's is QuadTerms
+    QuadTerms<G> terms;
+    QuadScan<G> scan;
+};
+// A warp is a quad warp or a cooperative one for the whole launch.
+template <class T>
+union QuadOrCoop {
+    T quad;
+    CoopShared coop;
+};
 
 // One of a few registers by index.
 template <int N>
@@ -1343,11 +1373,21 @@ __device__ __forceinline__ QuadSums<G> quad_replay(uint32_t i, bool live, const 
     return sums;
 }
 
-// Particle, liveness and constants of a quad; the lanes past the end and those
-// of listed (heavy) particles run along with nothing to do.
-#define PBF_QUAD_PARTICLE(pl)                                                                 \
-    __shared__ QuadTerms<G> terms_[kQuadBlock / 32];                                          \
-    QuadTerms<G>& sm = terms_[threadIdx.x >> 5];                                              \
+// One sweep of a scene: the first `quads` blocks take the particles that are not
+// listed, a group of G lanes each, the blocks after them the listed ones, a warp
+// each (a launch of their own cost 2.5 us a sweep, mostly over an empty list).
+// Particle, liveness and constants of a quad follow; the lanes past the end and
+// those of listed particles run along with nothing to do.
+#define PBF_QUAD_PARTICLE(SHARED, pl, ...)                                                    \
+    __shared__ QuadOrCoop<SHARED> shared_[kQuadBlock / 32];                                   \
+    if (blockIdx.x >= quads) {                                                                \
+        coop_each(((blockIdx.x - quads) * blockDim.x + threadIdx.x) >> 5,                     \
+                  ((gridDim.x - quads) * blockDim.x) >> 5,                                    \
+                  CoopWork{pl.heavy_list, pl.heavy_count}, n, cp,                             \
+                  shared_[threadIdx.x >> 5].coop, __VA_ARGS__);                               \
+        return;                                                                               \
+    }                                                                                         \
+    SHARED& sm = shared_[threadIdx.x >> 5].quad;                                              \
     const uint32_t own_ = (blockIdx.x * blockDim.x + threadIdx.x) / G;                        \
     const bool live = own_ < n && !(pl.heavy && pl.heavy[own_]);                              \
     const uint32_t i = live ? own_ : 0u;                                                      \
@@ -1355,13 +1395,13 @@ __device__ __forceinline__ QuadSums<G> quad_replay(uint32_t i, bool live, const 
     const bool writes = live && (threadIdx.x & (G - 1)) == 0u
 
 template <class CP, int G>
-__global__ void __launch_bounds__(kQuadBlock)
-k_lambda_quad(const float4* __restrict__ P, float4* __restrict__ L, float4* __restrict__ aux,
-              PairLists pw, uint32_t n, CP cp) {
-    PBF_QUAD_PARTICLE(pw);
-    __shared__ QuadScan<G> scan_[kQuadBlock / 32];
+__global__ void __launch_bounds__(kQuadBlock, 16)
+k_lambda_quad(uint32_t quads, const float4* __restrict__ P, float4* __restrict__ L,
+              float4* __restrict__ aux, PairLists pw, uint32_t n, CP cp) {
+    PBF_QUAD_PARTICLE(QuadFirst<G>, pw, LambdaCoop{P, L, aux, pw.rows, n});
     const float3 pi = xyz(P[i]);
-    const QuadSums<G> s = quad_scan<G>(i, live, c, pw, P, pi, sm, scan_[threadIdx.x >> 5], CoopLambda{});
+    const QuadSums<G> s =
+        quad_scan<G>(i, live, c, pw, P, pi, sm.terms, sm.scan, CoopLambda{});
     const LambdaAcc a{s.get(0), s.get(1), make_float3(s.get(2), s.get(3), s.get(4))};
     if (writes) {
         L[i] = make_float4(pi.x, pi.y, pi.z, lambda_finish(c, a));
@@ -1371,9 +1411,9 @@ k_lambda_quad(const float4* __restrict__ P, float4* __restrict__ L, float4* __re
 
 template <class CP, int G>
 __global__ void __launch_bounds__(kQuadBlock)
-k_delta_p_quad(const float4* __restrict__ L, float4* __restrict__ Pn, PairLists pr, ScanPos sx_out,
-               uint32_t n, CP cp, uint32_t* status) {
-    PBF_QUAD_PARTICLE(pr);
+k_delta_p_quad(uint32_t quads, const float4* __restrict__ L, float4* __restrict__ Pn, PairLists pr,
+               ScanPos sx_out, uint32_t n, CP cp, uint32_t* status) {
+    PBF_QUAD_PARTICLE(QuadTerms<G>, pr, DeltaPCoop{L, Pn, sx_out, pr.rows, n, status});
     const float4 Li = L[i];
     const float3 pi = xyz(Li);
     const QuadSums<G> s = quad_replay<G>(i, live, c, pr, L, pi, sm, CoopDeltaP{Li.w});
@@ -1382,15 +1422,15 @@ k_delta_p_quad(const float4* __restrict__ L, float4* __restrict__ Pn, PairLists 
 }
 
 template <class CP, int G>
-__global__ void __launch_bounds__(kQuadBlock)
-k_vorticity_a_quad(const float4* __restrict__ P, const float4* __restrict__ VS,
+__global__ void __launch_bounds__(kQuadBlock, 16)
+k_vorticity_a_quad(uint32_t quads, const float4* __restrict__ P, const float4* __restrict__ VS,
                    float4* __restrict__ VX, float4* __restrict__ OM, float4* __restrict__ Q,
                    PairLists pw, uint32_t n, CP cp) {
-    PBF_QUAD_PARTICLE(pw);
-    __shared__ QuadScan<G> scan_[kQuadBlock / 32];
+    PBF_QUAD_PARTICLE(QuadFirst<G>, pw, VortACoop{P, VS, VX, OM, Q, pw.rows, n});
     const float3 pi = xyz(P[i]);
     const float3 vi = xyz(VS[i]);
-    const QuadSums<G> s = quad_scan<G>(i, live, c, pw, P, pi, sm, scan_[threadIdx.x >> 5], CoopVortA{VS, vi});
+    const QuadSums<G> s =
+        quad_scan<G>(i, live, c, pw, P, pi, sm.terms, sm.scan, CoopVortA{VS, vi});
     const float3 acc = make_float3(s.get(0), s.get(1), s.get(2));
     const float3 w = make_float3(s.get(3), s.get(4), s.get(5));
     if (writes) store_vorticity(i, pi, vi, acc, w, c, VX, OM, Q);
@@ -1398,11 +1438,11 @@ k_vorticity_a_quad(const float4* __restrict__ P, const float4* __restrict__ VS,
 
 template <class CP, int G>
 __global__ void __launch_bounds__(kQuadBlock)
-k_vorticity_b_quad(const float4* __restrict__ Q, const float4* __restrict__ VX,
+k_vorticity_b_quad(uint32_t quads, const float4* __restrict__ Q, const float4* __restrict__ VX,
                    const float4* __restrict__ OM, const uint32_t* __restrict__ perm,
                    float4* __restrict__ v, float4* __restrict__ eta_out, PairLists pr, uint32_t n,
                    CP cp) {
-    PBF_QUAD_PARTICLE(pr);
+    PBF_QUAD_PARTICLE(QuadTerms<G>, pr, VortBCoop{Q, VX, OM, perm, v, eta_out, pr.rows, n});
     const float3 pi = xyz(Q[i]);
     const QuadSums<G> s = quad_replay<G>(i, live, c, pr, Q, pi, sm, CoopVortB{});
     const float3 eta = make_float3(s.get(0), s.get(1), s.get(2));
@@ -1481,13 +1521,17 @@ inline unsigned heavy_grid(uint32_t n) { return 152u * (n < 1048576u ? 8u : 20u)
 // lanes, us: 16,384 particles lambda 13.7 / 13.6, delta-p 6.2 / 5.1; 32,768
 // lambda 18.5 / 27.6, delta-p 6.9 / 8.8.
 constexpr uint32_t kOctsBelow = 24576;
-inline unsigned quad_grid(uint32_t n, uint32_t lanes) { return grid_for(lanes * n, kQuadBlock); }
-#define PBF_QUAD_LAUNCH(KERNEL, ...)                                                     \
-    do {                                                                                 \
-        if (n < kOctsBelow)                                                              \
-            KERNEL<CP, 8><<<quad_grid(n, 8), kQuadBlock, 0, st>>>(__VA_ARGS__);          \
-        else                                                                             \
-            KERNEL<CP, 4><<<quad_grid(n, 4), kQuadBlock, 0, st>>>(__VA_ARGS__);          \
+inline unsigned quad_blocks(uint32_t n, uint32_t lanes) { return grid_for(lanes * n, kQuadBlock); }
+// Blocks (of two warps) for the listed particles.
+inline unsigned quad_heavy_blocks(uint32_t n) { return n / 2u < 4864u ? n / 2u + 1u : 4864u; }
+#define PBF_QUAD_LAUNCH(KERNEL, ...)                                                      \
+    do {                                                                                  \
+        const unsigned lanes_ = n < kOctsBelow ? 8u : 4u, q_ = quad_blocks(n, lanes_);    \
+        const unsigned g_ = q_ + quad_heavy_blocks(n);                                    \
+        if (lanes_ == 8u)                                                                 \
+            KERNEL<CP, 8><<<g_, kQuadBlock, 0, st>>>(q_, __VA_ARGS__);                    \
+        else                                                                              \
+            KERNEL<CP, 4><<<g_, kQuadBlock, 0, st>>>(q_, __VA_ARGS__);                    \
     } while (0)
 inline unsigned coop_grid(uint32_t n) { return (unsigned)(((size_t)n * 32 + kBlock - 1) / kBlock); }
 
@@ -1759,17 +1803,17 @@ void launch_lambda_build(SweepCfg sw, cudaStream_t st, const float4* XP, const u
                          const int32_t* cstart, const int32_t* cend, float4* L, float4* aux,
                          NbrLists nl, PairLists pw, ScanPos sx, uint32_t n, CP cp) {
     if (sw.mode == kCoop) {
-        k_lambda_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(XP, L, aux, n, cp,
-                                                           CoopWork{nullptr, nullptr, pw.rows});
+        k_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(LambdaCoop{XP, L, aux, pw.rows, n}, n, cp,
+                                               CoopWork{nullptr, nullptr});
         return;
     }
     if (sw.mode == kQuad)
         PBF_QUAD_LAUNCH(k_lambda_quad, XP, L, aux, pw, n, cp);
     else
         PBF_SWEEP_LAUNCH(k_lambda_build, XP, skeys, cstart, cend, L, aux, nl, pw, sx, n, cp);
-    if (pw.heavy)
-        k_lambda_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(XP, L, aux, n, cp,
-                                                         CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
+    if (pw.heavy && sw.mode != kQuad)
+        k_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(LambdaCoop{XP, L, aux, pw.rows, n}, n, cp,
+                                               CoopWork{pw.heavy_list, pw.heavy_count});
 }
 template <class CP>
 void launch_lambda(SweepCfg sw, cudaStream_t st, const float4* P, const float4* XP,
@@ -1777,17 +1821,17 @@ void launch_lambda(SweepCfg sw, cudaStream_t st, const float4* P, const float4* 
                    float4* aux, NbrLists nl, PairLists pw, ScanPos sx, int dmax_slot, uint32_t n,
                    CP cp) {
     if (sw.mode == kCoop) {
-        k_lambda_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(P, L, aux, n, cp,
-                                                           CoopWork{nullptr, nullptr, pw.rows});
+        k_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(LambdaCoop{P, L, aux, pw.rows, n}, n, cp,
+                                               CoopWork{nullptr, nullptr});
         return;
     }
     if (sw.mode == kQuad)
         PBF_QUAD_LAUNCH(k_lambda_quad, P, L, aux, pw, n, cp);
     else
         PBF_SWEEP_LAUNCH(k_lambda, P, XP, skeys, cstart, cend, L, aux, nl, pw, sx, dmax_slot, n, cp);
-    if (pw.heavy)
-        k_lambda_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(P, L, aux, n, cp,
-                                                         CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
+    if (pw.heavy && sw.mode != kQuad)
+        k_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(LambdaCoop{P, L, aux, pw.rows, n}, n, cp,
+                                               CoopWork{pw.heavy_list, pw.heavy_count});
 }
 template <class CP>
 void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4* XP,
@@ -1797,8 +1841,8 @@ void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4*
     if (sw.mode == kCoop) {
         // (with its scan copy where the vorticity passes scan it: they may run
         // under another configuration than the solver)
-        k_delta_p_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(L, Pn, sx_out, n, cp, status,
-                                                            CoopWork{nullptr, nullptr, pr.rows});
+        k_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(DeltaPCoop{L, Pn, sx_out, pr.rows, n, status}, n, cp,
+                                               CoopWork{nullptr, nullptr});
         return;
     }
     if (sw.mode == kQuad)
@@ -1806,10 +1850,9 @@ void launch_delta_p(SweepCfg sw, cudaStream_t st, const float4* L, const float4*
     else
         PBF_SWEEP_LAUNCH(k_delta_p, L, XP, skeys, cstart, cend, Pn, nl, pr, sx, sx_out, dmax_slot,
                      out_slot, n, cp, status);
-    if (pr.heavy)
-        k_delta_p_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(L, Pn, sx_out, n, cp,
-                                                          status,
-                                                          CoopWork{pr.heavy_list, pr.heavy_count, pr.rows});
+    if (pr.heavy && sw.mode != kQuad)
+        k_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(DeltaPCoop{L, Pn, sx_out, pr.rows, n, status}, n, cp,
+                                               CoopWork{pr.heavy_list, pr.heavy_count});
 }
 template <class CP>
 void launch_stencil_rows(cudaStream_t st, const float4* XP, const int32_t* cstart,
@@ -1833,8 +1876,8 @@ void launch_vorticity_a(SweepCfg sw, cudaStream_t st, const float4* P, const flo
                         const int32_t* cend, float4* VX, float4* OM, float4* Q, NbrLists nl,
                         PairLists pw, ScanPos sx, int dmax_slot, uint32_t n, CP cp) {
     if (sw.mode == kCoop) {
-        k_vorticity_a_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(P, VS, VX, OM, Q,
-                                                               n, cp, CoopWork{nullptr, nullptr, pw.rows});
+        k_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(VortACoop{P, VS, VX, OM, Q, pw.rows, n}, n, cp,
+                                               CoopWork{nullptr, nullptr});
         return;
     }
     if (sw.mode == kQuad)
@@ -1842,9 +1885,9 @@ void launch_vorticity_a(SweepCfg sw, cudaStream_t st, const float4* P, const flo
     else
         PBF_SWEEP_LAUNCH(k_vorticity_a, P, XP, VS, skeys, cstart, cend, VX, OM, Q, nl, pw, sx, dmax_slot,
                      n, cp);
-    if (pw.heavy)
-        k_vorticity_a_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(
-            P, VS, VX, OM, Q, n, cp, CoopWork{pw.heavy_list, pw.heavy_count, pw.rows});
+    if (pw.heavy && sw.mode != kQuad)
+        k_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(VortACoop{P, VS, VX, OM, Q, pw.rows, n}, n, cp,
+                                               CoopWork{pw.heavy_list, pw.heavy_count});
 }
 template <class CP>
 void launch_vorticity_b(SweepCfg sw, cudaStream_t st, const float4* Q, const float4* XP,
@@ -1853,8 +1896,8 @@ void launch_vorticity_b(SweepCfg sw, cudaStream_t st, const float4* Q, const flo
                         float4* v, float4* eta_out, NbrLists nl, PairLists pr, ScanPos sx,
                         int dmax_slot, uint32_t n, CP cp) {
     if (sw.mode == kCoop) {
-        k_vorticity_b_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(Q, VX, OM, perm, v,
-                                                               eta_out, n, cp, CoopWork{nullptr, nullptr, pr.rows});
+        k_coop<CP><<<coop_grid(n), kBlock, 0, st>>>(VortBCoop{Q, VX, OM, perm, v, eta_out, pr.rows, n}, n, cp,
+                                               CoopWork{nullptr, nullptr});
         return;
     }
     if (sw.mode == kQuad)
@@ -1862,10 +1905,9 @@ void launch_vorticity_b(SweepCfg sw, cudaStream_t st, const float4* Q, const flo
     else
         PBF_SWEEP_LAUNCH(k_vorticity_b, Q, XP, VX, OM, skeys, perm, cstart, cend, v, eta_out, nl, pr, sx,
                      dmax_slot, n, cp);
-    if (pr.heavy)
-        k_vorticity_b_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(
-            Q, VX, OM, perm, v, eta_out, n, cp,
-            CoopWork{pr.heavy_list, pr.heavy_count, pr.rows});
+    if (pr.heavy && sw.mode != kQuad)
+        k_coop<CP><<<heavy_grid(n), kBlock, 0, st>>>(VortBCoop{Q, VX, OM, perm, v, eta_out, pr.rows, n}, n, cp,
+                                               CoopWork{pr.heavy_list, pr.heavy_count});
 }
 template <class CP>
 void launch_diagnostics(unsigned g, cudaStream_t st, const float4* P, const float4* v,
@@ -1936,10 +1978,10 @@ cudaError_t preload_sweeps() {
     load((const void*)k_vorticity_b<CP, kDirect, false>);
     load((const void*)k_vorticity_b<CP, kMasked, false>);
     load((const void*)k_vorticity_b<CP, kPairs, false>);
-    load((const void*)k_lambda_coop<CP>);
-    load((const void*)k_delta_p_coop<CP>);
-    load((const void*)k_vorticity_a_coop<CP>);
-    load((const void*)k_vorticity_b_coop<CP>);
+    load((const void*)k_coop<CP, LambdaCoop>);
+    load((const void*)k_coop<CP, DeltaPCoop>);
+    load((const void*)k_coop<CP, VortACoop>);
+    load((const void*)k_coop<CP, VortBCoop>);
     load((const void*)k_lambda_quad<CP, 4>);
     load((const void*)k_lambda_quad<CP, 8>);
     load((const void*)k_delta_p_quad<CP, 4>);
