@@ -207,12 +207,14 @@ typedef struct pbf_tuning {
                                      chunks of 32 candidates, marks the ones within h in
                                      a bit mask, then evaluates the marked ones, in the
                                      same order (a warp's lanes stay converged);
-                                     PBF_SWEEP_COOP: a warp per particle, its lanes
-                                     testing 32 candidates at once and computing their
-                                     pair terms in parallel, folded in the same order
-                                     (for scenes too small to fill the GPU with a
-                                     thread per particle, and clumped states; the
-                                     default below 32,768 particles per handle) */
+                                     PBF_SWEEP_COOP: several lanes per particle (a warp,
+                                     or four to eight lanes for particles of at most
+                                     256 candidates in scenes below 49,152 particles)
+                                     test candidates and compute pair terms in parallel,
+                                     folded in the same order (for scenes too small to
+                                     fill the GPU with a thread per particle, and
+                                     clumped states; the default below 32,768 particles
+                                     per handle) */
     uint32_t pair_list_capacity;  /* with PBF_SWEEP_MASKED and > 0: each lambda sweep
                                      records every particle's candidates within h (in
                                      visit order, up to this many), evaluates its own
