@@ -436,6 +436,7 @@ k_adj_flags(const uint32_t* __restrict__ perm, const float4* __restrict__ XPc,
 // Blocks per SM each body is compiled for (Body::kBlocksPerSM): 4 (64 registers)
 // fit every body without spills; the delta-p body alone would take 71 and run
 // 3.  Measured, 1.2 million particles: delta-p 318 -> 250 us per launch.
+//
 // One neighbour reversal (Body::run<W>): blocks below `tblocks` take a
 // thread per unflagged particle, the blocks after them a warp per flagged
 // particle (in turn, from the list).
