@@ -1061,6 +1061,11 @@ pbf_status pbf_forward_record(pbf_sim* s, uint32_t substeps, uint32_t checkpoint
             PBF_CUDA(s, record_segment(s, t, seg, cnt));
             s->launched += (uint64_t)cnt * pbf_kernels_per_substep(s);
             s->autop.count += cnt;
+            // (a recorded substep keeps its lambdas in its slot: pbf_get_solver
+            // reads the handle's, beside the last substep's predicted positions)
+            if (iters > 0)
+                PBF_CUDA(s, cudaMemcpyAsync(s->L, t->slots[cnt - 1].L[iters - 1], b,
+                                            cudaMemcpyDeviceToDevice, s->stream));
         }
     }
     PBF_CUDA(s, cudaMemcpyAsync(t->final_x, s->x, b, cudaMemcpyDeviceToDevice, s->stream));

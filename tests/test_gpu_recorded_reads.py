@@ -1,0 +1,38 @@
+"""GPU tests of what the handle shows after a recorded run: the debug reads of
+the last substep, the automatic mode's trials and the launch count are those of
+the same substeps run by pbf_step."""
+import numpy as np
+import pytest
+
+import pbf_gb300 as pg
+from pbf_gb300 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def make(iterations=3, vorticity=True, **tuning):
+    x4, v4 = scenes.block((11, 9, 10), origin=(4.0, 4.0, 4.0), seed=6, vel_uniform=0.5)
+    p = scenes.dam_params((32, 32, 32), iterations, epsilon=5.0, vorticity=vorticity)
+    sim = pg.SPH(x4.shape[0], tuple(p.grid), p)
+    if tuning:
+        sim.set_tuning(**tuning)
+    sim.set_state(x4, v4)
+    return sim
+
+
+def reads(sim):
+    return [*sim.get_solver(), *sim.get_sort(), *sim.get_cells(), *sim.get_state()]
+
+
+@pytest.mark.parametrize("substeps,every", [(1, 1), (4, 4), (3, 8), (5, 2), (6, 2)])
+@pytest.mark.parametrize("iterations,vorticity", [(3, True), (1, False), (0, True)])
+def test_reads_of_the_last_substep(gpu, substeps, every, iterations, vorticity):
+    stepped, recorded = make(iterations, vorticity), make(iterations, vorticity)
+    stepped.step(substeps)
+    recorded.forward_record(substeps, every)
+    want, got = reads(stepped), reads(recorded)
+    if iterations == 0:  # no sweep writes a lambda
+        want, got = want[1:], got[1:]
+    for a, b in zip(got, want):
+        assert np.array_equal(np.ascontiguousarray(a).view(np.uint32),
+                              np.ascontiguousarray(b).view(np.uint32))
