@@ -945,8 +945,9 @@ cudaError_t reverse_dispatch(pbf_sim* s, Tape* t, const Tape::Slot& sl) {
 }
 
 // Runs segment `seg` (`count` substeps) from the current state, recording each
-// substep into a slot.
-cudaError_t record_segment(pbf_sim* s, Tape* t, uint32_t seg, uint32_t count) {
+// substep into a slot; with `step` they are the handle's next substeps
+// (recorded_substep), otherwise a repetition of earlier ones.
+pbf_status record_segment(pbf_sim* s, Tape* t, uint32_t seg, uint32_t count, bool step) {
     cudaStream_t st = s->stream;
     const size_t n = s->n;
     t->held = Tape::kNone;
@@ -960,30 +961,30 @@ cudaError_t record_segment(pbf_sim* s, Tape* t, uint32_t seg, uint32_t count) {
         rec.OM = sl.OM;
         rec.Q = sl.Q;
         rec.ETA = sl.ETA;
-        cudaError_t e = cudaSuccess;
         if (t->list_cap) {
             rec.lists = sl.lists.data();
             // particles that a cooperative sweep takes write no list
             for (const PairLists& pl : sl.lists)
-                if (pl.cap && e == cudaSuccess)
-                    e = cudaMemsetAsync(pl.cnt, 0xFF, sizeof(int32_t) * n, st);
-            if (e != cudaSuccess) return e;
+                if (pl.cap) PBF_CUDA(s, cudaMemsetAsync(pl.cnt, 0xFF, sizeof(int32_t) * n, st));
         }
-        e = enqueue_substep(s, nullptr, &rec);
-        if (e != cudaSuccess) return e;
-        e = cudaMemcpyAsync(sl.perm, s->perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st);
-        if (e != cudaSuccess) return e;
+        if (step) {
+            pbf_status r = recorded_substep(s, rec);
+            if (r != PBF_OK) return r;
+        } else {
+            PBF_CUDA(s, enqueue_substep(s, nullptr, &rec));
+        }
+        PBF_CUDA(s, cudaMemcpyAsync(sl.perm, s->perm, sizeof(uint32_t) * n,
+                                    cudaMemcpyDeviceToDevice, st));
         const float4* XPc = t->iters > 0 ? sl.L[0] : sl.PF;
         if (s->nscenes == 1)
             launch_adj_rows(st, sl.perm, XPc, s->cstart, s->cend, sl.rows, s->n, OneScene{s->dc});
         else
             launch_adj_rows(st, sl.perm, XPc, s->cstart, s->cend, sl.rows, s->n,
                             ManyScenes{s->d_consts, s->sid});
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        PBF_CUDA(s, cudaGetLastError());
     }
     t->held = seg;
-    return cudaSuccess;
+    return PBF_OK;
 }
 
 }  // namespace
@@ -1058,9 +1059,8 @@ pbf_status pbf_forward_record(pbf_sim* s, uint32_t substeps, uint32_t checkpoint
             pbf_status r = pbf_step(s, cnt);
             if (r != PBF_OK) return r;
         } else {
-            PBF_CUDA(s, record_segment(s, t, seg, cnt));
-            s->launched += (uint64_t)cnt * pbf_kernels_per_substep(s);
-            s->autop.count += cnt;
+            pbf_status r = record_segment(s, t, seg, cnt, true);
+            if (r != PBF_OK) return r;
             // (a recorded substep keeps its lambdas in its slot: pbf_get_solver
             // reads the handle's, beside the last substep's predicted positions)
             if (iters > 0)
@@ -1111,7 +1111,8 @@ pbf_status pbf_backward(pbf_sim* s, const float* dL_dx4, const float* dL_dv4, in
         if (t->held != (uint32_t)seg) {
             PBF_CUDA(s, cudaMemcpyAsync(s->x, t->ckpt_x[seg], b, cudaMemcpyDeviceToDevice, st));
             PBF_CUDA(s, cudaMemcpyAsync(s->v, t->ckpt_v[seg], b, cudaMemcpyDeviceToDevice, st));
-            PBF_CUDA(s, record_segment(s, t, (uint32_t)seg, cnt));
+            pbf_status r = record_segment(s, t, (uint32_t)seg, cnt, false);
+            if (r != PBF_OK) return r;
         }
         for (int k = (int)cnt - 1; k >= 0; --k) PBF_CUDA(s, reverse_dispatch(s, t, t->slots[k]));
     }

@@ -438,11 +438,23 @@ pbf_status launch_graph(pbf_sim* s, uint32_t count) {
     return PBF_OK;
 }
 
+// Whether the next substep belongs to a PBF_SWEEP_AUTO trial; starts one that
+// is due.
+bool trial_next(pbf_sim* s) {
+    if (s->tuning.sweep_mode != PBF_SWEEP_AUTO) return false;
+    if (s->auto_trial < 0 && s->autop.trial_due()) {
+        pick_trial_candidates(s);
+        s->auto_trial = 0;
+    }
+    return s->auto_trial >= 0;
+}
+
 // One substep of a PBF_SWEEP_AUTO trial: the next candidate configuration for
 // both passes, eager, with stage events.  After the last candidate, waits for
 // the trial's events and hands each candidate's solver and vorticity times
 // to the policy (auto_policy.h), which keeps the choices and the schedule.
-pbf_status trial_substep(pbf_sim* s) {
+// `rec`: as in enqueue_substep.
+pbf_status trial_substep(pbf_sim* s, const Recording* rec = nullptr) {
     NvtxRange nvtx_("sweep trial substep");
     const uint32_t iters = s->params.num_solver_iterations;
     const size_t per = 7 + 2 * (size_t)iters;
@@ -455,7 +467,7 @@ pbf_status trial_substep(pbf_sim* s) {
     const uint32_t keep_s = s->pass_solver, keep_v = s->pass_vort;
     const int k = s->auto_trial;
     s->pass_solver = s->pass_vort = s->auto_cands[k];
-    cudaError_t e = enqueue_substep(s, s->trial_ev.data() + per * k);
+    cudaError_t e = enqueue_substep(s, s->trial_ev.data() + per * k, rec);
     s->launched += kernels_per_substep(s);
     s->pass_solver = keep_s;
     s->pass_vort = keep_v;
@@ -674,6 +686,18 @@ cudaError_t enqueue_substep(pbf_sim* s, cudaEvent_t* ev, const Recording* rec) {
     if (s->nscenes == 1) return enqueue_impl(s, ev, rec, OneScene{s->dc}, OneScene{s->dc});
     return enqueue_impl(s, ev, rec, ManyScenes{s->d_consts, s->sid},
                         ManyScenes{s->d_consts, s->sid_sorted});
+}
+
+pbf_status recorded_substep(pbf_sim* s, const Recording& rec) {
+    if (trial_next(s)) {
+        pbf_status r = trial_substep(s, &rec);
+        if (r != PBF_OK) return r;
+    } else {
+        PBF_CUDA(s, enqueue_substep(s, nullptr, &rec));
+        s->launched += kernels_per_substep(s);
+    }
+    ++s->autop.count;
+    return PBF_OK;
 }
 
 void invalidate_graph(pbf_sim* s) {
@@ -1094,11 +1118,7 @@ pbf_status pbf_step(pbf_sim* s, uint32_t substeps) {
     const bool autom = s->tuning.sweep_mode == PBF_SWEEP_AUTO;
     uint32_t left = substeps;
     while (left > 0) {
-        if (autom && s->auto_trial < 0 && s->autop.trial_due()) {
-            pick_trial_candidates(s);
-            s->auto_trial = 0;
-        }
-        if (autom && s->auto_trial >= 0) {
+        if (trial_next(s)) {
             pbf_status r = trial_substep(s);
             if (r != PBF_OK) return r;
             --left;

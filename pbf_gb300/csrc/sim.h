@@ -123,6 +123,9 @@ pbf_status check_status(pbf_sim* s);
 // Enqueues one substep on s->stream; with `rec`, the stage outputs land in
 // the recording's buffers.  `ev`: optional stage events (timing mode).
 cudaError_t enqueue_substep(pbf_sim* s, cudaEvent_t* ev, const Recording* rec = nullptr);
+// One substep of pbf_step (its place in the automatic mode's schedule, its
+// launch count), enqueued eagerly into the recording's buffers.
+pbf_status recorded_substep(pbf_sim* s, const Recording& rec);
 void invalidate_graph(pbf_sim* s);
 void free_tape(pbf_sim* s);
 // Drops the recorded run but keeps its buffers for the next one.

@@ -36,3 +36,24 @@ def test_reads_of_the_last_substep(gpu, substeps, every, iterations, vorticity):
     for a, b in zip(got, want):
         assert np.array_equal(np.ascontiguousarray(a).view(np.uint32),
                               np.ascontiguousarray(b).view(np.uint32))
+
+
+@pytest.mark.parametrize("substeps,every", [(8, 8), (8, 3), (6, 4)])
+def test_trials_go_on_in_the_recorded_segment(gpu, substeps, every):
+    # the first trial starts at substep 3 and takes three substeps; the next
+    # cannot end before substep 9
+    stepped, recorded = make(auto_period=3), make(auto_period=3)
+    stepped.step(substeps)
+    recorded.forward_record(substeps, every)
+    assert stepped.sweep_choice()["trials"] == 1
+    assert recorded.sweep_choice()["trials"] == 1
+    for a, b in zip(recorded.get_state(), stepped.get_state()):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    rng = np.random.default_rng(2)
+    w = rng.standard_normal((990, 4)).astype(np.float32)
+    plain = make(sweep_mode="masked")
+    plain.forward_record(substeps, every)
+    for a, b in zip(recorded.backward(w, w), plain.backward(w, w)):
+        # (recorded lists and scans agree to rounding: test_gpu_adjoint_record.py)
+        a, b = np.asarray(a, np.float64), np.asarray(b, np.float64)
+        assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max()
