@@ -879,15 +879,18 @@ pbf_status pbf_set_scene_params(pbf_sim* s, uint32_t scene, const pbf_params* p)
          (p->vorticity_confinement != 0) != (s->params.vorticity_confinement != 0)))
         return fail(s, PBF_ERR_INVALID_ARGUMENT,
                     "all scenes share the iteration count and the vorticity flag");
-    if (std::memcmp(p, &s->sparams[scene], sizeof *p) == 0) {
+    if (s->settled && std::memcmp(p, &s->sparams[scene], sizeof *p) == 0) {
         // nothing changes but the recorded run, which ends with any call
-        // (a training step sets every scene's parameters, mostly the same)
+        // (a training step sets every scene's parameters, mostly the same);
+        // after a change that failed part-way the whole path runs again
         invalidate_tape(s);
         s->auto_trial = -1;
         return PBF_OK;
     }
     DeviceGuard dg(s->device);
     PBF_CUDA(s, cudaStreamSynchronize(s->stream));
+    const bool was_settled = s->settled;
+    s->settled = false;
     const uint32_t base = s->sdc[scene].cell_base;
     s->sparams[scene] = *p;
     s->sdc[scene] = make_consts(*p);
@@ -895,13 +898,16 @@ pbf_status pbf_set_scene_params(pbf_sim* s, uint32_t scene, const pbf_params* p)
     apply_tuning(s->sdc[scene], *p, s->tuning);
     bind_checks(s);
     if (scene == 0) s->params = *p;
+    const uint32_t first = was_settled ? scene : 0u;  // (every scene's after a failed change)
     if (s->nscenes > 1)
-        PBF_CUDA(s, cudaMemcpy(s->d_consts + scene, &s->sdc[scene], sizeof(DevConsts),
+        PBF_CUDA(s, cudaMemcpy(s->d_consts + first, &s->sdc[first],
+                               sizeof(DevConsts) * (was_settled ? 1u : s->nscenes),
                                cudaMemcpyHostToDevice));
     invalidate_graph(s);
     invalidate_tape(s);  // a recorded run is only valid for the parameters it ran with
     s->auto_trial = -1;  // a running trial's events may not match the new iteration count
     PBF_CUDA(s, ensure_lists(s));
+    s->settled = true;
     return PBF_OK;
 }
 
@@ -940,6 +946,7 @@ pbf_status pbf_set_tuning(pbf_sim* s, const pbf_tuning* t) {
                     "PBF_SWEEP_AUTO");
     DeviceGuard dg(s->device);
     PBF_CUDA(s, cudaStreamSynchronize(s->stream));
+    s->settled = false;
     s->tuning = *t;
     for (uint32_t k = 0; k < s->nscenes; ++k) apply_tuning(s->sdc[k], s->sparams[k], s->tuning);
     s->dc = s->sdc[0];
@@ -948,6 +955,7 @@ pbf_status pbf_set_tuning(pbf_sim* s, const pbf_tuning* t) {
                                cudaMemcpyHostToDevice));
     invalidate_graph(s);
     PBF_CUDA(s, ensure_lists(s));
+    s->settled = true;
     reset_sweep_choice(s);
     return PBF_OK;
 }

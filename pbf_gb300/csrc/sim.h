@@ -96,6 +96,10 @@ struct pbf_sim {
 
     pbf::Tape* tape = nullptr;  // recorded forward run for pbf_backward
 
+    // whether the last change of parameters or tuning was carried out whole
+    // (buffers allocated, constants on the device)
+    bool settled = true;
+
     std::string err;
 };
 
