@@ -38,6 +38,7 @@ pbf_status pbf::fail(pbf_sim* s, pbf_status st, const std::string& msg) {
 }
 
 pbf_status pbf::cuda_fail(pbf_sim* s, cudaError_t e, const char* what) {
+    cudaGetLastError();  // reported here: the next launch check does not see it again
     std::string msg = std::string(what) + ": " + cudaGetErrorString(e);
     return fail(s, e == cudaErrorMemoryAllocation ? PBF_ERR_OUT_OF_MEMORY : PBF_ERR_CUDA, msg);
 }

@@ -345,6 +345,7 @@ static cudaError_t sort_scratch_address(int dev, void** out) {
 }
 
 static pbf_status noalloc_fail(pbf_status st, const std::string& msg) {
+    cudaGetLastError();  // (as in cuda_fail)
     pbf::set_last_error(msg.c_str());
     return st;
 }

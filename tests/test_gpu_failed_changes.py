@@ -3,9 +3,10 @@ part-way (host-side fault injection): the same call, repeated with the same
 values, carries it out, and the handle steps as a new one would."""
 import numpy as np
 import pytest
+import torch
 
 import pbf_gb300 as pg
-from pbf_gb300 import scenes
+from pbf_gb300 import _capi, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -73,3 +74,29 @@ def test_parameters_set_after_a_failed_tuning(gpu, scene_count, after):
         sim.set_scene_params(1, p)
     for a, b in zip(stepped(sim, x4, v4), want):
         assert np.array_equal(a, b)
+
+
+def test_a_real_out_of_memory_is_reported_once(gpu):
+    # entries of 4,096 candidates for this many particles do not fit on any GPU
+    x4, v4, p = scene()
+    sim = pg.SPH(x4.shape[0], tuple(p.grid), p)
+    want = stepped(sim, x4, v4)
+    many = pg.SPH(20_000_000, tuple(p.grid), p)
+    many.set_tuning(pair_list_capacity=0)
+
+    def run_out():
+        with pytest.raises(pg.PbfError) as e:
+            many.set_tuning(pair_list_capacity=4096)
+        assert e.value.status == OUT_OF_MEMORY
+
+    run_out()
+    new = pg.SPH(x4.shape[0], tuple(p.grid), p)
+    for a, b in zip(stepped(new, x4, v4), want):  # captures its graph
+        assert np.array_equal(a, b)
+    run_out()
+    keys = torch.tensor([0, 0, 2, 5], dtype=torch.int32, device="cuda")
+    start, end = (torch.empty(6, dtype=torch.int32, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    _capi.check(gpu.pbf_find_cells(keys.data_ptr(), 4, 6, start.data_ptr(), end.data_ptr(), None))
+    assert start.tolist() == [0, -1, 2, -1, -1, 3] and end.tolist() == [2, -1, 3, -1, -1, 4]
+    many.close()
