@@ -375,10 +375,23 @@ typedef struct pbf_param_grads {
 } pbf_param_grads;
 
 /* Runs `substeps` substeps from the current state like pbf_step and keeps
- * what pbf_backward needs: the state every `checkpoint_every` substeps (the
- * substeps in between are recomputed during the backward pass) and the final
- * state.  Parameters must not change until pbf_backward; pbf_set_params and
- * pbf_set_scene_params drop the recording. */
+ * what pbf_backward needs: the state every `checkpoint_every` substeps, the
+ * last `checkpoint_every` substeps whole (the others are recomputed during the
+ * backward pass) and the final state.  Parameters must not change until
+ * pbf_backward; pbf_set_params and pbf_set_scene_params drop the recording.
+ *
+ * Device memory, in bytes per particle: 32 per checkpoint, 156 + 32 per solver
+ * iteration for each of the `checkpoint_every` substeps, and 300 more; and the
+ * substeps' pair lists, 4 per entry, for each iteration and the vorticity
+ * passes (as many entries as pair_list_capacity while all stays below 4 GiB,
+ * otherwise 48; none where they would take more than an eighth of the free
+ * memory).  At 4 iterations and 48 entries a substep takes 1,260 bytes per
+ * particle, 980 of them lists.  The memory stays with the handle for the next
+ * recorded run, also after the recording was dropped; pbf_release_record and
+ * pbf_destroy free it, and while it holds no recording so does any other
+ * allocation of this library on the device that would fail without it.  A
+ * program that needs it back for allocations of its own calls
+ * pbf_release_record. */
 pbf_status pbf_forward_record(pbf_sim* sim, uint32_t substeps, uint32_t checkpoint_every);
 
 /* Reverse-mode gradient of a loss L(x_final, v_final) through the recorded
@@ -393,7 +406,7 @@ pbf_status pbf_forward_record(pbf_sim* sim, uint32_t substeps, uint32_t checkpoi
 pbf_status pbf_backward(pbf_sim* sim, const float* dL_dx4, const float* dL_dv4, int where,
                         float* dL_dx0_4, float* dL_dv0_4, pbf_param_grads* grads);
 
-/* Frees the recording of pbf_forward_record. */
+/* Frees the recording of pbf_forward_record and its memory. */
 pbf_status pbf_release_record(pbf_sim* sim);
 
 /* SPH's highlight pass (clearhighlight.glsl:7, highlight.glsl:16-30, run from

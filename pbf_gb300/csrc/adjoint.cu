@@ -47,6 +47,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 
 namespace pbf {
 
@@ -57,8 +58,11 @@ constexpr int kParams = 4;  // epsilon, tensile k, XSPH c, vorticity epsilon
 // kept with the handle and reused by the next pbf_forward_record of the same
 // shape (a training step records again and again: allocating and freeing them
 // in pieces cost 4 ms of a 21 ms step with 32,768 particles and 14 ms of 165 ms
-// with 1.2 million); pbf_release_record and the handle's end give them back.
+// with 1.2 million).  pbf_release_record and the handle's end give them back,
+// and so does any allocation of the library that finds no memory, of any
+// handle, while they hold no recorded run (IdleTapes).
 struct Tape {
+    int device = 0;
     uint32_t substeps = 0, every = 0, iters = 0, nslots = 0;
     bool vort = false;
     bool valid = false;    // holds a complete recorded run
@@ -797,6 +801,41 @@ k_adj_param_sums(const double* __restrict__ acc, const uint32_t* __restrict__ fi
 
 // ---- host side ------------------------------------------------------------------
 
+// The tapes that hold no recorded run.  A tape is in this list or claimed by the
+// thread that uses its handle, and `mem` of one in the list changes under the
+// lock only, so handles in other threads may free it.  Nothing runs on a tape
+// in the list (its stream was waited for).
+struct IdleTapes {
+    std::mutex mu;
+    std::vector<Tape*> list;
+};
+IdleTapes& idle_tapes() {
+    static IdleTapes* t = new IdleTapes;  // outlives every handle
+    return *t;
+}
+void park(Tape* t) {
+    IdleTapes& idle = idle_tapes();
+    std::lock_guard<std::mutex> lock(idle.mu);
+    if (std::find(idle.list.begin(), idle.list.end(), t) == idle.list.end())
+        idle.list.push_back(t);
+}
+// Whether the tape still has its buffers.
+bool claim(Tape* t) {
+    IdleTapes& idle = idle_tapes();
+    std::lock_guard<std::mutex> lock(idle.mu);
+    idle.list.erase(std::remove(idle.list.begin(), idle.list.end(), t), idle.list.end());
+    return t->mem != nullptr;
+}
+// A run that ends without a complete record leaves its tape idle.
+struct ParkUnlessValid {
+    pbf_sim* s;
+    ~ParkUnlessValid() {
+        if (!s->tape || s->tape->valid) return;
+        cudaStreamSynchronize(s->stream);
+        park(s->tape);
+    }
+};
+
 // Hands out 256-byte aligned pieces of one allocation (base null: only counts).
 struct Carver {
     uint8_t* base;
@@ -852,11 +891,14 @@ void carve_tape(const pbf_sim* s, Tape* t, Carver& a) {
 }
 
 // Capacity of the recorded pair lists: the handle's while the tape then stays
-// below kAdjListBytes; otherwise kAdjListCap entries per particle (a fluid at
-// its rest density has about 33 neighbours; a longer list is not kept), and
-// none where that would take more than half of the free memory.
+// below kAdjListBytes, otherwise kAdjListCap entries per particle (a fluid at
+// its rest density has about 33 neighbours; a longer list is not kept), and none
+// where the lists would take more than 1 / kAdjListShare of the free memory:
+// they are four fifths of a tape, which the host program's own allocator cannot
+// call back.
 constexpr size_t kAdjListBytes = size_t(4) << 30;
 constexpr uint32_t kAdjListCap = 48;
+constexpr size_t kAdjListShare = 8;
 
 cudaError_t alloc_tape(pbf_sim* s, Tape* t) {
     auto bytes = [&](uint32_t cap) {
@@ -865,19 +907,19 @@ cudaError_t alloc_tape(pbf_sim* s, Tape* t) {
         carve_tape(s, t, a);
         return a.used;
     };
+    size_t free_b = 0, total_b = 0;
+    cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+    if (e != cudaSuccess) return e;
+    const size_t bare = bytes(0), share = free_b / kAdjListShare;
     size_t need = bytes(s->pair_cap);
-    if (need > kAdjListBytes) need = bytes(std::min(s->pair_cap, kAdjListCap));
-    if (t->list_cap && need > kAdjListBytes) {
-        size_t free_b = 0, total_b = 0;
-        const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
-        if (e != cudaSuccess) return e;
-        if (need > free_b / 2) need = bytes(0);
-    }
-    cudaError_t e = cudaMalloc(&t->mem, need);
+    if (need > kAdjListBytes || need - bare > share)
+        need = bytes(std::min(s->pair_cap, kAdjListCap));
+    if (need - bare > share) need = bytes(0);
+    e = device_alloc(&t->mem, need);
     if (e == cudaErrorMemoryAllocation && t->list_cap) {
         cudaGetLastError();
         need = bytes(0);
-        e = cudaMalloc(&t->mem, need);
+        e = device_alloc(&t->mem, need);
     }
     if (e != cudaSuccess) {
         t->mem = nullptr;
@@ -991,20 +1033,31 @@ pbf_status record_segment(pbf_sim* s, Tape* t, uint32_t seg, uint32_t count, boo
 
 void free_tape(pbf_sim* s) {
     if (!s->tape) return;
-    if (s->tape->mem) cudaFree(s->tape->mem);
+    if (claim(s->tape)) cudaFree(s->tape->mem);
     delete s->tape;
     s->tape = nullptr;
 }
 
 void invalidate_tape(pbf_sim* s) {
-    if (s->tape) s->tape->valid = false;
+    if (!s->tape || !s->tape->valid) return;
+    s->tape->valid = false;
+    cudaStreamSynchronize(s->stream);
+    park(s->tape);
 }
 
-bool free_idle_tape(pbf_sim* s) {
-    if (!s->tape || s->tape->valid) return false;
-    cudaStreamSynchronize(s->stream);
-    free_tape(s);
-    return true;
+bool free_idle_tapes() {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    IdleTapes& idle = idle_tapes();
+    std::lock_guard<std::mutex> lock(idle.mu);
+    bool freed = false;
+    for (Tape* t : idle.list)
+        if (t->device == device && t->mem) {
+            cudaFree(t->mem);
+            t->mem = nullptr;  // (its handle allocates anew: claim)
+            freed = true;
+        }
+    return freed;
 }
 
 }  // namespace pbf
@@ -1025,13 +1078,14 @@ pbf_status pbf_forward_record(pbf_sim* s, uint32_t substeps, uint32_t checkpoint
     const bool vort = s->params.vorticity_confinement != 0;
     Tape* t = s->tape;
     // (the recorded lists' capacity follows the handle's)
-    if (t && !(t->substeps == substeps && t->every == every && t->iters == iters &&
+    if (t && !(claim(t) && t->substeps == substeps && t->every == every && t->iters == iters &&
                t->vort == vort && t->list_pairs == s->pair_cap)) {
         free_tape(s);
         t = nullptr;
     }
     if (!t) {
         t = s->tape = new Tape();
+        t->device = s->device;
         t->substeps = substeps;
         t->every = every;
         t->iters = iters;
@@ -1046,6 +1100,7 @@ pbf_status pbf_forward_record(pbf_sim* s, uint32_t substeps, uint32_t checkpoint
     }
     t->valid = false;
     t->held = Tape::kNone;
+    const ParkUnlessValid unless_valid{s};
     const size_t b = sizeof(float4) * s->n;
     // every segment but the last is stepped as usual and recorded when the
     // reverse pass reaches it; the last is recorded at once (its slots are the

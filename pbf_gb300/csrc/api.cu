@@ -290,7 +290,7 @@ bool rows_on(const pbf_sim* s) {
 std::atomic<int> g_fail_alloc_after{-1};
 
 template <typename T>
-cudaError_t dalloc(T** p, size_t count, pbf_sim* s = nullptr) {
+cudaError_t dalloc(T** p, size_t count) {
     int k = g_fail_alloc_after.load();
     while (k >= 0) {
         if (g_fail_alloc_after.compare_exchange_weak(k, k - 1)) {
@@ -301,14 +301,7 @@ cudaError_t dalloc(T** p, size_t count, pbf_sim* s = nullptr) {
             break;
         }
     }
-    const size_t bytes = sizeof(T) * (count > 0 ? count : 1);
-    cudaError_t e = cudaMalloc((void**)p, bytes);
-    // a tape that holds no recorded run gives its memory back first
-    if (e == cudaErrorMemoryAllocation && s && free_idle_tape(s)) {
-        cudaGetLastError();
-        e = cudaMalloc((void**)p, bytes);
-    }
-    return e;
+    return device_alloc(p, sizeof(T) * (count > 0 ? count : 1));
 }
 
 // (Re)allocates the neighbour-list and guard buffers for the current
@@ -321,8 +314,8 @@ cudaError_t ensure_lists(pbf_sim* s) {
         s->nbr_idx = nullptr;
         s->nbr_cnt = nullptr;
         s->nbr_cap = 0;
-        cudaError_t e = dalloc(&s->nbr_idx, (size_t)(cap > 0 ? cap : 1) * s->n, s);
-        if (e == cudaSuccess) e = dalloc(&s->nbr_cnt, s->n, s);
+        cudaError_t e = dalloc(&s->nbr_idx, (size_t)(cap > 0 ? cap : 1) * s->n);
+        if (e == cudaSuccess) e = dalloc(&s->nbr_cnt, s->n);
         if (e != cudaSuccess) return e;
         s->nbr_cap = cap;
     }
@@ -334,8 +327,8 @@ cudaError_t ensure_lists(pbf_sim* s) {
         s->pair_cnt = nullptr;
         s->pair_cap = 0;
         if (pcap > 0) {
-            cudaError_t e = dalloc(&s->pair_idx, (size_t)pcap * s->n, s);
-            if (e == cudaSuccess) e = dalloc(&s->pair_cnt, s->n, s);
+            cudaError_t e = dalloc(&s->pair_idx, (size_t)pcap * s->n);
+            if (e == cudaSuccess) e = dalloc(&s->pair_cnt, s->n);
             if (e != cudaSuccess) return e;
             s->pair_cap = pcap;
         }
@@ -345,7 +338,7 @@ cudaError_t ensure_lists(pbf_sim* s) {
         if (s->guard) cudaFree(s->guard);
         s->guard = nullptr;
         s->guard_slots = 0;
-        cudaError_t e = dalloc(&s->guard, slots, s);
+        cudaError_t e = dalloc(&s->guard, slots);
         if (e != cudaSuccess) return e;
         s->guard_slots = slots;
     }
@@ -808,7 +801,7 @@ pbf_status pbf_create_batch(const pbf_params* scene_params, const uint32_t* scen
         ALLOC(d_consts, num_scenes) ALLOC(sid, n) ALLOC(sid_sorted, n)
     }
 #undef ALLOC
-    if (e == cudaSuccess) e = cudaMalloc(&s->sort_mem, SortWorkspace::bytes_for(n));
+    if (e == cudaSuccess) e = device_alloc(&s->sort_mem, SortWorkspace::bytes_for(n));
     if (e == cudaSuccess) e = ensure_lists(s);
     if (e == cudaSuccess) e = cudaMallocHost((void**)&s->h_status, 2 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking);
@@ -968,8 +961,8 @@ pbf_status pbf_autotune(pbf_sim* s, uint32_t trial_substeps, pbf_tuning* best) {
     DeviceGuard dg(s->device);
     const size_t b = sizeof(float4) * s->n;
     float4 *sx = nullptr, *sv = nullptr;
-    PBF_CUDA(s, cudaMalloc(&sx, b));
-    cudaError_t e = cudaMalloc(&sv, b);
+    PBF_CUDA(s, device_alloc(&sx, b));
+    cudaError_t e = device_alloc(&sv, b);
     if (e != cudaSuccess) {
         cudaFree(sx);
         return cuda_fail(s, e, "autotune snapshot");
@@ -1375,7 +1368,7 @@ pbf_status pbf_radix_sort(const uint32_t* keys_in, uint32_t* keys_out, uint32_t*
         }
         const size_t wsb = (SortWorkspace::bytes_for(n) + 255) & ~size_t(255);
         const size_t bytes = wsb + sizeof(uint32_t) * (size_t)n;
-        cudaError_t e = cudaMalloc(&c.mem, bytes);
+        cudaError_t e = device_alloc(&c.mem, bytes);
         if (e != cudaSuccess) return cuda_fail(nullptr, e, "sort scratch allocation");
         c.capacity = n;
         c.ws.carve(c.mem, n);
@@ -1421,7 +1414,12 @@ pbf_status pbf_highlight_neighbours(pbf_sim* s, uint32_t* flags, int where) {
     const size_t b = sizeof(uint32_t) * s->n;
     uint32_t* d = flags;
     if (where == PBF_HOST) {
-        PBF_CUDA(s, cudaMallocAsync((void**)&d, b, st));
+        cudaError_t e = cudaMallocAsync((void**)&d, b, st);
+        if (e == cudaErrorMemoryAllocation && free_idle_tapes()) {
+            cudaGetLastError();
+            e = cudaMallocAsync((void**)&d, b, st);
+        }
+        PBF_CUDA(s, e);
         PBF_CUDA(s, cudaMemcpyAsync(d, flags, b, cudaMemcpyHostToDevice, st));
     }
     const unsigned g = grid_for(s->n);

@@ -132,10 +132,24 @@ cudaError_t enqueue_substep(pbf_sim* s, cudaEvent_t* ev, const Recording* rec = 
 pbf_status recorded_substep(pbf_sim* s, const Recording& rec);
 void invalidate_graph(pbf_sim* s);
 void free_tape(pbf_sim* s);
-// Drops the recorded run but keeps its buffers for the next one.
+// Drops the recorded run but keeps its buffers for the next one, or for any
+// allocation of the library that needs their memory (device_alloc).
 void invalidate_tape(pbf_sim* s);
-// Frees the buffers when they hold no recorded run; whether it freed any.
-bool free_idle_tape(pbf_sim* s);
+// Frees the buffers of every handle on the current device that hold no recorded
+// run; whether it freed any.
+bool free_idle_tapes();
+
+// Device memory for the library: cudaMalloc, and again after free_idle_tapes
+// where that finds none.
+template <typename T>
+cudaError_t device_alloc(T** p, size_t bytes) {
+    cudaError_t e = cudaMalloc((void**)p, bytes);
+    if (e == cudaErrorMemoryAllocation && free_idle_tapes()) {
+        cudaGetLastError();
+        e = cudaMalloc((void**)p, bytes);
+    }
+    return e;
+}
 
 struct DeviceGuard {
     int prev = -1;

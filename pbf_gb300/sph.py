@@ -336,7 +336,8 @@ class SPH:
     PARAM_NAMES = ("epsilon", "tensile_instability_k", "xsph_viscosity_c", "vorticity_epsilon")
 
     def forward_record(self, substeps: int, checkpoint_every: int = 8) -> None:
-        """Steps like step() and records what backward() needs (pbf_forward_record)."""
+        """Steps like step() and records what backward() needs (pbf_forward_record).
+        The handle keeps the memory for the next recorded run: release_record()."""
         check(self._lib.pbf_forward_record(self._h, int(substeps), int(checkpoint_every)),
               self._h)
 
@@ -365,6 +366,7 @@ class SPH:
         return np.array([[getattr(grads[k], nm) for nm in self.PARAM_NAMES] for k in range(ns)])
 
     def release_record(self) -> None:
+        """Frees the recording and its memory (pbf_release_record)."""
         check(self._lib.pbf_release_record(self._h), self._h)
 
     # ---- debug reads of the last substep ---------------------------------------
