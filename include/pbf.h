@@ -200,7 +200,9 @@ typedef struct pbf_tuning {
                                      full stencil scan for that particle */
     float skin_h;                 /* list radius is h * (1 + skin_h) */
     uint32_t block_size;          /* threads per block of the neighbour sweeps: a
-                                     multiple of 32 in [32, 256]; 0 = 256 */
+                                     multiple of 32 in [32, 256]; 0 (default): chosen by
+                                     the library, 256, and up to 1,024 for the scanning
+                                     sweeps of scenes from 1,572,864 particles */
     uint32_t sweep_mode;          /* PBF_SWEEP_DIRECT: a full stencil scan evaluates each
                                      candidate within h where it finds it;
                                      PBF_SWEEP_MASKED (default): it scans each run in
@@ -270,7 +272,8 @@ pbf_status pbf_get_tuning(const pbf_sim* sim, pbf_tuning* out);
 pbf_status pbf_get_sweep_choice(const pbf_sim* sim, uint32_t out[3]);
 
 /* Autotuner: times `trial_substeps` substeps from the current state under
- * each candidate tuning (sweep block size 128 / 256; direct or masked
+ * each candidate tuning (sweep block size 128 / 256, or 128 / 0 from 1,572,864
+ * particles; direct or masked
  * sweeps; neighbour lists off, or on with skin 0.05h / 0.1h / 0.2h),
  * restoring the state before every trial
  * and after the last, and keeps the fastest, which it also writes to `best`

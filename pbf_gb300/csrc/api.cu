@@ -15,6 +15,7 @@
 #include "../../include/pbf.h"
 #include "common.cuh"
 #include "internal.h"
+#include "scan_block.h"
 #include "sim.h"
 #include "sort.cuh"
 #include "substep.cuh"
@@ -166,7 +167,7 @@ pbf_tuning default_tuning() {
     t.use_neighbour_lists = 0;
     t.list_capacity = 128;
     t.skin_h = 0.15f;
-    t.block_size = 256;
+    t.block_size = 0;
     t.sweep_mode = PBF_SWEEP_AUTO;
     t.pair_list_capacity = 128;
     return t;
@@ -233,23 +234,6 @@ bool pass_mixed(const pbf_sim* s, uint32_t pass) {
     if (s->tuning.coop_candidates == 0) return false;
     const PassModes m = modes_of(s, pass);
     return m.first != 3 || m.second != 3;
-}
-// Threads per block of the scanning sweeps under the default block size.  The
-// blocks that share an SM come from all over the particle order, so a larger
-// block means fewer places whose records and lists have to fit in the SM's L1;
-// it also waits longer for its slowest warp.  Measured at 256 / 512 / 1024
-// threads, us per launch: 9.3 million particles in 256 scenes lambda 2,410 /
-// 2,159 / 1,976, vorticity A (at most 512: registers) 2,570 / 2,328; 2,097,152
-// lambda 466 / 454 / 464, vorticity A 541 / 537; 1.2 million lambda 259 / 263 /
-// 278; 250,000 lambda 57.5 / 62.3 / 61.6.
-constexpr uint32_t kMidScene = 1572864, kLargeScene = 4194304;
-unsigned lam_block(const pbf_sim* s, unsigned blk) {
-    if (blk != (unsigned)kBlock) return blk;
-    return s->n < kMidScene ? blk : s->n < kLargeScene ? 512u : 1024u;
-}
-unsigned vort_block(const pbf_sim* s, unsigned blk) {
-    if (blk != (unsigned)kBlock) return blk;
-    return s->n < kMidScene ? blk : 512u;
 }
 uint32_t heavy_threshold(const pbf_sim* s) {
     return s->tuning.coop_candidates ? s->tuning.coop_candidates : kMixedCandidates;
@@ -535,15 +519,17 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
     if (!s->nbr_cnt || s->guard_slots < 2 + s->params.num_solver_iterations)
         return cudaErrorInvalidValue;  // ensure_lists() runs before any capture
     const unsigned g = grid_for(n);
-    const unsigned blk = s->tuning.block_size ? s->tuning.block_size : (unsigned)kBlock;
+    const uint32_t asked = s->tuning.block_size;
+    const unsigned blk = asked ? asked : kScanBlock;
     const bool lists = skin_lists_on(s);
     auto modes = [&](uint32_t pass) {
         return !pass_quads(s, pass) ? modes_of(s, pass)
                : s->n < kQuadScanBelow ? PassModes{4, 4} : PassModes{2, 4};
     };
     const PassModes ms = modes(s->pass_solver), mv = modes(s->pass_vort);
-    const SweepCfg s_lam{lam_block(s, blk), ms.first, lists}, s_dp{blk, ms.second, lists},
-        s_va{vort_block(s, blk), mv.first, lists}, s_vb{blk, mv.second, lists};
+    const SweepCfg s_lam{scan_block(asked, n, kLambdaMaxBlock), ms.first, lists},
+        s_dp{blk, ms.second, lists}, s_va{scan_block(asked, n, kVortMaxBlock), mv.first, lists},
+        s_vb{blk, mv.second, lists};
     const bool vort = s->params.vorticity_confinement != 0;
     // delta-p writes the scan copy of its output when a sweep reading that
     // position set scans through it (masked modes; a pair-list replay falls
@@ -985,7 +971,9 @@ pbf_status pbf_autotune(pbf_sim* s, uint32_t trial_substeps, pbf_tuning* best) {
     }
     const pbf_tuning original = s->tuning;
     std::vector<pbf_tuning> cand;
-    for (uint32_t blk : {128u, 256u})
+    // (the larger blocks of large scenes are the library's own choice)
+    const uint32_t full = s->n < kMidScene ? kScanBlock : 0u;
+    for (uint32_t blk : {128u, full})
         for (uint32_t mode : {(uint32_t)PBF_SWEEP_DIRECT, (uint32_t)PBF_SWEEP_MASKED}) {
             pbf_tuning t = original;
             t.block_size = blk;
@@ -1003,11 +991,12 @@ pbf_status pbf_autotune(pbf_sim* s, uint32_t trial_substeps, pbf_tuning* best) {
     {
         pbf_tuning t = original;  // the warp-cooperative sweeps (block size and lists unused)
         t.sweep_mode = PBF_SWEEP_COOP;
+        if (t.block_size == 0) t.block_size = full;
         t.use_neighbour_lists = 0;
         t.coop_candidates = 0;
         cand.push_back(t);
         t.sweep_mode = PBF_SWEEP_MASKED;  // mixed: warps for the particles in dense stencils
-        t.block_size = 256;
+        t.block_size = full;
         t.coop_candidates = kMixedCandidates;
         cand.push_back(t);
     }

@@ -428,10 +428,6 @@ constexpr int kSweepBlocksPerSM = 8;
 // than 8 blocks with spills on the 2M window.
 constexpr int kVortThreadsPerSM = 1536;
 
-// Largest blocks the scanning sweeps are launched with (api.cu: lam_block,
-// vort_block), at the same registers per thread.
-constexpr int kLambdaMaxBlock = 1024, kVortMaxBlock = 512;
-
 // Instantiations of the sweep kernels (pbf_tuning): MODE is the stencil scan
 // (kDirect: the reference's loop shape; kMasked: masked scans; kPairs: masked
 // scans recording the exact pair lists the next sweep replays), LISTS whether

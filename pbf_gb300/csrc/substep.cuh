@@ -30,6 +30,9 @@ __global__ void k_find_cells(const uint32_t* __restrict__ skeys, const uint32_t*
 // candidates, and as first sweeps (which scan) scenes below this many particles.
 constexpr uint32_t kQuadCandidates = 256;
 constexpr uint32_t kQuadScanBelow = 49152;
+// Largest blocks of the scanning sweeps (scan_block.h), at the same registers
+// per thread.
+constexpr unsigned kLambdaMaxBlock = 1024, kVortMaxBlock = 512;
 
 struct SweepCfg {
     unsigned block;
