@@ -201,8 +201,9 @@ typedef struct pbf_tuning {
     float skin_h;                 /* list radius is h * (1 + skin_h) */
     uint32_t block_size;          /* threads per block of the neighbour sweeps: a
                                      multiple of 32 in [32, 256]; 0 (default): chosen by
-                                     the library, 256, and up to 1,024 for the scanning
-                                     sweeps of scenes from 1,572,864 particles */
+                                     the library, 256, and up to 1,024 for the sweeps
+                                     that record pair lists of scenes from 1,572,864
+                                     particles */
     uint32_t sweep_mode;          /* PBF_SWEEP_DIRECT: a full stencil scan evaluates each
                                      candidate within h where it finds it;
                                      PBF_SWEEP_MASKED (default): it scans each run in

@@ -527,9 +527,11 @@ cudaError_t enqueue_impl(pbf_sim* s, cudaEvent_t* ev, const Recording* rec, cons
                : s->n < kQuadScanBelow ? PassModes{4, 4} : PassModes{2, 4};
     };
     const PassModes ms = modes(s->pass_solver), mv = modes(s->pass_vort);
-    const SweepCfg s_lam{scan_block(asked, n, kLambdaMaxBlock), ms.first, lists},
-        s_dp{blk, ms.second, lists}, s_va{scan_block(asked, n, kVortMaxBlock), mv.first, lists},
-        s_vb{blk, mv.second, lists};
+    auto scan = [&](int mode, unsigned largest) {
+        return SweepCfg{scan_block(asked, n, mode == 2 && !lists, largest), mode, lists};
+    };
+    const SweepCfg s_lam = scan(ms.first, kLambdaMaxBlock), s_dp{blk, ms.second, lists},
+                   s_va = scan(mv.first, kVortMaxBlock), s_vb{blk, mv.second, lists};
     const bool vort = s->params.vorticity_confinement != 0;
     // delta-p writes the scan copy of its output when a sweep reading that
     // position set scans through it (masked modes; a pair-list replay falls

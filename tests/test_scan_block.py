@@ -1,6 +1,7 @@
 """CPU test of the scanning sweeps' block size (pbf_gb300/csrc/scan_block.h): a
 size that the caller chose is kept at every particle count, 256 too; the
-library's own choice is 256 threads below 1,572,864 particles."""
+library's own choice is 256 threads below 1,572,864 particles, and at every count
+for the sweeps that record no pair lists."""
 import os
 import shutil
 import subprocess
@@ -20,9 +21,12 @@ int main() {
     const unsigned own[] = {256, 256, 512, 512, 1024, 1024};
     for (int k = 0; k < 6; ++k) {
         for (uint32_t asked : {32u, 96u, 128u, 256u})
-            for (unsigned largest : {512u, 1024u}) bad += scan_block(asked, sizes[k], largest) != asked;
-        bad += scan_block(0, sizes[k], 1024) != own[k];
-        bad += scan_block(0, sizes[k], 512) != (own[k] < 512 ? own[k] : 512);
+            for (unsigned largest : {512u, 1024u})
+                for (bool pairs : {false, true})
+                    bad += scan_block(asked, sizes[k], pairs, largest) != asked;
+        bad += scan_block(0, sizes[k], true, 1024) != own[k];
+        bad += scan_block(0, sizes[k], true, 512) != (own[k] < 512 ? own[k] : 512);
+        bad += scan_block(0, sizes[k], false, 1024) != 256;
     }
     std::printf("%d bad\n", bad);
     return bad;
