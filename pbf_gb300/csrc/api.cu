@@ -1292,10 +1292,10 @@ public:
                 free_words().pop_back();
             }
         }
-        if (!word_ && cudaHostAlloc((void**)&word_, sizeof(uint32_t),
-                                    cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-            cudaGetLastError();
-            word_ = nullptr;
+        if (!word_) {
+            error_ = cudaHostAlloc((void**)&word_, sizeof(uint32_t),
+                                   cudaHostAllocPortable | cudaHostAllocMapped);
+            if (error_ != cudaSuccess) word_ = nullptr;
         }
         if (word_) *word_ = 0u;
     }
@@ -1312,7 +1312,8 @@ public:
     }
     StatusWord(const StatusWord&) = delete;
     StatusWord& operator=(const StatusWord&) = delete;
-    uint32_t* get() const { return word_; }  // NULL: no memory
+    uint32_t* get() const { return word_; }  // NULL: error()
+    cudaError_t error() const { return error_; }
     uint32_t read() const { return *(volatile uint32_t*)word_; }
 
 private:
@@ -1326,6 +1327,7 @@ private:
         return *v;
     }
     uint32_t* word_ = nullptr;
+    cudaError_t error_ = cudaSuccess;
 };
 std::mutex g_scratch_mu;
 std::map<int, CachedSortScratch> g_scratch;
@@ -1367,7 +1369,7 @@ pbf_status pbf_radix_sort(const uint32_t* keys_in, uint32_t* keys_out, uint32_t*
     }
     uint32_t* kout = keys_out ? keys_out : c.keys_scratch;
     StatusWord status;
-    if (!status.get()) return fail(nullptr, PBF_ERR_OUT_OF_MEMORY, "pbf_radix_sort: status word");
+    if (!status.get()) return cuda_fail(nullptr, status.error(), "pbf_radix_sort status word");
     cudaError_t e = sort_pairs(c.ws, keys_in, kout, perm_out, n, numbits, status.get(), st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(nullptr, e, "pbf_radix_sort");
@@ -1383,7 +1385,7 @@ pbf_status pbf_find_cells(const uint32_t* sorted_keys, uint32_t n, uint32_t num_
     if (num_cells > 0x7FFFFFFFu || n > 0x7FFFFFFFu) return fail(nullptr, PBF_ERR_INVALID_ARGUMENT, "sizes above 2^31-1");
     cudaStream_t st = (cudaStream_t)stream;
     StatusWord bad;
-    if (!bad.get()) return fail(nullptr, PBF_ERR_OUT_OF_MEMORY, "pbf_find_cells: status word");
+    if (!bad.get()) return cuda_fail(nullptr, bad.error(), "pbf_find_cells status word");
     launch_empty_cells(st, start, end, num_cells);
     if (n > 0)
         k_find_cells<<<grid_for(n), kBlock, 0, st>>>(sorted_keys, nullptr, nullptr, nullptr, n,
