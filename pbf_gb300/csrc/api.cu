@@ -1281,10 +1281,12 @@ struct CachedSortScratch {
 // fill, no copy back and no device allocation in between (those were 150 of the
 // 257 us that a sort and a cell pass of 16,384 keys took).  Each call holds a
 // word of its own, so calls from several threads and streams do not meet; up to
-// kWordsKept free words are kept for later calls, the others freed.
+// kWordsKept free words are kept for later calls, the others freed.  The call's
+// kernels may write the word until they have ended, so the stream is waited for
+// (finish) before the word goes back, on the error paths too.
 class StatusWord {
 public:
-    StatusWord() {
+    explicit StatusWord(cudaStream_t st) : stream_(st) {
         {
             std::lock_guard<std::mutex> lock(mu());
             if (!free_words().empty()) {
@@ -1301,6 +1303,7 @@ public:
     }
     ~StatusWord() {
         if (!word_) return;
+        finish(cudaSuccess);
         {
             std::lock_guard<std::mutex> lock(mu());
             if (free_words().size() < kWordsKept) {
@@ -1315,6 +1318,15 @@ public:
     uint32_t* get() const { return word_; }  // NULL: error()
     cudaError_t error() const { return error_; }
     uint32_t read() const { return *(volatile uint32_t*)word_; }
+    // Waits for the stream; the first error of `e` and the wait.
+    cudaError_t finish(cudaError_t e) {
+        if (!finished_) {
+            const cudaError_t w = cudaStreamSynchronize(stream_);
+            finished_ = true;
+            if (e == cudaSuccess) e = w;
+        }
+        return e;
+    }
 
 private:
     static constexpr size_t kWordsKept = 64;
@@ -1326,6 +1338,8 @@ private:
         static std::vector<uint32_t*>* v = new std::vector<uint32_t*>;  // outlives every caller
         return *v;
     }
+    cudaStream_t stream_;
+    bool finished_ = false;
     uint32_t* word_ = nullptr;
     cudaError_t error_ = cudaSuccess;
 };
@@ -1368,10 +1382,10 @@ pbf_status pbf_radix_sort(const uint32_t* keys_in, uint32_t* keys_out, uint32_t*
         c.keys_scratch = (uint32_t*)((uint8_t*)c.mem + wsb);
     }
     uint32_t* kout = keys_out ? keys_out : c.keys_scratch;
-    StatusWord status;
+    StatusWord status(st);
     if (!status.get()) return cuda_fail(nullptr, status.error(), "pbf_radix_sort status word");
-    cudaError_t e = sort_pairs(c.ws, keys_in, kout, perm_out, n, numbits, status.get(), st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    const cudaError_t e = status.finish(
+        sort_pairs(c.ws, keys_in, kout, perm_out, n, numbits, status.get(), st));
     if (e != cudaSuccess) return cuda_fail(nullptr, e, "pbf_radix_sort");
     if (status.read() & kDevSortTimeout)
         return fail(nullptr, PBF_ERR_DEVICE_FAULT, "radix-sort lookback timed out");
@@ -1384,7 +1398,7 @@ pbf_status pbf_find_cells(const uint32_t* sorted_keys, uint32_t n, uint32_t num_
     if (n > 0 && !sorted_keys) return fail(nullptr, PBF_ERR_INVALID_ARGUMENT, "sorted_keys is NULL");
     if (num_cells > 0x7FFFFFFFu || n > 0x7FFFFFFFu) return fail(nullptr, PBF_ERR_INVALID_ARGUMENT, "sizes above 2^31-1");
     cudaStream_t st = (cudaStream_t)stream;
-    StatusWord bad;
+    StatusWord bad(st);
     if (!bad.get()) return cuda_fail(nullptr, bad.error(), "pbf_find_cells status word");
     launch_empty_cells(st, start, end, num_cells);
     if (n > 0)
@@ -1392,8 +1406,7 @@ pbf_status pbf_find_cells(const uint32_t* sorted_keys, uint32_t n, uint32_t num_
                                                      num_cells, start, end, bad.get(), nullptr,
                                                      nullptr, ScanPos{nullptr, nullptr}, nullptr,
                                                      nullptr);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    const cudaError_t e = bad.finish(cudaGetLastError());
     if (e != cudaSuccess) return cuda_fail(nullptr, e, "pbf_find_cells");
     if (bad.read()) return fail(nullptr, PBF_ERR_INVALID_ARGUMENT, "a sorted key is >= num_cells");
     return PBF_OK;
