@@ -927,8 +927,9 @@ cudaError_t alloc_tape(pbf_sim* s, Tape* t) {
     }
     Carver a{(uint8_t*)t->mem};
     carve_tape(s, t, a);
-    return cudaMemcpy(t->scene_first, s->offsets.data(), sizeof(uint32_t) * (s->nscenes + 1),
-                      cudaMemcpyHostToDevice);
+    // (on the handle's stream, which does not wait for a copy on the legacy one)
+    return cudaMemcpyAsync(t->scene_first, s->offsets.data(), sizeof(uint32_t) * (s->nscenes + 1),
+                           cudaMemcpyHostToDevice, s->stream);
 }
 
 template <class CP>

@@ -701,6 +701,14 @@ void bind_checks(pbf_sim* s) {
     if (!s->sdc.empty()) s->dc = s->sdc[0];
 }
 
+// Sends scenes' constants to the device on the handle's stream: a plain copy may
+// return before its transfer ends, and runs on the legacy stream, for which the
+// handle's own (non-blocking) stream does not wait.
+cudaError_t send_consts(pbf_sim* s, uint32_t first, uint32_t count) {
+    return cudaMemcpyAsync(s->d_consts + first, &s->sdc[first], sizeof(DevConsts) * count,
+                           cudaMemcpyHostToDevice, s->stream);
+}
+
 pbf_status check_status(pbf_sim* s) {
     PBF_CUDA(s, cudaMemcpyAsync(s->h_status, s->status, 2 * sizeof(uint32_t),
                                 cudaMemcpyDeviceToHost, s->stream));
@@ -826,8 +834,7 @@ pbf_status pbf_create_batch(const pbf_params* scene_params, const uint32_t* scen
         }
         if (e == cudaSuccess) e = cudaMemsetAsync(s->skeys, 0, sizeof(uint32_t) * n, s->stream);
         if (e == cudaSuccess)
-            e = cudaMemcpy(s->d_consts, s->sdc.data(), sizeof(DevConsts) * num_scenes,
-                           cudaMemcpyHostToDevice);
+            e = send_consts(s, 0, num_scenes);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) {
@@ -882,9 +889,7 @@ pbf_status pbf_set_scene_params(pbf_sim* s, uint32_t scene, const pbf_params* p)
     if (scene == 0) s->params = *p;
     const uint32_t first = was_settled ? scene : 0u;  // (every scene's after a failed change)
     if (s->nscenes > 1)
-        PBF_CUDA(s, cudaMemcpy(s->d_consts + first, &s->sdc[first],
-                               sizeof(DevConsts) * (was_settled ? 1u : s->nscenes),
-                               cudaMemcpyHostToDevice));
+        PBF_CUDA(s, send_consts(s, first, was_settled ? 1u : s->nscenes));
     invalidate_graph(s);
     invalidate_tape(s);  // a recorded run is only valid for the parameters it ran with
     s->auto_trial = -1;  // a running trial's events may not match the new iteration count
@@ -933,8 +938,7 @@ pbf_status pbf_set_tuning(pbf_sim* s, const pbf_tuning* t) {
     for (uint32_t k = 0; k < s->nscenes; ++k) apply_tuning(s->sdc[k], s->sparams[k], s->tuning);
     s->dc = s->sdc[0];
     if (s->nscenes > 1)
-        PBF_CUDA(s, cudaMemcpy(s->d_consts, s->sdc.data(), sizeof(DevConsts) * s->nscenes,
-                               cudaMemcpyHostToDevice));
+        PBF_CUDA(s, send_consts(s, 0, s->nscenes));
     invalidate_graph(s);
     PBF_CUDA(s, ensure_lists(s));
     s->settled = true;
