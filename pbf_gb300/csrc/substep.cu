@@ -190,7 +190,7 @@ k_find_cells(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ pe
              const uint32_t* __restrict__ sid, uint32_t* __restrict__ sid_sorted, ScanPos sx,
              uint32_t* __restrict__ runs, uint32_t* status) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < n;
+    bool valid = i < n;
     if (status) {
         // neighbourcells.glsl:83 packs a 3-cell run's count into 8 bits
         // (foreachneighbour.glsl:5 drops counts >= 128).  Particles i and
@@ -203,10 +203,15 @@ k_find_cells(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ pe
     }
     float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #ifdef PBF_CHECK
-    if (valid && perm[i] >= n) {  // bounds-checked build: a bad permutation entry
-        atomicOr(status, kDevIndexFault);
-        return;
+    // bounds-checked build: a bad permutation entry (the standalone cell finder
+    // passes no permutation, and it and the diagnostics no status word)
+    auto entry_ok = [&](uint32_t k) { return !perm || perm[k] < n; };
+    if (valid && !entry_ok(i)) {
+        if (status) atomicOr(status, kDevIndexFault);
+        valid = false;  // (the lane stays for the warp's shuffles)
     }
+#else
+    auto entry_ok = [](uint32_t) { return true; };
 #endif
     if (valid && P0) {
         p = __ldg(xstar + perm[i]);
@@ -220,7 +225,8 @@ k_find_cells(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ pe
         float3 q = make_float3(__shfl_up_sync(0xFFFFFFFFu, p.x, 1),
                                __shfl_up_sync(0xFFFFFFFFu, p.y, 1),
                                __shfl_up_sync(0xFFFFFFFFu, p.z, 1));
-        if ((threadIdx.x & 31u) == 0u && valid && i > 0) q = xyz(__ldg(xstar + perm[i - 1]));
+        if ((threadIdx.x & 31u) == 0u && valid && i > 0 && entry_ok(i - 1))
+            q = xyz(__ldg(xstar + perm[i - 1]));
         store_run_bits(i, n, xyz(p), q, runs);
     }
     if (!valid) return;
