@@ -483,6 +483,11 @@ void pbf_debug_fail_allocation(int after);
  * invalid and the call that synchronises reports PBF_ERR_DEVICE_FAULT.  No
  * wait is unbounded and every write stays in bounds.  0 disarms. */
 void pbf_debug_sort_stall(uint32_t spins);
+/* Test hook (no reference counterpart): the PBF_PASS_* configurations of the
+ * solver sweeps and of the vorticity passes from the next substep on, whatever
+ * the sweep mode, until the next state upload, tuning change or trial.  No
+ * configuration changes any result. */
+pbf_status pbf_debug_set_passes(pbf_sim* sim, uint32_t solver, uint32_t vorticity);
 /* Message of the last failed call on `sim`, or of the last failed call
  * without a handle when sim is NULL.  Never NULL. */
 const char* pbf_last_error(const pbf_sim* sim);

@@ -164,6 +164,7 @@ SIGNATURES = {
     "pbf_status_string": (C.c_char_p, [C.c_int]),
     "pbf_debug_fail_allocation": (None, [C.c_int]),
     "pbf_debug_sort_stall": (None, [C.c_uint32]),
+    "pbf_debug_set_passes": (C.c_int, [_P, C.c_uint32, C.c_uint32]),
     "pbf_last_error": (C.c_char_p, [_P]),
     "pbf_abi_version": (C.c_int, []),
 }

@@ -1483,6 +1483,16 @@ pbf_status pbf_load_state(pbf_sim* s, const char* path) {
 
 void pbf_debug_fail_allocation(int after) { g_fail_alloc_after.store(after < 0 ? -1 : after); }
 
+pbf_status pbf_debug_set_passes(pbf_sim* s, uint32_t solver, uint32_t vorticity) {
+    if (!s) return fail(nullptr, PBF_ERR_INVALID_ARGUMENT, "sim is NULL");
+    if (solver > PBF_PASS_MIXED || vorticity > PBF_PASS_MIXED)
+        return fail(s, PBF_ERR_INVALID_ARGUMENT, "not a PBF_PASS_* value");
+    s->pass_solver = solver;
+    s->pass_vort = vorticity;
+    s->auto_trial = -1;
+    return PBF_OK;
+}
+
 const char* pbf_last_error(const pbf_sim* s) {
     if (s) return s->err.c_str();
     return g_error.c_str();
