@@ -289,8 +289,10 @@ __device__ __forceinline__ bool fragment(const Sprite& q, const Tri& t0, const T
     return d < seen;
 }
 
-// Depth pass.  A warp takes kGroup sprites: its first lanes project them
-// and the whole warp fills them one after the other, 8 x 4 pixels at a time.
+// Depth pass.  A warp takes kGroup sprites, a share of its lanes each.  Where none
+// of them has more than kSmallPixels pixels in its box every share fills its own
+// sprite, otherwise the whole warp fills them one after the other, 8 x 4 pixels at
+// a time.
 //
 // What bounds it: instruction issue and the latency of the pixel reads.  A
 // fragment's depth takes 12 rounded divisions, and a million sprites at 1920 x
@@ -299,11 +301,20 @@ __device__ __forceinline__ bool fragment(const Sprite& q, const Tri& t0, const T
 // there (read kTiles tiles at a time; an older, larger value at worst) is
 // dropped before any interpolation, and a fragment by its estimated depth.
 // That pays when the front sprites come first (sprite_order); back to front,
-// the million took 3,190 us.  Four sprites per warp give a scene of some ten
-// thousand enough warps, eight spend less on projecting them: 65,536 sprites
-// 58 and 72 us, 1,046,272 sprites 704 and 648 us; the line is kManySprites.
-// Measured, us: 65,536 sprites at 1280 x 720 99 -> 58; 1,046,272 at 1920 x
-// 1080 1,919 -> 648 (in a random order 891 at four per warp).
+// the million took 3,190 us.  Filled by the whole warp, a sprite of a few pixels
+// waits for its pixel reads and its triangles all the same, one sprite after the
+// other.  Measured, us, whole call (35 of them the launches, the fill and the
+// wait): a thread per sprite without the depth bound / all sprites by the warp /
+// as now:
+//   1,000,000 sprites at spacing 0.5 on 320 x 240 134 / 245 / 129, on 1280 x 720
+//     - / 345 / 250, on 1920 x 1080 - / 515 / 453; 65,600 on 320 x 240 45 / 56 / 45,
+//     on 1280 x 720 - / 77 / 71.
+// kSmallPixels: 8, 32 and 128 for the million on 1280 x 720 300 / 301 / 250, on 640 x
+// 480 257 / 200 / 173; no case was slower with 128.  Four sprites per warp give a
+// scene of some ten thousand enough warps, eight spend less on projecting them:
+// 65,600 sprites on 1920 x 1080 96 and 109, on 320 x 240 52 and 47; 262,144 on 1280 x
+// 720 129 and 119, 1,000,000 on 1920 x 1080 475 and 454.  The lines are kManySprites
+// and, on images below kSmallImage pixels, kManyOnSmallImage.
 constexpr int kTiles = 2;
 
 // The order in which the groups of sprites are taken, from 16 sprites spread
@@ -347,6 +358,8 @@ __device__ __forceinline__ Order sprite_order(const float4* __restrict__ pos, ui
 }
 
 constexpr uint32_t kManySprites = 262144;
+constexpr uint32_t kSmallImage = 500000, kManyOnSmallImage = 16384;
+constexpr int kSmallPixels = 128;
 template <uint32_t kGroup>
 __global__ void __launch_bounds__(128, 8)
 k_splat_depth(const float4* __restrict__ pos, uint32_t n, View view, uint32_t W, uint32_t H,
@@ -357,20 +370,49 @@ k_splat_depth(const float4* __restrict__ pos, uint32_t n, View view, uint32_t W,
     const Order order = sprite_order(pos, n, kGroup, view);
     const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (group >= order.groups) return;
-    const uint32_t k = order.at(group) * kGroup + lane;
+    // every lane of a sprite's share projects it (as fast as one of them would)
+    constexpr uint32_t kShare = 32 / kGroup;
+    const uint32_t slot = lane / kShare, part = lane & (kShare - 1u);
+    const uint32_t k = order.at(group) * kGroup + slot;
     bool drawn = false;
-    if (lane < kGroup && k < n) {
+    int pixels = 0;
+    if (k < n) {
         Sprite q;
         drawn = make_sprite<PBF_SPLAT_DEPTH>(pos[k], view, W, H, q);
-        if (drawn) mine[lane] = q;
+        if (drawn) {
+            pixels = (q.x1 - q.x0 + 1) * (q.y1 - q.y0 + 1);
+            if (part == 0u) mine[slot] = q;
+        }
     }
     __syncwarp();
-    uint32_t todo = __ballot_sync(0xFFFFFFFFu, drawn);
+    if (!__any_sync(0xFFFFFFFFu, pixels > kSmallPixels)) {
+        if (!drawn) return;
+        const Sprite& s = mine[slot];
+        const int cols = s.x1 - s.x0 + 1;
+        Tri t0, t1;
+        bool made = false;
+        for (int p = (int)part; p < pixels; p += (int)kShare) {
+            const int row = p / cols, tx = s.x0 + p - row * cols, ty = s.y0 + row;
+            float* const at = out + (size_t)ty * W + tx;
+            const float seen = __ldcg(at);
+            if (seen < s.dlow) continue;
+            if (!made) {
+                t0 = make_tri(s, 0, 2, 1);
+                t1 = make_tri(s, 2, 0, 3);
+                made = true;
+            }
+            float d;
+            if (fragment<PBF_SPLAT_DEPTH>(s, t0, t1, view, tx, ty, seen, d))
+                atomicMin(reinterpret_cast<unsigned int*>(at), __float_as_uint(d));
+        }
+        return;
+    }
+    uint32_t todo = __ballot_sync(0xFFFFFFFFu, drawn && part == 0u);
     const int dx = (int)(lane & 7u), dy = (int)(lane >> 3);
     while (todo) {
         const int src = __ffs((int)todo) - 1;
         todo &= todo - 1;
-        const Sprite& s = mine[src];
+        const Sprite& s = mine[src / (int)kShare];
         Tri t0, t1;  // made for the first tile that may be in front
         bool made = false;
         const int cols = (s.x1 - s.x0 + 8) >> 3, tiles = cols * ((s.y1 - s.y0 + 4) >> 2);
@@ -535,7 +577,9 @@ extern "C" pbf_status pbf_splat(int pass, const float* positions, uint32_t n, co
     if (n > 0) {
         const float4* p = (const float4*)positions;
         if (pass == PBF_SPLAT_DEPTH) {
-            if (n < kManySprites)
+            const bool many = n >= kManySprites ||
+                              (n >= kManyOnSmallImage && count < kSmallImage);
+            if (!many)
                 k_splat_depth<4><<<(n + 15) / 16, 128, 0, st>>>(p, n, v, width, height, out);
             else
                 k_splat_depth<8><<<(n + 31) / 32, 128, 0, st>>>(p, n, v, width, height, out);
