@@ -469,10 +469,19 @@ k_splat_depth(const float4* __restrict__ pos, uint32_t n, View view, uint32_t W,
 // rounded weights (8 divisions a fragment) are needed at the disc's edge only.
 // Measured, us, both halves: 65,536 sprites at 512 x 512 25 -> 17;
 // 1,046,272 at 960 x 540 386 -> 234.
+// Few sprites, and sprites on a small image, are added pixel by pixel (!kRows: below
+// kFewSprites, or below kMoreSprites on images below kFewPixels): there the second
+// half costs more than its atomics save.  Whole call, us, pixels / rows: 4,096 sprites
+// on 320 x 240 37 / 44, on 640 x 480 46 / 46, on 960 x 540 50 / 48; 65,600 on 320 x
+// 240 41 / 44, on 480 x 360 47 / 45; 262,144 on 256 x 256 57 / 56; 400 on 1920 x 1080
+// 38 / 45.
 constexpr int kOwnPixels = 256;
+constexpr uint32_t kFewSprites = 1024, kMoreSprites = 131072, kFewPixels = 200000;
+template <bool kRows>
 __global__ void __launch_bounds__(128)
 k_splat_thickness(const float4* __restrict__ pos, uint32_t n, View view, uint32_t W, uint32_t H,
-                  int* __restrict__ diff) {
+                  float* __restrict__ out) {
+    int* const diff = reinterpret_cast<int*>(out);
     __shared__ Sprite shared[128];
     const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
@@ -488,10 +497,14 @@ k_splat_thickness(const float4* __restrict__ pos, uint32_t n, View view, uint32_
             bool on = false;
             for (int tx = q.x0; tx <= q.x1; ++tx) {
                 const bool in = fragment<PBF_SPLAT_THICKNESS>(q, t0, t1, view, tx, ty, 0.0f, unused);
+                if (!kRows) {
+                    if (in) atomicAdd(out + (size_t)ty * W + tx, 1.0f);
+                    continue;
+                }
                 if (in != on) atomicAdd(row + tx, in ? 1 : -1);
                 on = in;
             }
-            if (on && q.x1 + 1 < (int)W) atomicAdd(row + q.x1 + 1, -1);
+            if (kRows && on && q.x1 + 1 < (int)W) atomicAdd(row + q.x1 + 1, -1);
         }
     }
     __syncwarp();
@@ -506,6 +519,10 @@ k_splat_thickness(const float4* __restrict__ pos, uint32_t n, View view, uint32_
             for (int tx = s.x0 + dx; tx - dx <= s.x1; tx += 8) {
                 const bool in = tx <= s.x1 && ty <= s.y1 &&
                                 fragment<PBF_SPLAT_THICKNESS>(s, t0, t1, view, tx, ty, 0.0f, unused);
+                if (!kRows) {
+                    if (in) atomicAdd(out + (size_t)ty * W + tx, 1.0f);
+                    continue;
+                }
                 const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
                 int* const at = diff + (size_t)ty * W + tx;
                 if (in && (dx == 0 || !(m >> (lane - 1u) & 1u))) atomicAdd(at, 1);
@@ -516,17 +533,20 @@ k_splat_thickness(const float4* __restrict__ pos, uint32_t n, View view, uint32_
 }
 
 // Thickness pass, second half: running sums along each row, in place, as the
-// float counts that adding 1 at a time gives (it stops at 2^24).  One warp per
-// row, 128 pixels at a time.
-__global__ void __launch_bounds__(128)
-k_splat_count(float* __restrict__ out, uint32_t W, uint32_t H) {
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (row >= H) return;
-    float* const o = out + (size_t)row * W;
+// float counts that adding 1 at a time gives (it stops at 2^24).  A block per
+// row, kCountBlock pixels of it at a time, four per thread.  What bounds it: the
+// latency of one step of a row, so rows take one or two steps (a warp per row,
+// 128 pixels at a time, took 15 at 1920 pixels: 10 us of the call where a few
+// sprites are drawn).
+constexpr int kCountThreads = 256, kCountBlock = 4 * kCountThreads;
+__global__ void __launch_bounds__(kCountThreads) k_splat_count(float* __restrict__ out, uint32_t W) {
+    __shared__ int warps[kCountThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    float* const o = out + (size_t)blockIdx.x * W;
     int carry = 0;
-    for (uint32_t x0 = 0; x0 < W; x0 += 128) {
+    for (uint32_t x0 = 0; x0 < W; x0 += kCountBlock) {
         int v[4];
-        const uint32_t x = x0 + 4 * lane;
+        const uint32_t x = x0 + 4 * threadIdx.x;
 #pragma unroll
         for (int k = 0; k < 4; ++k) v[k] = x + k < W ? __float_as_int(o[x + k]) : 0;
         v[1] += v[0];
@@ -538,12 +558,20 @@ k_splat_count(float* __restrict__ out, uint32_t W, uint32_t H) {
             const int y = __shfl_up_sync(0xFFFFFFFFu, before, d);
             if ((int)lane >= d) before += y;
         }
-        const int total = __shfl_sync(0xFFFFFFFFu, before, 31);
+        if (lane == 31u) warps[warp] = before;
+        __syncthreads();
+        int total = 0;
         before += carry - v[3];
+#pragma unroll
+        for (uint32_t w = 0; w < kCountThreads / 32; ++w) {
+            if (w < warp) before += warps[w];
+            total += warps[w];
+        }
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (x + k < W) o[x + k] = (float)min(before + v[k], 1 << 24);
         carry += total;
+        __syncthreads();
     }
 }
 
@@ -584,8 +612,13 @@ extern "C" pbf_status pbf_splat(int pass, const float* positions, uint32_t n, co
             else
                 k_splat_depth<8><<<(n + 31) / 32, 128, 0, st>>>(p, n, v, width, height, out);
         } else {
-            k_splat_thickness<<<(n + 127) / 128, 128, 0, st>>>(p, n, v, width, height, (int*)out);
-            k_splat_count<<<(height + 3) / 4, 128, 0, st>>>(out, width, height);
+            const unsigned g = (n + 127) / 128;
+            if (n < kFewSprites || (n < kMoreSprites && count < kFewPixels)) {
+                k_splat_thickness<false><<<g, 128, 0, st>>>(p, n, v, width, height, out);
+            } else {
+                k_splat_thickness<true><<<g, 128, 0, st>>>(p, n, v, width, height, out);
+                k_splat_count<<<height, kCountThreads, 0, st>>>(out, width);
+            }
         }
     }
     cudaError_t e = cudaGetLastError();

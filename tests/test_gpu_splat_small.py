@@ -1,7 +1,7 @@
-"""GPU tests of the depth pass where sprites are filled by a share of a warp's
-lanes: boxes of one pixel up to the largest that a share fills and beyond, counts
-and images on both sides of the lines where the share changes, sprites of very
-different sizes in one warp."""
+"""GPU tests of the splat passes on small and wide images, and of the depth pass
+where sprites are filled by a share of a warp's lanes: boxes of one pixel up to
+the largest that a share fills and beyond, counts and images on both sides of the
+lines where the share changes, sprites of very different sizes in one warp."""
 import math
 
 import numpy as np
@@ -53,3 +53,24 @@ def test_box_sizes(gpu, oracle_mod, n, distance):
     same_as_oracle(oracle_mod, x4, v, 320, 200)
     x4[::3] = cloud(n, 1)[::3]  # mixed sizes
     same_as_oracle(oracle_mod, x4, v, 320, 200)
+
+
+@pytest.mark.parametrize("n", [1, 700, 1023, 1024, 1500])
+@pytest.mark.parametrize("w,h", [(447, 447), (448, 447), (1023, 197), (1024, 196), (1025, 196),
+                                 (2050, 101), (5, 16384), (13, 16001)])
+def test_thickness_added_or_summed_along_rows(gpu, oracle_mod, n, w, h):
+    # (below 1,024 sprites, or 200,000 pixels, they are added pixel by pixel); rows of one step and
+    # of several, of less than a thread's four pixels
+    x4 = cloud(n, 2)
+    for eye in ((9.0, 6.0, 7.0), (1.0, 3.5, 1.2)):
+        v = view(eye, w, h)
+        want = oracle_mod.splat(splat.THICKNESS, x4, *v.columns(), w, h)
+        got = splat.splat(splat.THICKNESS, x4, v, w, h).cpu().numpy()
+        assert np.array_equal(got, want), eye
+
+
+@pytest.mark.parametrize("n", [131071, 131072])
+def test_thickness_of_many_on_a_small_image(gpu, oracle_mod, n):
+    x4, v = cloud(n, 4), view((14.0, 10.0, 12.0), 300, 220)
+    want = oracle_mod.splat(splat.THICKNESS, x4, *v.columns(), 300, 220)
+    assert np.array_equal(splat.splat(splat.THICKNESS, x4, v, 300, 220).cpu().numpy(), want)
