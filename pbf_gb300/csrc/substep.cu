@@ -338,8 +338,9 @@ __device__ __forceinline__ void sweep_visit(uint32_t i, Ctr&& ctr, const DevCons
 // together over their own list positions (the same shape as the replaying
 // sweeps) instead of chunk by chunk.  A list longer than its capacity keeps
 // its first `cap` entries (and is marked -1 for the replaying sweep); the
-// candidates past them are found by walking the rows again, `near(j)` being
-// the in-range test, and evaluated in order.
+// candidates past them are found by walking the rows again from the last entry
+// on (the visit order is that of the sorted indices: the rows ascend), `near(j)`
+// being the in-range test, and evaluated in order.
 template <bool LIST, class S, class N, class F>
 __device__ __forceinline__ void scan_then_eval(uint32_t i, const DevConsts& c, const ScanPos& X,
                                                float3 pi, const PairLists& pw, S&& list, N&& near,
@@ -363,13 +364,13 @@ __device__ __forceinline__ void scan_then_eval(uint32_t i, const DevConsts& c, c
         }
     }
     if (tot > pw.cap) {
-        uint32_t rank = 0;
+        const int32_t from = (int32_t)out[(size_t)(pw.cap - 1u) * stride] + 1;
 #pragma unroll 1
         for (int o = 0; o < 9; ++o) {
             const int2 be = __ldg(pw.rows + (size_t)o * pw.n + i);
 #pragma unroll 1
-            for (int32_t j = be.x; j < be.y; ++j)
-                if ((uint32_t)j != i && near((uint32_t)j) && rank++ >= pw.cap) eval((uint32_t)j);
+            for (int32_t j = max(be.x, from); j < be.y; ++j)
+                if ((uint32_t)j != i && near((uint32_t)j)) eval((uint32_t)j);
         }
     }
 }
