@@ -346,8 +346,7 @@ void free_sim(pbf_sim* s) {
                     s->VS, s->VX, s->OM,    s->Q,    s->keys,   s->skeys, s->perm,
                     s->cstart, s->cend, s->status, s->sort_mem, s->nbr_idx, s->nbr_cnt,
                     s->guard, s->d_consts, s->sid, s->sid_sorted, s->pair_idx, s->pair_cnt,
-                    s->scan_xy, s->scan_z, s->heavy, s->heavy_list, s->heavy_count,
-                    s->runs, s->rows};
+                    s->sweep_mem};
     for (void* b : bufs)
         if (b) cudaFree(b);
     if (s->h_status) cudaFreeHost(s->h_status);
@@ -790,9 +789,27 @@ pbf_status pbf_create_batch(const pbf_params* scene_params, const uint32_t* scen
     ALLOC(x, n) ALLOC(v, n) ALLOC(xstar, n) ALLOC(XP, n) ALLOC(Pa, n) ALLOC(Pb, n) ALLOC(L, n)
     ALLOC(VS, n) ALLOC(VX, n) ALLOC(OM, n) ALLOC(Q, n) ALLOC(keys, n) ALLOC(skeys, n)
     ALLOC(perm, n) ALLOC(cstart, s->ncells) ALLOC(cend, s->ncells) ALLOC(status, 2)
-    ALLOC(scan_xy, 3 * scan_pairs(n)) ALLOC(scan_z, 3 * scan_pairs(n))
-    ALLOC(heavy, n) ALLOC(heavy_list, n) ALLOC(heavy_count, 1) ALLOC(runs, (size_t)n / 32 + 2)
-    ALLOC(rows, 9 * (size_t)n)
+    // the sweeps' scan copies, rows, list, run bits, count and flags in one (a piece
+    // of its own for each: 1,717 us for a handle of 125,000 particles, now 1,630)
+    auto padded = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+    const size_t xy_b = padded(sizeof(float4) * 3 * scan_pairs(n)),
+                 z_b = padded(sizeof(float2) * 3 * scan_pairs(n)),
+                 rows_b = padded(sizeof(int2) * 9 * n), list_b = padded(sizeof(uint32_t) * n),
+                 runs_b = padded(sizeof(uint32_t) * ((size_t)n / 32 + 2));
+    ALLOC(sweep_mem, xy_b + z_b + rows_b + list_b + runs_b + 256 + n)
+    uint8_t* at = s->sweep_mem;
+    auto piece = [&](size_t bytes) {
+        uint8_t* const p = at;
+        if (at) at += bytes;
+        return p;
+    };
+    s->scan_xy = (float4*)piece(xy_b);
+    s->scan_z = (float2*)piece(z_b);
+    s->rows = (int2*)piece(rows_b);
+    s->heavy_list = (uint32_t*)piece(list_b);
+    s->runs = (uint32_t*)piece(runs_b);
+    s->heavy_count = (uint32_t*)piece(256);
+    s->heavy = piece(n);
     if (num_scenes > 1) {
         ALLOC(d_consts, num_scenes) ALLOC(sid, n) ALLOC(sid_sorted, n)
     }

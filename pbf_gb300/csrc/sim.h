@@ -56,6 +56,7 @@ struct pbf_sim {
     uint32_t* pair_idx = nullptr;
     int32_t* pair_cnt = nullptr;
     uint32_t pair_cap = 0;
+    uint8_t* sweep_mem = nullptr;  // holds the buffers from here to scan_z
     // mixed sweeps (pbf_tuning::coop_candidates): per-particle flag, the
     // flagged sorted indices and their count
     uint8_t* heavy = nullptr;
