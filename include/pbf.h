@@ -183,7 +183,7 @@ pbf_status pbf_device_buffers(pbf_sim* sim, float** x4, float** v4);
  * Asynchronous on the handle's stream.  After the first call the substep is
  * replayed from a captured CUDA graph (one per sweep configuration).  Under
  * PBF_SWEEP_AUTO, a call in which a trial completes waits on the host for the
- * trial's substeps (at most once per trial period, 32 to 256 substeps). */
+ * trial's substeps (at most once per trial period, 16 to 256 substeps). */
 pbf_status pbf_step(pbf_sim* sim, uint32_t substeps);
 
 /* Performance knobs of a handle.  None of them changes any result: every
@@ -234,7 +234,9 @@ typedef struct pbf_tuning {
     uint32_t auto_period;         /* PBF_SWEEP_AUTO: substeps before the first trial and
                                      between trials while the choice or its measured
                                      time keeps changing (doubling up to 256 substeps
-                                     while both hold); 0 = 32 */
+                                     while both hold, half after a first trial without
+                                     a change or while the time more than doubles
+                                     between trials); 0 = 32 */
     uint32_t adjoint_warp_candidates; /* pbf_backward: particles whose stencil holds more
                                      than this many candidates get a warp each in the
                                      reverse neighbour sweeps (their pair terms summed

@@ -15,10 +15,19 @@
 //  - the period returns to `base` when a choice changed or the chosen
 //    configurations' time drifted by more than kAutoDrift either way since
 //    the last trial, and doubles up to kAutoPeriodMax otherwise;
+//  - it is half of `base` after a first trial that changed nothing (there is no
+//    earlier time to hold against) and after one whose time grew by more than
+//    kAutoSurge: a scene that is collapsing outgrows its configuration within
+//    a period.  (The 2M dam break keeps the mixed sweeps at its first trial, at
+//    substep 32, and is better off direct from 50: doubling left the next trial
+//    at 99 and the first 100 substeps at 124 s, 1,420 and 3,243 ms per substep
+//    over the last two quarters);
 //  - a candidate whose total time exceeded kAutoPrune times the best one's
 //    sits out the next kAutoPruneFirst trials, twice as many each time it
 //    loses that way again (up to kAutoPruneMax); the current configurations
-//    always run.
+//    always run.  A sit-out for a loss below kAutoNarrow ends when the time surged:
+//    it was measured in another state (a larger loss is rarely made good, and
+//    trying the masked sweeps in a collapsed scene costs many substeps).
 #pragma once
 
 #include <algorithm>
@@ -33,6 +42,8 @@ constexpr uint32_t kAutoPeriod = 32;
 constexpr uint32_t kAutoPeriodMax = 256;
 constexpr double kAutoMargin = 0.97;
 constexpr double kAutoDrift = 1.25;
+constexpr double kAutoSurge = 2.0;
+constexpr double kAutoNarrow = 2.25;
 constexpr double kAutoPrune = 2.0;
 constexpr uint32_t kAutoPruneFirst = 3;
 constexpr uint32_t kAutoPruneMax = 64;
@@ -45,6 +56,7 @@ struct AutoPolicy {
     double last_ms = 0.0;          // the chosen configurations' time at the last trial
     uint32_t skip[5] = {};         // trials a configuration still sits out
     uint32_t skip_len[5] = {};     // its last sit-out
+    double lost[5] = {};           // and its time over the best one's then
     uint32_t trials = 0;
 
     void reset(uint32_t base_period) {
@@ -54,6 +66,7 @@ struct AutoPolicy {
         last_ms = 0.0;
         for (uint32_t& k : skip) k = 0;
         for (uint32_t& k : skip_len) k = 0;
+        for (double& k : lost) k = 0.0;
         trials = 0;
     }
 
@@ -99,6 +112,7 @@ struct AutoPolicy {
         double now = solver_ms[index_of(ns)] + (use_vort ? vort_ms[index_of(nv)] : 0.0);
         const bool drifted =
             last_ms > 0.0 && (now > kAutoDrift * last_ms || now * kAutoDrift < last_ms);
+        const bool first = last_ms == 0.0, surged = !first && now > kAutoSurge * last_ms;
         last_ms = now;
         double best = 0.0;
         for (size_t c = 0; c < nc; ++c) {
@@ -111,14 +125,21 @@ struct AutoPolicy {
             if (t > kAutoPrune * best) {
                 len = len ? std::min(2 * len, kAutoPruneMax) : kAutoPruneFirst;
                 skip[cands[c]] = len;
+                lost[cands[c]] = t / best;
             } else {
                 len = 0;
             }
         }
+        if (surged)
+            for (uint32_t p = 0; p < 5; ++p)
+                if (lost[p] < kAutoNarrow) skip[p] = 0;
         const bool changed = ns != solver || nv != vort || drifted;
         solver = ns;
         vort = nv;
-        period = changed ? base : std::min(2 * period, std::max(base, kAutoPeriodMax));
+        const uint32_t half = base > kAutoPeriodMax ? base : std::max(base / 2, 1u);
+        period = surged || (first && !changed) ? half
+                 : changed                     ? base
+                                               : std::min(2 * period, std::max(base, kAutoPeriodMax));
         next = count + 1 + period;
         ++trials;
     }

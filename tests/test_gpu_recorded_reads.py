@@ -38,11 +38,11 @@ def test_reads_of_the_last_substep(gpu, substeps, every, iterations, vorticity):
                               np.ascontiguousarray(b).view(np.uint32))
 
 
-@pytest.mark.parametrize("substeps,every", [(8, 8), (8, 3), (6, 4)])
+@pytest.mark.parametrize("substeps,every", [(8, 8), (8, 3), (8, 6), (7, 4)])
 def test_trials_go_on_in_the_recorded_segment(gpu, substeps, every):
-    # the first trial starts at substep 3 and takes three substeps; the next
-    # cannot end before substep 9
-    stepped, recorded = make(auto_period=3), make(auto_period=3)
+    # the first trial starts at substep 4 and takes three substeps; the next
+    # starts at substep 9 at the earliest
+    stepped, recorded = make(auto_period=4), make(auto_period=4)
     stepped.step(substeps)
     recorded.forward_record(substeps, every)
     assert stepped.sweep_choice()["trials"] == 1
