@@ -201,8 +201,18 @@ struct PairDirs {
 // outside the grid, whose one-way candidates the forward lists lack) scans its
 // stencil in the first of the two sweeps, writing its candidates to the
 // handle's own pair-list buffer, and replays those in the second; without
-// room there it visits the stencil both times.  Results are the same either
-// way (the pair terms test r2 themselves, in the same order).
+// room there it visits the stencil both times.  The same pairs are added in the
+// same order either way, but for pairs within rounding of the radius: the forward
+// lists test r2 with fused multiply-adds, the reverse scans and terms without.
+// There h - r rounds to 0, and what such a pair adds (dW of (h^2 - r^2)^2) is below
+// 1e-13 of the others'.
+//
+// Every index stays in range: list entries are candidates of the rows, written
+// and counted by the sweep that found them (a count above the capacity is stored
+// as -1, and the recorded counts start at -1, so a list that no sweep wrote is not
+// read); the rows come from the cell tables, whose bounds are sorted indices; and
+// the own list's count is written by the first sweep for exactly the particles
+// for which the second reads it.
 struct AdjLists {
     PairLists rec;         // the forward run's list of this position set (cap 0: none)
     PairLists own;         // scratch list (cap 0: none)

@@ -187,7 +187,9 @@ void reset_sweep_choice(pbf_sim* s) {
                                           : PBF_PASS_MASKED;
     // (mixed for one large scene: the 2M dam break's window runs 2.1x faster
     // under it than masked; a batch of small scenes starts masked, where mixed
-    // measured slower)
+    // measured slower, with the quads too: masked / mixed, us, lambda and delta-p of
+    // 6 scenes of 61,372 particles in all 33.0 / 37.4 and 18.4 / 16.4, of 16 of
+    // 131,025 44.5 / 49.0 and 20.7 / 26.5)
     if (m == PBF_SWEEP_AUTO)
         pass = s->n < kCoopBelow ? PBF_PASS_COOP
                                  : (s->nscenes == 1 ? PBF_PASS_MIXED : PBF_PASS_MASKED);

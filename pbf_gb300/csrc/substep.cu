@@ -1128,6 +1128,10 @@ __global__ void __launch_bounds__(kBlock) k_coop(Body body, uint32_t n, CP cp, C
 // 14.5, 19.4 -> 5.2; 32,768 (a thread each) 26.0 -> 18.5, 14.8 -> 6.9, 29.7 ->
 // 21.0, 15.1 -> 7.0; 65,536 (two blocks, 32 candidates per particle) delta-p
 // 11.9 -> 10.0, but lambda 19.2 -> 23.9: there only the second sweeps are quads.
+// With 216 candidates per particle, stage times with a thread and with four lanes:
+// lambda 34.3 / 22.8 at 32,768 particles, 35.8 / 33.0 at 46,656, 36.2 / 36.7 at
+// 47,652, 36.4 / 37.1 at 63,960, vorticity A 37.1 / 24.8, 38.9 / 37.1, 39.4 / 42.0,
+// 39.4 / 42.2: hence kQuadScanBelow.
 // What bounds it now: latency (scan of 16,384: 5.8 of 13.6 us, the pairs 4.4).
 constexpr int kQuad = 4;  // SweepCfg mode
 constexpr int kQuadBlock = 64;
@@ -1518,7 +1522,6 @@ k_stencil_rows(const float4* __restrict__ XP, const int32_t* __restrict__ cstart
 // counter per launch instead was slower (lambda 87 us, 5.2 us empty).
 inline unsigned heavy_grid(uint32_t n) { return 152u * (n < 1048576u ? 8u : 20u); }
 
-// Grid of warps, one per particle.
 // Grid and launch of a quad sweep: eight lanes per particle below kOctsBelow
 // particles (shorter chains), four above (fewer instructions).  Four / eight
 // lanes, us: 16,384 particles lambda 13.7 / 13.6, delta-p 6.2 / 5.1; 32,768
@@ -1536,6 +1539,7 @@ inline unsigned quad_heavy_blocks(uint32_t n) { return n / 2u < 4864u ? n / 2u +
         else                                                                              \
             KERNEL<CP, 4><<<g_, kQuadBlock, 0, st>>>(q_, __VA_ARGS__);                    \
     } while (0)
+// Grid of warps, one per particle.
 inline unsigned coop_grid(uint32_t n) { return (unsigned)(((size_t)n * 32 + kBlock - 1) / kBlock); }
 
 // update.glsl:16-28: v = (x* - x_old) / dt, x = x*, scattered back to id order.

@@ -20,12 +20,8 @@ __global__ void k_find_cells(const uint32_t* __restrict__ skeys, const uint32_t*
 
 // Host launchers of the templated stage kernels (explicitly instantiated for
 // OneScene and ManyScenes in substep.cu).  The neighbour-sweep launchers take
-// their block size (32..256, a multiple of 32); the others take a grid of
-// kBlock-thread blocks.
-// Launch shape of the neighbour sweeps: threads per block; the stencil scan
-// (0: the reference's loop shape, visit_full; 1: masked scans, visit_masked;
-// 2: masked scans that record the exact pair lists the next sweep replays);
-// whether the skin-radius neighbour lists are used.
+// their shape (SweepCfg); the others take a grid of kBlock-thread blocks.
+
 // The quad sweeps (substep.cu) take particles of at most this many stencil
 // candidates, and as first sweeps (which scan) scenes below this many particles.
 constexpr uint32_t kQuadCandidates = 256;
@@ -34,6 +30,12 @@ constexpr uint32_t kQuadScanBelow = 49152;
 // per thread.
 constexpr unsigned kLambdaMaxBlock = 1024, kVortMaxBlock = 512;
 
+// Launch shape of a neighbour sweep: threads per block (a multiple of 32: up to 256
+// where the caller chose it, scan_block.h otherwise; the cooperative and quad
+// sweeps have their own); the stencil scan (0: the reference's loop shape,
+// visit_full; 1: masked scans, visit_masked; 2: masked scans that record the exact
+// pair lists the next sweep replays; 3: cooperative; 4: quads); whether the
+// skin-radius neighbour lists are used.
 struct SweepCfg {
     unsigned block;
     int mode;
