@@ -25,9 +25,12 @@
 //  - a candidate whose total time exceeded kAutoPrune times the best one's
 //    sits out the next kAutoPruneFirst trials, twice as many each time it
 //    loses that way again (up to kAutoPruneMax); the current configurations
-//    always run.  A sit-out for a loss below kAutoNarrow ends when the time surged:
-//    it was measured in another state (a larger loss is rarely made good, and
-//    trying the masked sweeps in a collapsed scene costs many substeps).
+//    always run.  The direct sweeps' sit-out ends when the time surged: they are the
+//    ones that gain as a scene collapses (they skip runs of equal positions), so a
+//    loss in an earlier state says little.  (Trying the masked sweeps again there
+//    costs many substeps.)  ms for the first substeps of a collapse, sat out / called
+//    back: 16,384 particles, 300 substeps 458 / 293, 29,791, 200 substeps 1,350 /
+//    554, 45,360, 125 substeps 1,728 / 1,596, 62,400, 80 substeps 758 / 851.
 #pragma once
 
 #include <algorithm>
@@ -43,7 +46,6 @@ constexpr uint32_t kAutoPeriodMax = 256;
 constexpr double kAutoMargin = 0.97;
 constexpr double kAutoDrift = 1.25;
 constexpr double kAutoSurge = 2.0;
-constexpr double kAutoNarrow = 2.25;
 constexpr double kAutoPrune = 2.0;
 constexpr uint32_t kAutoPruneFirst = 3;
 constexpr uint32_t kAutoPruneMax = 64;
@@ -56,7 +58,6 @@ struct AutoPolicy {
     double last_ms = 0.0;          // the chosen configurations' time at the last trial
     uint32_t skip[5] = {};         // trials a configuration still sits out
     uint32_t skip_len[5] = {};     // its last sit-out
-    double lost[5] = {};           // and its time over the best one's then
     uint32_t trials = 0;
 
     void reset(uint32_t base_period) {
@@ -66,7 +67,6 @@ struct AutoPolicy {
         last_ms = 0.0;
         for (uint32_t& k : skip) k = 0;
         for (uint32_t& k : skip_len) k = 0;
-        for (double& k : lost) k = 0.0;
         trials = 0;
     }
 
@@ -125,14 +125,11 @@ struct AutoPolicy {
             if (t > kAutoPrune * best) {
                 len = len ? std::min(2 * len, kAutoPruneMax) : kAutoPruneFirst;
                 skip[cands[c]] = len;
-                lost[cands[c]] = t / best;
             } else {
                 len = 0;
             }
         }
-        if (surged)
-            for (uint32_t p = 0; p < 5; ++p)
-                if (lost[p] < kAutoNarrow) skip[p] = 0;
+        if (surged) skip[PBF_PASS_DIRECT] = 0;
         const bool changed = ns != solver || nv != vort || drifted;
         solver = ns;
         vort = nv;
